@@ -890,20 +890,17 @@ DG_HD void dt_face(int64_t f, const HotView<T>& h) {
   double nx = h.faceNormal[2 * f], ny = h.faceNormal[2 * f + 1], area = h.faceArea[f];
   double UL[4];
   load4<T>(&h.u[(int64_t)L * 4], UL);
-  double pL, aL2, HL, pR, aR2, HR;
-  double uL = UL[1] / UL[0], vL = UL[2] / UL[0], uR = uL, vR = vL;
-  thermal(UL[3], UL[0], uL * uL + vL * vL, h.gamma, pL, aL2, HL);
-  pR = pL; aR2 = aL2;
-  double rhoMean = UL[0];
-  if (R >= 0) {
-    double UR[4];
-    load4<T>(&h.u[(int64_t)R * 4], UR);
-    rhoMean = (UL[0] + UR[0]) * 0.5;
-    uR = UR[1] / UR[0]; vR = UR[2] / UR[0];
-    thermal(UR[3], UR[0], uR * uR + vR * vR, h.gamma, pR, aR2, HR);
-  }
-  double vn = 0.5 * ((uL + uR) * nx + (vL + vR) * ny);
-  double pMean = (pL + pR) * 0.5;
+  const double g1 = h.gamma - 1;
+  double UR[4] = {UL[0], UL[1], UL[2], UL[3]};
+  if (R >= 0) load4<T>(&h.u[(int64_t)R * 4], UR);
+  const double iLR = 1.0 / (UL[0] * UR[0]), irL = iLR * UR[0], irR = iLR * UL[0];  // one quotient for both densities
+  const double uL = UL[1] * irL, vL = UL[2] * irL;
+  const double pL = g1 * (UL[3] - UL[0] * 0.5 * (uL * uL + vL * vL)), aL2 = h.gamma * pL * irL;
+  const double uR = UR[1] * irR, vR = UR[2] * irR;
+  const double pR = g1 * (UR[3] - UR[0] * 0.5 * (uR * uR + vR * vR)), aR2 = h.gamma * pR * irR;
+  const double rhoMean = (UL[0] + UR[0]) * 0.5;
+  const double vn = 0.5 * ((uL + uR) * nx + (vL + vR) * ny);
+  const double pMean = (pL + pR) * 0.5;
   double lam = fabs(vn) + sqrt(h.gamma * pMean / rhoMean);
   if (h.mu > 0) {  // viscous part (DNDS_FV_EulerEvaluator.cpp:80-99)
     const double lamVis = sutherland_mu(h, pMean, rhoMean) / rhoMean * dmax(4. / 3., h.gamma / h.pr);

