@@ -390,6 +390,10 @@ __device__ __forceinline__ double stage_time(const double* scal, int useDev, dou
   return useDev ? (c == 0.0 ? scal[S_T] : scal[S_T] + c * scal[S_DT]) : tHost;
 }
 
+__device__ __forceinline__ void reset_dtmin(double* scal) {
+  reinterpret_cast<unsigned long long*>(scal)[S_DTMIN] = 0x7ff0000000000000ull;
+}
+
 // faces [f0, f1): interior faces first (BND = false), then boundary faces.  The FP32 Roe interior
 // kernel runs 4 blocks per SM (64 registers, a few spilled words): the gathers want the occupancy
 // more than the registers (measured: 2 blocks 0.296 ms, 3: 0.283, 4: 0.243, 5: 0.318 per RHS on
@@ -398,16 +402,20 @@ __device__ __forceinline__ double stage_time(const double* scal, int useDev, dou
 // registers and 172 B spilled 8.02-8.04 ms)
 // DT = true (the first stage of an SSP-RK3 step): each thread first writes its face's EvaluateDt terms
 // (dt_face: lambda A and the entropy-fix dLambda, from the same means this stage reads), which the
-// flux then reads back, so the step needs no separate face pass for dt
+// flux then reads back, so the step needs no separate face pass for dt; the dt minimum is reset for the
+// cell pass that follows
 template <class T, int RIEMANN, bool BND, bool DT = false>
-__global__ void __launch_bounds__(kBlock, (sizeof(T) == 4 && RIEMANN == 1 && !BND) ? 4 : ((sizeof(T) == 4 && !BND) ? 3 : 2)) k_face_flux(HotView<T> h, int64_t f0, int64_t f1, const double* scal,
+__global__ void __launch_bounds__(kBlock, (sizeof(T) == 4 && RIEMANN == 1 && !BND) ? 4 : ((sizeof(T) == 4 && !BND) ? 3 : 2)) k_face_flux(HotView<T> h, int64_t f0, int64_t f1, double* scal,
                                                          int useDev, double tHost, double c, unsigned* flags,
                                                          unsigned long long* nred) {
   int64_t f = f0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int r = 0;
   bool bad = false;
   if (f < f1) {
-    if constexpr (DT) dt_face<T>(f, h);
+    if constexpr (DT) {
+      if (f == f0) reset_dtmin(scal);
+      dt_face<T>(f, h);
+    }
     double out[4];
     double t = stage_time(scal, useDev, tHost, c);
     if constexpr (sizeof(T) == 4 && RIEMANN == 1 && !BND)
@@ -471,8 +479,7 @@ __global__ void __launch_bounds__(kBlock) k_dt_face(HotView<T> h) {
 }
 
 __global__ void k_init_dtmin(double* scal) {
-  unsigned long long inf = 0x7ff0000000000000ull;
-  reinterpret_cast<unsigned long long*>(scal)[S_DTMIN] = inf;
+  reset_dtmin(scal);
   scal[S_INC] = 0.0;
 }
 
@@ -505,11 +512,11 @@ __global__ void __launch_bounds__(kBlock) k_dt_cell(HotView<T> h, double cfl, do
 }
 
 // step dt = min(dt_min, t_end - t)
-__global__ void k_dt_finalize(double* scal, double tEnd) {
-  double dmin = __longlong_as_double((long long)reinterpret_cast<unsigned long long*>(scal)[S_DTMIN]);
-  double rem = tEnd - scal[S_T];
-  scal[S_DT] = fmax(0.0, fmin(dmin, rem));
+__device__ __forceinline__ double step_dt(const double* scal, double tEnd) {
+  const double dmin = __longlong_as_double((long long)reinterpret_cast<const unsigned long long*>(scal)[S_DTMIN]);
+  return fmax(0.0, fmin(dmin, tEnd - scal[S_T]));
 }
+__global__ void k_dt_finalize(double* scal, double tEnd) { scal[S_DT] = step_dt(scal, tEnd); }
 __global__ void k_advance_time(double* scal) { scal[S_T] += scal[S_DT]; }
 
 __global__ void k_fill_dt(double* dt, int64_t n, const double* scal) {
@@ -517,9 +524,14 @@ __global__ void k_fill_dt(double* dt, int64_t n, const double* scal) {
   if (i < n) dt[i] = __longlong_as_double((long long)reinterpret_cast<const unsigned long long*>(scal)[S_DTMIN]);
 }
 
-// rhs gather + (optionally) SSP-RK3 stage update (ExplicitSSPRK3LocalDt::Step, DNDS_ODE.hpp:140-163)
-template <class T, int STAGE>
-__global__ void __launch_bounds__(kBlock) k_cell_update(HotView<T> h, const double* scal) {
+// rhs gather + (optionally) SSP-RK3 stage update (ExplicitSSPRK3LocalDt::Step, DNDS_ODE.hpp:140-163).
+// STEP = true, the whole-step composition: the first stage takes dt from the minimum itself (and writes it
+// for the later stages) and keeps its means as uLast, the last stage advances the time, so that a step
+// needs no launches of their own for these (10 launches instead of 13; ten graph-replayed steps on 1,600
+// quads 394 -> 361 us) and no pass that copies the means.  One thread writes each scalar; no other thread of
+// the launch reads that one
+template <class T, int STAGE, bool STEP = false>
+__global__ void __launch_bounds__(kBlock) k_cell_update(HotView<T> h, double* scal, double tEnd = 0.0) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= h.N) return;
   double r[4];
@@ -530,9 +542,16 @@ __global__ void __launch_bounds__(kBlock) k_cell_update(HotView<T> h, const doub
     o[1] = make_double2(r[2], r[3]);
     return;
   }
-  const double dt = scal[S_DT];
+  const double dt = STEP && STAGE == 0 ? step_dt(scal, tEnd) : scal[S_DT];
+  if (STEP && STAGE == 0 && i == 0) scal[S_DT] = dt;
+  if (STEP && STAGE == 2 && i == 0) scal[S_T] += dt;
   double x[4];
   load4<T>(&h.u[i * 4], x);
+  if (STEP && STAGE == 0) {
+    double2* o = reinterpret_cast<double2*>(&h.uLast[i * 4]);
+    o[0] = make_double2(x[0], x[1]);
+    o[1] = make_double2(x[2], x[3]);
+  }
   for (int v = 0; v < 4; v++) x[v] += r[v] * dt;
   if (STAGE > 0) {
     const double cf = STAGE == 1 ? 0.25 : 2.0 / 3.0;
@@ -760,29 +779,18 @@ int run_dt(dndsg_ctx* c, double cfl, double maxDt, bool copyLast, cudaStream_t s
 template <class T>
 int run_step(dndsg_ctx* c, double cfl, double tEnd, cudaStream_t s) {
   const bool fuseDt = !(c->s.mu_gas > 0);
-  if (fuseDt) {
-    k_init_dtmin<<<1, 1, 0, s>>>(c->scal);
-  } else {
-    run_dt<T>(c, cfl, 1e100, true, s);
-    k_dt_finalize<<<1, 1, 0, s>>>(c->scal, tEnd);
-  }
+  if (!fuseDt) run_dt<T>(c, cfl, 1e100, false, s);
   const double cst[3] = {0.0, 1.0, 0.5};
   for (int stg = 0; stg < 3; stg++) {
     run_vr<T>(c, false, s);
     if (c->s.limiter) run_limiter<T>(c, 0, s);
     HotView<T> h = view<T>(c);
-    if (stg == 0 && fuseDt) {
-      launch_flux<T>(c, 1, 0.0, cst[stg], s, true);
-      k_dt_cell<T, true><<<grid_for(c->N), kBlock, 0, s>>>(h, cfl, 1e100, c->scal);
-      k_dt_finalize<<<1, 1, 0, s>>>(c->scal, tEnd);
-    } else {
-      launch_flux<T>(c, 1, 0.0, cst[stg], s);
-    }
-    if (stg == 0) k_cell_update<T, 0><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
-    else if (stg == 1) k_cell_update<T, 1><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
-    else k_cell_update<T, 2><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
+    launch_flux<T>(c, 1, 0.0, cst[stg], s, stg == 0 && fuseDt);
+    if (stg == 0 && fuseDt) k_dt_cell<T, false><<<grid_for(c->N), kBlock, 0, s>>>(h, cfl, 1e100, c->scal);
+    if (stg == 0) k_cell_update<T, 0, true><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal, tEnd);
+    else if (stg == 1) k_cell_update<T, 1, true><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal, tEnd);
+    else k_cell_update<T, 2, true><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal, tEnd);
   }
-  k_advance_time<<<1, 1, 0, s>>>(c->scal);
   return 0;
 }
 
@@ -1445,7 +1453,7 @@ int dndsg_ssprk3_step(dndsg_ctx* c, double cfl, double t_end, void* s) {
 }
 
 // n SSP-RK3 steps, pairs of them replayed from a CUDA graph: on small meshes a step is a handful of
-// microseconds of work behind 14 launches, and one graph launch replaces 28.  The graph is captured
+// microseconds of work behind 10 launches, and one graph launch replaces 20.  The graph is captured
 // (on a private stream) the first time a cfl / t_end / buffer parity is seen and kept.
 int dndsg_ssprk3_steps(dndsg_ctx* c, double cfl, double t_end, int64_t n, void* s) {
   if (!c || n < 0) return DNDSG_BAD_ARGUMENT;

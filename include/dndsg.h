@@ -174,7 +174,7 @@ int dndsg_ssprk3_step(dndsg_ctx* ctx, double cfl, double t_end, void* stream);
 
 /* n calls of dndsg_ssprk3_step, with the same results: pairs of steps are
  * replayed from a CUDA graph captured on first use for this cfl / t_end (one
- * graph launch instead of 26 kernel launches, 28 with a viscous flux; small
+ * graph launch instead of 20 kernel launches, 24 with a viscous flux; small
  * meshes are launch-bound).
  * Same arguments as dndsg_ssprk3_step plus the step count n >= 0. */
 int dndsg_ssprk3_steps(dndsg_ctx* ctx, double cfl, double t_end, int64_t n, void* stream);
