@@ -20,6 +20,7 @@
 #include "dndsg_async.cuh"
 #include "dndsg_mlp.cuh"
 #include "dndsg_sa.cuh"
+#include "dndsg_lusgs.cuh"
 
 using namespace dg;
 
@@ -82,19 +83,19 @@ struct dndsg_ctx {
   // increment, residual accumulator
   int32_t *rankOf = nullptr, *fwdCells = nullptr, *bwdCells = nullptr;
   std::vector<int64_t> fwdOff, bwdOff;
-  int64_t *fwdOffDev = nullptr, *bwdOffDev = nullptr;  // level offsets on the device (scan-order mode)
-  int32_t *fwdNbF = nullptr, *fwdNbJ = nullptr, *bwdNbF = nullptr, *bwdNbJ = nullptr;  // [pos][4] records
-  void* lusgsMat = nullptr;  // per-position neighbour-matrix records of one sweep (scan-order mode)
-  int32_t *fwdNbP = nullptr, *bwdNbP = nullptr;  // [pos][4] neighbour schedule positions (-1: not in the ring)
-  int64_t maxLevelWidth = 0;
+  // scan-order mode: the walk schedule of each sweep on the device (dndsg_lusgs_sched.hpp) and the
+  // records of one sweep
+  struct Walk {
+    WalkDev dev{};
+    int ns = 2, blocks = 1;
+  } fwdWalk, bwdWalk;
+  void *walkRec = nullptr, *walkRec5 = nullptr;
   std::vector<int32_t> colourHost;  // greedy colouring, kept for dndsg_lusgs_colours
   int lusgsOrder = 0;               // 0 colour batches, 1 level-scheduled scan order
   // partitioned scan-order sweeps (the reference on several ranks): the part of every cell (empty:
-  // one part), and per sweep the index of every part's first level in fwdOff / bwdOff ([parts + 1],
-  // device) with the most levels of one part
+  // one part), and the most levels of one part per sweep
   std::vector<int32_t> lusgsPart;
   int lusgsParts = 1;
-  int32_t *fwdPartLev = nullptr, *bwdPartLev = nullptr;
   int fwdPartMax = 0, bwdPartMax = 0;
   std::vector<int64_t> scanHost;  // the scan order last set (empty: natural cell order)
   double *Dinv = nullptr, *inc = nullptr, *resAcc = nullptr;
@@ -140,6 +141,16 @@ int dalloc(dndsg_ctx* c, P*& p, size_t bytes) {
   c->allocs.push_back(q);
   p = (P*)q;
   return 0;
+}
+
+// gives back one of the context's buffers
+template <class P>
+void dfree(dndsg_ctx* c, P*& p) {
+  auto it = std::find(c->allocs.begin(), c->allocs.end(), (void*)p);
+  if (it == c->allocs.end()) return;
+  c->allocs.erase(it);
+  cudaFree((void*)p);
+  p = nullptr;
 }
 
 // ------------------------------------------------------------------ warp/block reductions
@@ -2334,349 +2345,6 @@ __global__ void __launch_bounds__(kBlock) k_lusgs_batch(HotView<T> h, const int3
   if (t < n) lusgs_cell<T, FWD>(h, rankOf, cells[t], alpha, Dinv, rhs, inc);
 }
 
-// the parts of one LU-SGS cell update that do not depend on the increments of earlier cells
-struct LusgsPre {
-  int64_t i;
-  bool use[4];  // slot k holds a neighbour that enters this sweep (static slot index: registers)
-  int32_t j[4];
-  double U[4][4], nx[4], ny[4], lam[4], w[4];
-  double base[4], di;
-};
-
-// everything of the cell at schedule position t that does not depend on this sweep's increments.
-// nbF / nbJ [t][4] hold, per face slot, the slot's face (cellFace encoding) and the neighbour when
-// that neighbour enters this sweep (-1 otherwise), so every load here is independent of the others
-template <class T, bool FWD>
-__device__ __forceinline__ void lusgs_prefetch(const HotView<T>& h, const int32_t* cells, const int32_t* nbF,
-                                               const int32_t* nbJ, int64_t t, double alpha, const double* Dinv,
-                                               const double* rhs, LusgsPre& p) {
-  const int64_t i = cells[t];
-  const int4 sf4 = reinterpret_cast<const int4*>(nbF)[t];
-  const int4 j4 = reinterpret_cast<const int4*>(nbJ)[t];
-  const int32_t sfa[4] = {sf4.x, sf4.y, sf4.z, sf4.w}, ja[4] = {j4.x, j4.y, j4.z, j4.w};
-  p.i = i;
-  if (FWD) load4<T>(&rhs[i * 4], p.base);
-  p.di = Dinv[i];
-  const double scale = -0.5 * alpha / h.vol[i];
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const bool use = ja[k] >= 0;
-    const int32_t sf = sfa[k];
-    const int32_t f = use ? (sf >= 0 ? sf : ~sf) : 0;   // index 0 is a valid face: loads stay unconditional
-    const int64_t j = use ? ja[k] : i;
-    const double sg = sf >= 0 ? 1.0 : -1.0;
-    const double area = h.faceArea[f];
-    p.use[k] = use;
-    p.j[k] = (int32_t)j;
-    load4<T>(&h.u[j * 4], p.U[k]);
-    p.nx[k] = sg * h.faceNormal[2 * f];
-    p.ny[k] = sg * h.faceNormal[2 * f + 1];
-    p.lam[k] = h.lamA[f] / area;
-    p.w[k] = scale * area;
-  }
-}
-
-constexpr int kRecMaxLevels = 4095;  // level offsets of one sweep held in shared memory
-
-// ---- scan-order sweep over precomputed neighbour records.
-// The neighbour term of UpdateLUSGSForward/Backward, w_q (dF(U_q; n_q, dU_q) - lam_q dU_q)
-// (fluxJacobian0_Right_Times_du, DNDS_FV_EulerEvaluator.hpp:928-956), is linear in the neighbour's
-// increment dU_q, and everything else in it is fixed during the sweep.  So one parallel pass writes,
-// per schedule position, the dU-independent quantities of its up to 4 neighbour terms, and the
-// sequential level walk is left with a short product per neighbour over increments that mostly sit
-// in a shared-memory ring.  With a = nx dU1 + ny dU2 - vn dU0 (= rho dvn) and
-// dp = (gamma - 1)(dU3 - vx dU1 - vy dU2 + kq dU0), kq = |v|^2 / 2:
-//   dF = (nx dU1 + ny dU2, vn dU1 + vx a + nx dp, vn dU2 + vy a + ny dp, H a + vn (dU3 + dp)),
-// the term is w dF - wl dU (wl = w lam), and the U5 row of an SA context adds c a + (w vn - wl) dU5
-// with c = w nuTilde_q / rho_q.  Ten doubles per neighbour instead of the 4x4 matrix (16, plus 4 for
-// the U5 row): the walk moves every record through one SM's shared memory, and record bytes are
-// what its levels wait on.  Fields are grouped in 16-byte pairs and read as such.
-struct __align__(16) LuSlot {
-  double vx, vy, vn, H, kq, wl, nx, ny, w, c;
-};
-struct __align__(16) LuMatF {
-  LuSlot s[4];      // per face slot
-  double x0[4];     // forward: the BDF rhs, where the sum starts; backward: the forward increment, added to di * sum
-  double di;
-  int32_t i, nu;    // cell; number of neighbours that enter this sweep, in s / j / p [0, nu) in face-slot order
-  int32_t j[4];     // neighbour cell
-  int32_t p[4];     // neighbour schedule position in this sweep (-1: not in the ring; read global memory)
-};
-struct __align__(16) LuMatS {
-  LuMatF f;
-  double x0S, diS;  // the U5 part of x0 and di
-  double pad[2];    // 432-B stride: 16-byte loads of 32 consecutive records hit every bank evenly
-};
-static_assert(sizeof(LuMatF) == 400 && sizeof(LuMatS) == 432, "records are bulk-copied in 16-byte units");
-template <bool SA>
-using LuMat = typename std::conditional<SA, LuMatS, LuMatF>::type;
-__device__ __forceinline__ LuMatF& mat_flow(LuMatF& r) { return r; }
-__device__ __forceinline__ LuMatF& mat_flow(LuMatS& r) { return r.f; }
-__device__ __forceinline__ const LuMatF& mat_flow(const LuMatF& r) { return r; }
-__device__ __forceinline__ const LuMatF& mat_flow(const LuMatS& r) { return r.f; }
-
-// the neighbour term w dF - wl dU of one record slot (fields as in LuSlot) added to buf, and its U5
-// row c a + (w vn - wl) dS added to bufS when SA
-template <bool SA>
-__device__ __forceinline__ void lu_term(double vx, double vy, double vn, double H, double kq, double wl, double nx,
-                                        double ny, double w, double c, const double d[4], double dS, double g1,
-                                        double buf[4], double& bufS) {
-  const double dmn = nx * d[1] + ny * d[2];
-  const double a = dmn - vn * d[0];
-  const double dp = g1 * (d[3] - vx * d[1] - vy * d[2] + kq * d[0]);
-  const double dF[4] = {dmn, vn * d[1] + vx * a + nx * dp, vn * d[2] + vy * a + ny * dp, H * a + vn * (d[3] + dp)};
-  for (int v = 0; v < 4; v++) buf[v] += w * dF[v] - wl * d[v];
-  if constexpr (SA) bufS += c * a + (w * vn - wl) * dS;
-}
-
-// writes the record of every schedule position of one sweep, all positions in parallel.  In a
-// partitioned backward sweep a neighbour in another part (position kGhostPos) is a ghost: its
-// increment is the one after the forward sweep, which is what inc holds while this kernel runs, so
-// its term is summed here and folded into x0 (x0 = dU_fwd + di * ghost terms) instead of taking a
-// slot of the walk
-constexpr int32_t kGhostPos = -2;
-template <class T, bool FWD, bool SA>
-__global__ void __launch_bounds__(kBlock) k_lusgs_pack_mat(HotView<T> h, SaView<T> sa, const int32_t* cells,
-                                                           const int32_t* nbF, const int32_t* nbJ, const int32_t* nbP,
-                                                           int64_t n, double alpha, const double* Dinv,
-                                                           const double* rhs, const double* inc, LuMat<SA>* rec) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  LusgsPre p;
-  lusgs_prefetch<T, FWD>(h, cells, nbF, nbJ, t, alpha, Dinv, rhs, p);
-  LuMatF& f = mat_flow(rec[t]);
-  const int4 p4 = reinterpret_cast<const int4*>(nbP)[t];
-  const int32_t pa[4] = {p4.x, p4.y, p4.z, p4.w};
-  const double g1 = h.gamma - 1;
-  int nu = 0;
-  for (int k = 0; k < 4; k++) {  // the used slots first, in slot order (the order of lusgs_cell's sum)
-    f.j[k] = p.i;
-    f.p[k] = 0;
-  }
-  double ghost[4] = {0, 0, 0, 0}, ghostS = 0.0;
-  bool anyGhost = false;
-  for (int k = 0; k < 4; k++) {
-    if (!p.use[k]) continue;
-    const double* U = p.U[k];
-    const double ir = 1.0 / U[0];
-    const double vx = U[1] * ir, vy = U[2] * ir, q2 = vx * vx + vy * vy;
-    const double pr = g1 * (U[3] - 0.5 * U[0] * q2);
-    LuSlot q;
-    q.vx = vx;
-    q.vy = vy;
-    q.vn = vx * p.nx[k] + vy * p.ny[k];
-    q.H = (U[3] + pr) * ir;
-    q.kq = 0.5 * q2;
-    q.wl = p.w[k] * p.lam[k];
-    q.nx = p.nx[k];
-    q.ny = p.ny[k];
-    q.w = p.w[k];
-    q.c = SA ? p.w[k] * sa.u[p.j[k]] * ir : 0.0;
-    if (!FWD && pa[k] == kGhostPos) {
-      double d[4];
-      load4<double>(&inc[(int64_t)p.j[k] * 4], d);
-      lu_term<SA>(q.vx, q.vy, q.vn, q.H, q.kq, q.wl, q.nx, q.ny, q.w, q.c, d, SA ? sa.inc[p.j[k]] : 0.0, g1, ghost,
-                  ghostS);
-      anyGhost = true;
-      continue;
-    }
-    f.s[nu] = q;
-    f.j[nu] = p.j[k];
-    f.p[nu] = pa[k];
-    nu++;
-  }
-  for (int k = nu; k < 4; k++) f.s[k] = LuSlot{};
-  double add[4] = {0, 0, 0, 0};
-  if (!FWD) load4<double>(&inc[p.i * 4], add);
-  if (anyGhost)
-    for (int v = 0; v < 4; v++) add[v] += p.di * ghost[v];
-  for (int v = 0; v < 4; v++) f.x0[v] = FWD ? p.base[v] : add[v];
-  f.di = p.di;
-  f.i = (int32_t)p.i;
-  f.nu = nu;
-  if constexpr (SA) {
-    LuMatS& r = rec[t];
-    const double diS = sa.Dinv[p.i];
-    r.diS = diS;
-    r.x0S = FWD ? sa.rhs[p.i] : sa.inc[p.i] + (anyGhost ? diS * ghostS : 0.0);
-    r.pad[0] = r.pad[1] = 0.0;
-  }
-}
-
-constexpr int kRecBlock = 128;  // threads of the level walk, and records buffered per level
-constexpr int kMatRing = 256;   // (a power of 2) increments of the most recent schedule positions kept in shared memory
-constexpr int kRecStages = 2;   // levels of records in flight: the current one and the next (3 measured no faster)
-constexpr uint32_t kBulkChunk = 16384;
-template <bool SA>
-constexpr size_t mat_smem() {
-  return 32 + sizeof(int32_t) * (kRecMaxLevels + 1) + sizeof(double) * kMatRing * (SA ? 5 : 4) +
-         sizeof(LuMat<SA>) * kRecStages * kRecBlock;
-}
-static_assert(mat_smem<true>() <= 227 * 1024, "level walk fits the shared memory of one block");
-
-// one position of the level walk.  A neighbour's increment comes from the ring when the record
-// gives its position (the schedule set that up: written there by this walk and not yet
-// overwritten), else (position -1) from global memory.  The sum runs over the slots in the order
-// of lusgs_cell.
-__device__ __forceinline__ double2 ld2(const double* p) { return *reinterpret_cast<const double2*>(p); }
-// the ring holds 32 B per position, two 16-B halves; the halves of every other group of four
-// positions are swapped, so 16-B accesses by 32 consecutive positions spread over all banks
-__device__ __forceinline__ double2* ring_half(double* ringF, int32_t pos, int h) {
-  const int r = pos & (kMatRing - 1);
-  return reinterpret_cast<double2*>(ringF + 4 * r + 2 * (h ^ ((r >> 2) & 1)));
-}
-template <bool FWD, bool SA, class T>
-__device__ __forceinline__ void lusgs_mat_cell(const SaView<T>& sa, const LuMat<SA>& r, int32_t t, double* ringF,
-                                               double* ringS, double* inc, double g1) {
-  const LuMatF& f = mat_flow(r);
-  const double2 x01 = ld2(&f.x0[0]), x23 = ld2(&f.x0[2]);
-  const double x0[4] = {x01.x, x01.y, x23.x, x23.y};
-  double buf[4], bufS = 0.0, x0S = 0.0, diS = 0.0;
-  for (int v = 0; v < 4; v++) buf[v] = FWD ? x0[v] : 0.0;
-  if constexpr (SA) {
-    const double2 sd = ld2(&r.x0S);
-    x0S = sd.x;
-    diS = sd.y;
-    bufS = FWD ? x0S : 0.0;
-  }
-  const int4 p4 = *reinterpret_cast<const int4*>(f.p);
-  const int32_t pa[4] = {p4.x, p4.y, p4.z, p4.w};
-  const int nu = f.nu;
-  // the neighbours' increments, all ring reads issued together (any position is a valid ring
-  // slot; values past nu are never used); the rare neighbour outside the ring from global memory
-  double dU[4][4], dS[4] = {0, 0, 0, 0};
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const double2 a = *ring_half(ringF, pa[q], 0), b = *ring_half(ringF, pa[q], 1);
-    dU[q][0] = a.x; dU[q][1] = a.y; dU[q][2] = b.x; dU[q][3] = b.y;
-    if constexpr (SA) dS[q] = ringS[pa[q] & (kMatRing - 1)];
-  }
-  if ((pa[0] | pa[1] | pa[2] | pa[3]) < 0) {
-    const int4 j4 = *reinterpret_cast<const int4*>(f.j);
-    const int32_t ja[4] = {j4.x, j4.y, j4.z, j4.w};
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (q < nu && pa[q] < 0) {
-        load4<double>(&inc[(int64_t)ja[q] * 4], dU[q]);
-        if constexpr (SA) dS[q] = sa.inc[ja[q]];
-      }
-  }
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    if (q >= nu) break;
-    const double* sl = &f.s[q].vx;
-    const double2 vxy = ld2(sl), vnH = ld2(sl + 2), kwl = ld2(sl + 4), nxy = ld2(sl + 6), wc = ld2(sl + 8);
-    lu_term<SA>(vxy.x, vxy.y, vnH.x, vnH.y, kwl.x, kwl.y, nxy.x, nxy.y, wc.x, wc.y, dU[q], dS[q], g1, buf, bufS);
-  }
-  double o[4];
-  for (int v = 0; v < 4; v++) o[v] = FWD ? f.di * buf[v] : x0[v] + f.di * buf[v];
-  double2* g = reinterpret_cast<double2*>(&inc[(int64_t)f.i * 4]);
-  g[0] = *ring_half(ringF, t, 0) = make_double2(o[0], o[1]);
-  g[1] = *ring_half(ringF, t, 1) = make_double2(o[2], o[3]);
-  if constexpr (SA) {
-    const double oS = FWD ? diS * bufS : x0S + diS * bufS;
-    sa.inc[f.i] = oS;
-    ringS[t & (kMatRing - 1)] = oS;
-  }
-}
-
-// a whole level-scheduled sweep in one block, one thread per position and a producer warp.  The
-// producer bulk-copies the next level's records (contiguous in schedule order) into the other half
-// of a shared-memory double buffer on an mbarrier while the other warps finish the current level;
-// the block barrier per level publishes the increments (global memory and the ring).  Positions of
-// a level beyond kRecBlock read their records from global memory.  A bulk copy that does not land
-// in time sets kFlagTimeout and ends the walk.  Partitioned sweeps (partLev non-null) launch one
-// block per part, each walking its own levels (partLev[b] to partLev[b + 1] of off) with its own
-// ring: the parts share no dependency inside a sweep, so the blocks never wait on one another.
-template <bool SA>
-constexpr int mat_threads() { return kRecBlock + 32; }
-template <class T, bool FWD, bool SA>
-__global__ void __launch_bounds__(mat_threads<SA>()) k_lusgs_levels_mat(SaView<T> sa, const LuMat<SA>* rec,
-                                                                        const int64_t* off, int nlev,
-                                                                        const int32_t* partLev, double* inc,
-                                                                        double g1, unsigned* flags) {
-  using R = LuMat<SA>;
-  constexpr int NT = kRecBlock;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smraw);
-  int32_t* so = reinterpret_cast<int32_t*>(smraw + 32);
-  double* ringF = reinterpret_cast<double*>(smraw + 32 + sizeof(int32_t) * (kRecMaxLevels + 1));
-  double* ringS = ringF + 4 * kMatRing;
-  R* buf = reinterpret_cast<R*>(ringS + (SA ? kMatRing : 0));
-  const int tid = threadIdx.x;
-  const bool producer = tid == NT;
-  if (partLev) {  // one block per part: this part's levels
-    const int32_t l0 = partLev[blockIdx.x];
-    nlev = partLev[blockIdx.x + 1] - l0;
-    off += l0;
-  }
-  for (int l = tid; l <= nlev; l += blockDim.x) so[l] = (int32_t)off[l];
-  if (tid == 0) {
-    for (int k = 0; k < kRecStages; k++) mbar_init(smem_u32(&bars[k]), 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  // level l uses buffer and mbarrier l % kRecStages, in phase (l / kRecStages) & 1
-  auto issue = [&](int l) {  // producer
-    const int32_t b = so[l];
-    const int32_t n = min(so[l + 1] - b, kRecBlock);
-    const uint32_t bar = smem_u32(&bars[l % kRecStages]), bytes = (uint32_t)(n * sizeof(R));
-    const uint32_t dst = smem_u32(buf + (l % kRecStages) * kRecBlock);
-    const char* src = reinterpret_cast<const char*>(rec + b);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(bar, bytes);
-    for (uint32_t o = 0; o < bytes; o += kBulkChunk) bulk_g2s(dst + o, src + o, min(kBulkChunk, bytes - o), bar);
-  };
-  if (producer)
-    for (int k = 0; k < kRecStages - 1 && k < nlev; k++) issue(k);
-  int l = 0;
-  bool failed = false;
-  int32_t b = so[0], e = nlev > 0 ? so[1] : 0;
-  for (; l < nlev; l++) {
-    // the buffer of level l + kRecStages - 1 held level l - 1, finished at the last barrier
-    if (producer && l + kRecStages - 1 < nlev) issue(l + kRecStages - 1);
-    const int32_t e2 = so[min(l + 2, nlev)];  // the next level's end, read ahead
-    const int stage = l % kRecStages;
-    bool ok = true;
-    if (tid < NT && b + tid < e) {
-      ok = mbar_wait(smem_u32(&bars[stage]), (l / kRecStages) & 1, kWaitLimit);
-      if (ok) {
-        // the record from the shared buffer, as a shared-memory reference (ld.shared, not generic loads)
-        lusgs_mat_cell<FWD, SA>(sa, buf[stage * kRecBlock + tid], b + tid, ringF, ringS, inc, g1);
-        for (int32_t t = b + tid + kRecBlock; t < e; t += kRecBlock)
-          lusgs_mat_cell<FWD, SA>(sa, rec[t], t, ringF, ringS, inc, g1);
-      }
-    }
-    if (__syncthreads_or(!ok)) {
-      failed = true;
-      break;
-    }
-    b = e;
-    e = e2;
-  }
-  if (failed && producer) {  // let the copies in flight (levels l to l + kRecStages - 1) land before the block exits
-    atomicOr(flags, kFlagTimeout);
-    for (int k = l; k < l + kRecStages && k < nlev; k++)
-      mbar_wait(smem_u32(&bars[k % kRecStages]), (k / kRecStages) & 1, kWaitLimit);
-  }
-}
-
-// a whole sweep of narrow batches (dependency levels) in one thread block: the levels run one
-// after another with a block barrier between them, which makes a level's increments visible to
-// the next; no grid-wide synchronisation and no waiting on flags
-constexpr int kLevelBlock = 512;
-template <class T, bool FWD>
-__global__ void __launch_bounds__(kLevelBlock) k_lusgs_levels(HotView<T> h, const int32_t* rankOf,
-                                                              const int32_t* cells, const int64_t* off, int nlev,
-                                                              double alpha, const double* Dinv, const double* rhs,
-                                                              double* inc) {
-  for (int l = 0; l < nlev; l++) {
-    const int64_t b = off[l], e = off[l + 1];
-    for (int64_t t = b + threadIdx.x; t < e; t += blockDim.x) lusgs_cell<T, FWD>(h, rankOf, cells[t], alpha, Dinv, rhs, inc);
-    __syncthreads();
-  }
-}
-
 // x += inc, with the L1 norm of inc per variable (volume-weighted on request) into acc[4]
 __global__ void __launch_bounds__(kBlock) k_add_inc(int64_t N, double* u, const double* inc, const double* vol,
                                                     int volWise, double* acc) {
@@ -2786,13 +2454,64 @@ int ensure_lusgs(dndsg_ctx* c) {
   return upload_schedule(c, col, fwd, bwd);
 }
 
+constexpr int kMaxPartLevels = 4095;  // of one part, in partitioned sweeps
+constexpr double kWalkHop = 3.0;      // a value from another block of the part, in batches of the walk
+
+template <int NS, bool SA>
+bool walk_attr(int K, int mail, int bars) {
+  const int bytes = (int)walk_smem(NS, SA, mail, bars);
+  if (cudaFuncSetAttribute(k_lusgs_walk<NS, SA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmemMax) != cudaSuccess)
+    return false;
+  if (K == 1) return true;
+  if (K > 8 && cudaFuncSetAttribute(k_lusgs_walk<NS, SA>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return false;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)K;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)K);
+  cfg.blockDim = dim3(walk_threads(SA));
+  cfg.dynamicSmemBytes = bytes;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  return cudaOccupancyMaxActiveClusters(&n, k_lusgs_walk<NS, SA>, &cfg) == cudaSuccess && n > 0;
+}
+// whether the device runs clusters of K blocks of the walk with this much shared memory (and the
+// kernel attributes for it)
+bool walk_fits(dndsg_ctx* c, int ns, int K, int mail, int bars) {
+  const bool ok = c->sa ? (ns == 2 ? walk_attr<2, true>(K, mail, bars) : ns == 3 ? walk_attr<3, true>(K, mail, bars) : walk_attr<4, true>(K, mail, bars))
+                        : (ns == 2 ? walk_attr<2, false>(K, mail, bars) : ns == 3 ? walk_attr<3, false>(K, mail, bars) : walk_attr<4, false>(K, mail, bars));
+  if (!ok) cudaGetLastError();  // not an error of the caller's
+  return ok;
+}
+int upload_walk(dndsg_ctx* c, const WalkSchedule& w, dndsg_ctx::Walk& d) {
+  if (!walk_fits(c, w.ns, w.K, w.mail, w.bars)) return fail(c, DNDSG_CUDA_ERROR, "kernel attributes of the LU-SGS walk");
+  d.ns = w.ns;
+  d.blocks = w.parts * w.K;
+  d.dev.K = w.K;
+  d.dev.mail = w.mail;
+  d.dev.bars = w.bars;
+  int rc;
+  auto put = [&](auto*& dst, const auto& src) -> int {
+    dfree(c, dst);
+    if ((rc = dalloc(c, dst, sizeof(src[0]) * src.size()))) return rc;
+    DG_CUDA(c, cudaMemcpy((void*)dst, src.data(), sizeof(src[0]) * src.size(), cudaMemcpyHostToDevice));
+    return 0;
+  };
+  if ((rc = put(d.dev.nbF, w.nbF)) || (rc = put(d.dev.nbJ, w.nbJ)) || (rc = put(d.dev.meta, w.meta)) ||
+      (rc = put(d.dev.batches, w.batches)) || (rc = put(d.dev.blockBatch, w.blockBatch)))
+    return rc;
+  return 0;
+}
+
 // the reference's sequential sweep in a given scan order, level-scheduled: the forward level of a
 // cell is one more than the largest forward level of its neighbours earlier in the scan (the
-// backward level likewise over the later ones), and each level is one batch.  With parts (the
-// reference on several ranks, DNDS_FV_EulerEvaluator.cpp:1177-1181, 1313-1317) every part sweeps its
-// own cells in the scan order: levels count only neighbours of the same part, the schedule holds
-// part after part (each part's levels contiguous), and a neighbour in another part enters the
-// backward sweep only, as a ghost (kGhostPos) with its post-forward increment
+// backward level likewise over the later ones).  With parts (the reference on several ranks,
+// DNDS_FV_EulerEvaluator.cpp:1177-1181, 1313-1317) every part sweeps its own cells in the scan order:
+// levels count only neighbours of the same part, and a neighbour in another part enters the backward
+// sweep only, as a ghost with its post-forward increment
 int set_scan_order(dndsg_ctx* c, const int64_t* scan2cell) {
   int rc;
   if ((rc = ensure_lusgs(c))) return rc;
@@ -2829,122 +2548,85 @@ int set_scan_order(dndsg_ctx* c, const int64_t* scan2cell) {
     lb[i] = l;
     nlb[part[i]] = std::max(nlb[part[i]], l + 1);
   }
-  // schedule keys: the part's first level plus the level within the part
-  std::vector<int32_t> baseF(P + 1, 0), baseB(P + 1, 0);
-  for (int p = 0; p < P; p++) {
-    baseF[p + 1] = baseF[p] + nlf[p];
-    baseB[p + 1] = baseB[p] + nlb[p];
-  }
   const int fMax = *std::max_element(nlf.begin(), nlf.end()), bMax = *std::max_element(nlb.begin(), nlb.end());
-  if (P > 1 && (std::max(fMax, bMax) > kRecMaxLevels || c->nfmax > 4))  // checked before anything changes
-    return fail(c, DNDSG_UNSUPPORTED, "partitioned sweeps need at most 4 faces per cell and " +
-                                          std::to_string(kRecMaxLevels) + " levels per part");
-  c->fwdPartMax = fMax;
-  c->bwdPartMax = bMax;
-  const int nf = baseF[P], nb = baseB[P];
-  for (int64_t i = 0; i < N; i++) {
-    lf[i] += baseF[part[i]];
-    lb[i] += baseB[part[i]];
-  }
-  std::vector<int32_t> fwd, bwd;
-  group_by(lf, nf, fwd, c->fwdOff);
-  group_by(lb, nb, bwd, c->bwdOff);
-  for (int32_t** d : {&c->fwdPartLev, &c->bwdPartLev}) {
-    if (*d) {
-      auto it = std::find(c->allocs.begin(), c->allocs.end(), (void*)*d);
-      if (it != c->allocs.end()) c->allocs.erase(it);
-      cudaFree(*d);
-      *d = nullptr;
-    }
-  }
-  if (P > 1) {
-    if ((rc = dalloc(c, c->fwdPartLev, sizeof(int32_t) * (P + 1))) || (rc = dalloc(c, c->bwdPartLev, sizeof(int32_t) * (P + 1))))
-      return rc;
-    DG_CUDA(c, cudaMemcpy(c->fwdPartLev, baseF.data(), sizeof(int32_t) * (P + 1), cudaMemcpyHostToDevice));
-    DG_CUDA(c, cudaMemcpy(c->bwdPartLev, baseB.data(), sizeof(int32_t) * (P + 1), cudaMemcpyHostToDevice));
-  }
-  c->maxLevelWidth = 0;
-  for (int k = 0; k < nf; k++) c->maxLevelWidth = std::max(c->maxLevelWidth, c->fwdOff[k + 1] - c->fwdOff[k]);
-  for (int k = 0; k < nb; k++) c->maxLevelWidth = std::max(c->maxLevelWidth, c->bwdOff[k + 1] - c->bwdOff[k]);
-  for (int64_t** d : {&c->fwdOffDev, &c->bwdOffDev}) {
-    if (*d) {
-      auto it = std::find(c->allocs.begin(), c->allocs.end(), (void*)*d);
-      if (it != c->allocs.end()) c->allocs.erase(it);
-      cudaFree(*d);
-      *d = nullptr;
-    }
-  }
-  if ((rc = dalloc(c, c->fwdOffDev, sizeof(int64_t) * (nf + 1))) || (rc = dalloc(c, c->bwdOffDev, sizeof(int64_t) * (nb + 1))))
-    return rc;
-  DG_CUDA(c, cudaMemcpy(c->fwdOffDev, c->fwdOff.data(), sizeof(int64_t) * (nf + 1), cudaMemcpyHostToDevice));
-  DG_CUDA(c, cudaMemcpy(c->bwdOffDev, c->bwdOff.data(), sizeof(int64_t) * (nb + 1), cudaMemcpyHostToDevice));
-  // per schedule position: the face slots and the neighbours that enter each sweep
-  std::vector<int32_t> slots((size_t)aos_size(N, c->nfmax)), L(c->F), R(c->F);
+  if (P > 1 && std::max(fMax, bMax) > kMaxPartLevels)  // checked before anything changes
+    return fail(c, DNDSG_UNSUPPORTED, "partitioned sweeps need at most " + std::to_string(kMaxPartLevels) + " levels per part");
+  // every cell's faces and the cells across
+  std::vector<int32_t> slots((size_t)aos_size(N, c->nfmax)), L(c->F), R(c->F), slotF(4 * N, kEmptySlot), slotJ(4 * N, -1);
   DG_CUDA(c, cudaMemcpy(slots.data(), c->cellFace, sizeof(int32_t) * slots.size(), cudaMemcpyDeviceToHost));
   DG_CUDA(c, cudaMemcpy(L.data(), c->faceL, sizeof(int32_t) * c->F, cudaMemcpyDeviceToHost));
   DG_CUDA(c, cudaMemcpy(R.data(), c->faceR, sizeof(int32_t) * c->F, cudaMemcpyDeviceToHost));
-  auto records = [&](const std::vector<int32_t>& cellsOf, bool forward, std::vector<int32_t>& nf,
-                     std::vector<int32_t>& nj, std::vector<int32_t>& np) {
-    nf.assign(4 * N, kEmptySlot);
-    nj.assign(4 * N, -1);
-    np.assign(4 * N, -1);
-    std::vector<int32_t> at(N);
-    for (int64_t t = 0; t < N; t++) at[cellsOf[t]] = (int32_t)t;
-    for (int64_t t = 0; t < N; t++) {
-      const int64_t i = cellsOf[t];
-      for (int k = 0; k < c->nfmax && k < 4; k++) {
-        const int32_t sf = slots[aos(i, k, c->nfmax)];
-        nf[4 * t + k] = sf;
-        if (sf == kEmptySlot) continue;
-        const int32_t f = sf >= 0 ? sf : ~sf;
-        const int32_t j = sf >= 0 ? R[f] : L[f];
-        if (j < 0) continue;
-        if (part[j] != part[i]) {
-          if (!forward) {
-            nj[4 * t + k] = j;
-            np[4 * t + k] = kGhostPos;
-          }
-        } else if (forward ? pos[j] < pos[i] : pos[j] > pos[i]) {
-          nj[4 * t + k] = j;
-          np[4 * t + k] = at[j];
-        }
-      }
+  for (int64_t i = 0; i < N; i++)
+    for (int k = 0; k < c->nfmax; k++) {
+      const int32_t sf = slots[aos(i, k, c->nfmax)];
+      slotF[4 * i + k] = sf;
+      if (sf != kEmptySlot) slotJ[4 * i + k] = sf >= 0 ? R[sf] : L[~sf];
     }
-  };
-  // the level walk keeps the increments of the last kMatRing positions in a ring; a neighbour at
-  // position pj is still there during level l when pj + kMatRing >= off[l + 1] (the position that
-  // overwrites its slot comes later).  Otherwise the walk reads global memory: position -1.
-  auto ring_or_global = [&](const std::vector<int64_t>& off, std::vector<int32_t>& np) {
-    for (size_t l = 0; l + 1 < off.size(); l++)
-      for (int64_t t = off[l]; t < off[l + 1]; t++)
-        for (int k = 0; k < 4; k++)
-          if (np[4 * t + k] >= 0 && np[4 * t + k] + kMatRing < off[l + 1]) np[4 * t + k] = -1;
-  };
-  std::vector<int32_t> ff, fj, fp, bf, bj, bp;
-  records(fwd, true, ff, fj, fp);
-  records(bwd, false, bf, bj, bp);
-  ring_or_global(c->fwdOff, fp);
-  ring_or_global(c->bwdOff, bp);
-  if (!c->fwdNbF)
-    if ((rc = dalloc(c, c->fwdNbF, sizeof(int32_t) * 4 * N)) || (rc = dalloc(c, c->fwdNbJ, sizeof(int32_t) * 4 * N)) ||
-        (rc = dalloc(c, c->bwdNbF, sizeof(int32_t) * 4 * N)) || (rc = dalloc(c, c->bwdNbJ, sizeof(int32_t) * 4 * N)) ||
-        (rc = dalloc(c, c->fwdNbP, sizeof(int32_t) * 4 * N)) || (rc = dalloc(c, c->bwdNbP, sizeof(int32_t) * 4 * N)))
-      return rc;
-  DG_CUDA(c, cudaMemcpy(c->fwdNbP, fp.data(), sizeof(int32_t) * 4 * N, cudaMemcpyHostToDevice));
-  DG_CUDA(c, cudaMemcpy(c->bwdNbP, bp.data(), sizeof(int32_t) * 4 * N, cudaMemcpyHostToDevice));
-  DG_CUDA(c, cudaMemcpy(c->fwdNbF, ff.data(), sizeof(int32_t) * 4 * N, cudaMemcpyHostToDevice));
-  DG_CUDA(c, cudaMemcpy(c->fwdNbJ, fj.data(), sizeof(int32_t) * 4 * N, cudaMemcpyHostToDevice));
-  DG_CUDA(c, cudaMemcpy(c->bwdNbF, bf.data(), sizeof(int32_t) * 4 * N, cudaMemcpyHostToDevice));
-  DG_CUDA(c, cudaMemcpy(c->bwdNbJ, bj.data(), sizeof(int32_t) * 4 * N, cudaMemcpyHostToDevice));
-  if (!c->lusgsMat && (rc = dalloc(c, c->lusgsMat, (c->sa ? sizeof(LuMatS) : sizeof(LuMatF)) * N))) return rc;
-  for (const void* fn : {(const void*)k_lusgs_levels_mat<float, true, false>, (const void*)k_lusgs_levels_mat<float, false, false>,
-                         (const void*)k_lusgs_levels_mat<double, true, false>, (const void*)k_lusgs_levels_mat<double, false, false>})
-    DG_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mat_smem<false>()));
-  for (const void* fn : {(const void*)k_lusgs_levels_mat<float, true, true>, (const void*)k_lusgs_levels_mat<float, false, true>,
-                         (const void*)k_lusgs_levels_mat<double, true, true>, (const void*)k_lusgs_levels_mat<double, false, true>})
-    DG_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mat_smem<true>()));
+  // one block per part walks the part as long as that is about as short as its levels; else a cluster of
+  // blocks, one per 8 cells of a mean level (measured estimates, 512 x 128 quads in natural order, levels of
+  // 103 cells: 1, 4, 8, 16 blocks take 583, 519, 338, 190 us a sweep; 256 x 64, levels of 51: 120, 130, 81, 83 us),
+  // if the walk gets shorter by that and the device and the mailboxes take it
+  WalkSchedule fwd, bwd;
+  bool several = false;
+  const double one = walk_length_one(N, P, part, lf, nlf) + walk_length_one(N, P, part, lb, nlb);
+  if (one > 1.05 * (fMax + bMax)) {
+    int K = 2;
+    while (K < kWalkMaxK && K * 8.0 < 2.0 * N / (fMax + bMax) / P) K *= 2;
+    while (K > 1 && (int64_t)P * K > c->sms) K /= 2;
+    const int maxMail = walk_max_mail(std::min(4, c->nfmax), c->sa);
+    several = K > 1 && build_walk(N, P, part, order, pos, lf, slotF, slotJ, true, K, maxMail, kWalkHop, fwd) &&
+              build_walk(N, P, part, order, pos, lb, slotF, slotJ, false, K, maxMail, kWalkHop, bwd) &&
+              fwd.time + bwd.time < 0.95 * one &&
+              walk_fits(c, std::max(fwd.ns, bwd.ns), K, std::max(fwd.mail, bwd.mail), std::max(fwd.bars, bwd.bars));
+  }
+  if (!several) {
+    build_walk(N, P, part, order, pos, lf, slotF, slotJ, true, 1, 0, kWalkHop, fwd);
+    build_walk(N, P, part, order, pos, lb, slotF, slotJ, false, 1, 0, kWalkHop, bwd);
+  }
+  if ((rc = upload_walk(c, fwd, c->fwdWalk)) || (rc = upload_walk(c, bwd, c->bwdWalk))) return rc;
+  dfree(c, c->walkRec);
+  dfree(c, c->walkRec5);
+  const int ns = std::max(fwd.ns, bwd.ns);
+  if ((rc = dalloc(c, c->walkRec, (size_t)walk_rec_bytes(ns) * N)) ||
+      (c->sa && (rc = dalloc(c, c->walkRec5, (size_t)walk_rec5_bytes(ns) * N))))
+    return rc;
+  c->fwdPartMax = fMax;
+  c->bwdPartMax = bMax;
   c->lusgsOrder = 1;
-  return upload_schedule(c, pos, fwd, bwd);
+  return 0;
+}
+
+// one sweep in scan order about the context's state: the records, then the walk
+template <int NS, bool SA>
+void launch_walk_ns(dndsg_ctx* c, bool forward, const dndsg_ctx::Walk& w, const WalkGeom& g, double alpha, const double* rhs,
+                    double* inc, const double* rhs5, double* inc5, cudaStream_t s) {
+  unsigned char *rec = (unsigned char*)c->walkRec, *rec5 = (unsigned char*)c->walkRec5;
+  const unsigned grid = grid_for(4 * c->N);
+  if (forward)
+    k_lusgs_records<NS, true, SA><<<grid, kBlock, 0, s>>>(g, w.dev, alpha, c->Dinv, rhs, inc, c->saU, c->saDinv, rhs5, inc5, rec, rec5);
+  else
+    k_lusgs_records<NS, false, SA><<<grid, kBlock, 0, s>>>(g, w.dev, alpha, c->Dinv, rhs, inc, c->saU, c->saDinv, rhs5, inc5, rec, rec5);
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)w.dev.K;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)w.blocks);
+  cfg.blockDim = dim3(walk_threads(SA));
+  cfg.dynamicSmemBytes = walk_smem(NS, SA, w.dev.mail, w.dev.bars);
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_lusgs_walk<NS, SA>, w.dev, (const unsigned char*)rec, (const unsigned char*)rec5, inc, inc5, c->flags);
+}
+template <bool SA>
+void launch_walk(dndsg_ctx* c, bool forward, double alpha, const double* rhs, double* inc, const double* rhs5, double* inc5,
+                 cudaStream_t s) {
+  const dndsg_ctx::Walk& w = forward ? c->fwdWalk : c->bwdWalk;
+  const WalkGeom g{c->N, c->u, c->vol, c->faceArea, c->faceNormal, c->lamA, c->s.gamma};
+  if (w.ns == 2) launch_walk_ns<2, SA>(c, forward, w, g, alpha, rhs, inc, rhs5, inc5, s);
+  else if (w.ns == 3) launch_walk_ns<3, SA>(c, forward, w, g, alpha, rhs, inc, rhs5, inc5, s);
+  else launch_walk_ns<4, SA>(c, forward, w, g, alpha, rhs, inc, rhs5, inc5, s);
 }
 
 template <class T>
@@ -2953,34 +2635,8 @@ void launch_lusgs_sweep(dndsg_ctx* c, bool forward, double alpha, const double* 
   const std::vector<int64_t>& off = forward ? c->fwdOff : c->bwdOff;
   const int32_t* cells = forward ? c->fwdCells : c->bwdCells;
   const int nb = (int)off.size() - 1;
-  // many narrow levels: one block walks them all over records packed in parallel beforehand
-  // (a launch per level would cost more than the work)
-  if (c->lusgsOrder == 1 && (forward ? c->fwdPartMax : c->bwdPartMax) <= kRecMaxLevels && c->nfmax <= 4) {
-    const int64_t* od = forward ? c->fwdOffDev : c->bwdOffDev;
-    const int32_t* nf = forward ? c->fwdNbF : c->bwdNbF;
-    const int32_t* nj = forward ? c->fwdNbJ : c->bwdNbJ;
-    const int32_t* np = forward ? c->fwdNbP : c->bwdNbP;
-    const int32_t* pl = c->lusgsParts > 1 ? (forward ? c->fwdPartLev : c->bwdPartLev) : nullptr;
-    const int nblk = c->lusgsParts > 1 ? c->lusgsParts : 1;
-    SaView<T> none{};
-    LuMatF* rec = (LuMatF*)c->lusgsMat;
-    if (forward) {
-      k_lusgs_pack_mat<T, true, false><<<grid_for(c->N), kBlock, 0, s>>>(h, none, cells, nf, nj, np, c->N, alpha, c->Dinv,
-                                                                          rhs, inc, rec);
-      k_lusgs_levels_mat<T, true, false><<<nblk, mat_threads<false>(), mat_smem<false>(), s>>>(none, rec, od, nb, pl, inc,
-                                                                                              h.gamma - 1, c->flags);
-    } else {
-      k_lusgs_pack_mat<T, false, false><<<grid_for(c->N), kBlock, 0, s>>>(h, none, cells, nf, nj, np, c->N, alpha, c->Dinv,
-                                                                           rhs, inc, rec);
-      k_lusgs_levels_mat<T, false, false><<<nblk, mat_threads<false>(), mat_smem<false>(), s>>>(none, rec, od, nb, pl, inc,
-                                                                                               h.gamma - 1, c->flags);
-    }
-    return;
-  }
-  if (c->lusgsOrder == 1 && c->maxLevelWidth <= 8 * kLevelBlock) {
-    const int64_t* od = forward ? c->fwdOffDev : c->bwdOffDev;
-    if (forward) k_lusgs_levels<T, true><<<1, kLevelBlock, 0, s>>>(h, c->rankOf, cells, od, nb, alpha, c->Dinv, rhs, inc);
-    else k_lusgs_levels<T, false><<<1, kLevelBlock, 0, s>>>(h, c->rankOf, cells, od, nb, alpha, c->Dinv, rhs, inc);
+  if (c->lusgsOrder == 1) {
+    launch_walk<false>(c, forward, alpha, rhs, inc, nullptr, nullptr, s);
     return;
   }
   for (int k = 0; k < nb; k++) {
@@ -3226,20 +2882,6 @@ __global__ void __launch_bounds__(kBlock) k_lusgs_batch_sa(HotView<T> h, SaView<
   if (t < n) lusgs_cell_sa<T, FWD>(h, sa, rankOf, cells[t], alpha, Dinv, rhs, inc);
 }
 
-// all narrow levels of one sweep in one block (as k_lusgs_levels), 5 variables
-template <class T, bool FWD>
-__global__ void __launch_bounds__(kLevelBlock) k_lusgs_levels_sa(HotView<T> h, SaView<T> sa, const int32_t* rankOf,
-                                                                 const int32_t* cells, const int64_t* off, int nlev,
-                                                                 double alpha, const double* Dinv, const double* rhs,
-                                                                 double* inc) {
-  for (int l = 0; l < nlev; l++) {
-    const int64_t b = off[l], e = off[l + 1];
-    for (int64_t t = b + threadIdx.x; t < e; t += blockDim.x)
-      lusgs_cell_sa<T, FWD>(h, sa, rankOf, cells[t], alpha, Dinv, rhs, inc);
-    __syncthreads();
-  }
-}
-
 // the U5 diagonal: the flow one plus alpha * the source Jacobian (LUSGSMatrixInit), its inverse
 // for the sweeps and (DS, may be null) itself for LUSGSMatrixVec
 __global__ void k_sa_diag(int64_t N, const double* D, const double* srcJac, double alpha, double* DinvS, double* DS) {
@@ -3325,33 +2967,8 @@ void launch_lusgs_sweep_sa(dndsg_ctx* c, bool forward, double alpha, const doubl
   const std::vector<int64_t>& off = forward ? c->fwdOff : c->bwdOff;
   const int32_t* cells = forward ? c->fwdCells : c->bwdCells;
   const int nb = (int)off.size() - 1;
-  if (c->lusgsOrder == 1 && (forward ? c->fwdPartMax : c->bwdPartMax) <= kRecMaxLevels && c->nfmax <= 4) {
-    const int64_t* od = forward ? c->fwdOffDev : c->bwdOffDev;
-    const int32_t* nf = forward ? c->fwdNbF : c->bwdNbF;
-    const int32_t* nj = forward ? c->fwdNbJ : c->bwdNbJ;
-    const int32_t* np = forward ? c->fwdNbP : c->bwdNbP;
-    const int32_t* pl = c->lusgsParts > 1 ? (forward ? c->fwdPartLev : c->bwdPartLev) : nullptr;
-    const int nblk = c->lusgsParts > 1 ? c->lusgsParts : 1;
-    LuMatS* rec = (LuMatS*)c->lusgsMat;
-    if (forward) {
-      k_lusgs_pack_mat<T, true, true><<<grid_for(c->N), kBlock, 0, s>>>(h, sa, cells, nf, nj, np, c->N, alpha, c->Dinv,
-                                                                         rhs4, inc4, rec);
-      k_lusgs_levels_mat<T, true, true><<<nblk, mat_threads<true>(), mat_smem<true>(), s>>>(sa, rec, od, nb, pl, inc4,
-                                                                                           h.gamma - 1, c->flags);
-    } else {
-      k_lusgs_pack_mat<T, false, true><<<grid_for(c->N), kBlock, 0, s>>>(h, sa, cells, nf, nj, np, c->N, alpha, c->Dinv,
-                                                                          rhs4, inc4, rec);
-      k_lusgs_levels_mat<T, false, true><<<nblk, mat_threads<true>(), mat_smem<true>(), s>>>(sa, rec, od, nb, pl, inc4,
-                                                                                            h.gamma - 1, c->flags);
-    }
-    return;
-  }
-  if (c->lusgsOrder == 1) {  // many narrow levels: one block walks them all
-    const int64_t* od = forward ? c->fwdOffDev : c->bwdOffDev;
-    if (forward)
-      k_lusgs_levels_sa<T, true><<<1, kLevelBlock, 0, s>>>(h, sa, c->rankOf, cells, od, nb, alpha, c->Dinv, rhs4, inc4);
-    else
-      k_lusgs_levels_sa<T, false><<<1, kLevelBlock, 0, s>>>(h, sa, c->rankOf, cells, od, nb, alpha, c->Dinv, rhs4, inc4);
+  if (c->lusgsOrder == 1) {
+    launch_walk<true>(c, forward, alpha, rhs4, inc4, rhs5, inc5, s);
     return;
   }
   for (int k = 0; k < nb; k++) {

@@ -30,6 +30,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
   return done != 0;
 }
+// thread-block clusters: a shared-memory address of this block in block `rank`, and the hardware barrier of all threads of the cluster (release / acquire)
+__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// a store into another block's shared memory that adds its bytes to a barrier there
+__device__ __forceinline__ void st_async_f64(uint32_t addr, double v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr unsigned kFlagTimeout = 4u;
 
