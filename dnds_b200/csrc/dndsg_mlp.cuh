@@ -155,10 +155,16 @@ struct MlpDev {
 // (stride byte offset), so the K step k0 of an instruction starts 32 k0 / 16 bytes further.
 constexpr int kTcRows = 128;
 constexpr int kTcCols = 64;  // tensor-memory columns: the widest layer (N = 64, FP32)
+// The forward operands have K = 80: 64 inputs and 16 more columns, of which three carry the bias.  The
+// activation rows hold ones there and the weight rows the bias as three BF16 numbers that sum to it exactly
+// (24 bits), so the accumulator comes out with the bias in.  The weights and biases of the SiLU layers are
+// halved (exact): the accumulator is w = z / 2 and SiLU(z) = w + w tanh(w).  Per activation the epilogue is
+// then one special-function operation, one multiply-add and half a conversion, where it had three more
+// operations and a shared-memory load; it is what bounds this kernel.
+constexpr int kTcK = 80;
 struct TcSmem {
-  alignas(128) unsigned char W[4][kHid * 64 * 2];  // W1..W4 (W4: 32 rows used), core-matrix layout
-  alignas(128) unsigned char A[kTcRows * 64 * 2];  // the current layer's input rows, same layout
-  float b[3 * kHid + kOutP];
+  alignas(128) unsigned char W[3 * kHid * kTcK * 2 + kOutP * kTcK * 2];  // W1..W4, core-matrix layout
+  alignas(128) unsigned char A[kTcRows * kTcK * 2];                      // the current layer's input rows, same layout
   uint64_t bar;
   uint32_t tmem;
 };
@@ -166,6 +172,7 @@ struct TcSmem {
 // tensor memory: every resident CTA holds kTcCols of the SM's 512 columns, and an allocation that
 // cannot be met waits; the launch keeps at most 4 CTAs per SM (shared memory and registers allow 4)
 static_assert(sizeof(TcSmem) > 233472 / 9, "at most 8 CTAs of k_mlp_tc per SM");
+static_assert(4 * (sizeof(TcSmem) + 1024) <= 233472, "4 CTAs of k_mlp_tc per SM");
 
 // the bias of layer l, entry k, from the FP32 master parameters
 __device__ __forceinline__ float tc_bias_s(const float* P, int layer, int k) {
@@ -173,14 +180,22 @@ __device__ __forceinline__ float tc_bias_s(const float* P, int layer, int k) {
   return P[off + k];
 }
 
-// byte offset of element (row, k) of a 64-wide K-major operand in the core-matrix layout
+// byte offset of element (row, k) of a K-major operand in the core-matrix layout: 64 wide (training) and
+// kTcK wide (inference)
 __device__ __forceinline__ uint32_t cm_off(int row, int k) {
   return (uint32_t)((row >> 3) * 1024 + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
 }
-// shared-memory matrix descriptor: start address, leading byte offset 128, stride byte offset 1024,
-// descriptor version 1, no swizzle (all addresses and offsets in 16-byte units)
+__device__ __forceinline__ uint32_t cm_off_k(int row, int k) {
+  return (uint32_t)((row >> 3) * (kTcK * 16) + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
+}
+// shared-memory matrix descriptor: start address, leading byte offset 128, stride byte offset 1024 (kTcK
+// wide: 1280), descriptor version 1, no swizzle (all addresses and offsets in 16-byte units)
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
   return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         (1ull << 46);
+}
+__device__ __forceinline__ uint64_t umma_desc_k(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(kTcK * 16 >> 4) << 32) |
          (1ull << 46);
 }
 // instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both K-major, M = 128, N
@@ -212,60 +227,59 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
   for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[k]);
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// SiLU through the identity sigmoid(z) = (1 + tanh(z / 2)) / 2 with the hardware tanh: one
-// special-function operation per activation instead of an exponential and a reciprocal (the
-// special-function unit bounds this kernel's epilogue); its error (about 2^-11 relative) is below
-// the BF16 rounding the activation gets next
-__device__ __forceinline__ float silu_tanh(float z) {
+// SiLU(z) from w = z / 2 through sigmoid(z) = (1 + tanh(z / 2)) / 2 with the hardware tanh: one
+// special-function operation per activation instead of an exponential and a reciprocal; its error (about
+// 2^-11 relative) is below the BF16 rounding the activation gets next
+__device__ __forceinline__ float silu_half(float w) {
   float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * z));
-  return 0.5f * z * (1.0f + t);
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(w));
+  return fmaf(w, t, w);
 }
-
-constexpr int kTcRowsX = kTcRows;
-__device__ __forceinline__ uint32_t cm_off_x(int row, int k) { return cm_off(row, k); }
-
-// one 64-value row of the layer input, as BF16, into the operand buffer
-__device__ __forceinline__ void tc_store_row(unsigned char* A, int row, const float* x) {
-  for (int kc = 0; kc < 8; kc++) {
-    __nv_bfloat162 p[4];
-    for (int e = 0; e < 4; e++) p[e] = __floats2bfloat162_rn(x[8 * kc + 2 * e], x[8 * kc + 2 * e + 1]);
-    *reinterpret_cast<uint4*>(A + cm_off(row, 8 * kc)) = *reinterpret_cast<uint4*>(p);
-  }
+__device__ __forceinline__ uint4 pack8(const float* x) {
+  __nv_bfloat162 p[4];
+  for (int e = 0; e < 4; e++) p[e] = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
+  return *reinterpret_cast<uint4*>(p);
 }
 
 // inputs and outputs of the tensor-core forward
-// Src::kTile: the whole tile is loaded by the CTA together (coalesced), else row by row;
-// Dst::kTile: the outputs go through shared memory and leave as one contiguous block
+// Src::kTile: the whole tile is loaded by the CTA together (coalesced), a tile ahead; else row by row
 struct TcFeaturesX {  // given features X [n][64]
   static constexpr bool kTile = true;
   const float* X;
-  // the 128 x 64 tile starting at row r0 into the operand buffer, 32 B of X per thread and step
-  __device__ void load_tile(int64_t r0, int64_t n, unsigned char* A) const {
-    for (int e = threadIdx.x; e < kTcRowsX * 8; e += blockDim.x) {
-      const int row = e >> 3, kc = e & 7;
-      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  // this thread's sixteenth of the 128 x 64 tile starting at row r0: 32 B of X per step
+  __device__ void fetch_tile(int64_t r0, int64_t n, float4 v[16]) const {
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const int e = threadIdx.x + j * kTcRows, row = e >> 3, kc = e & 7;
+      v[2 * j] = v[2 * j + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (r0 + row < n) {
         const float4* q = reinterpret_cast<const float4*>(X + (r0 + row) * kIn + 8 * kc);
-        const float4 a = q[0], b = q[1];
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        v[2 * j] = q[0];
+        v[2 * j + 1] = q[1];
       }
-      __nv_bfloat162 p[4];
-      for (int j = 0; j < 4; j++) p[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-      *reinterpret_cast<uint4*>(A + cm_off_x(row, 8 * kc)) = *reinterpret_cast<uint4*>(p);
+    }
+  }
+  __device__ void put_tile(const float4 v[16], unsigned char* A) const {
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const int e = threadIdx.x + j * kTcRows;
+      *reinterpret_cast<uint4*>(A + cm_off_k(e >> 3, 8 * (e & 7))) = pack8(&v[2 * j].x);
     }
   }
   __device__ void load(int64_t, int64_t, float*, float*) const {}
 };
 struct TcOutY {  // Y [n][20] = the network output
-  static constexpr bool kTile = true;
   float* Y;
-  // stage [128][20] FP32 (in the free operand buffer) -> one contiguous store of the tile
-  __device__ void store_tile(int64_t r0, int64_t n, const float* stage) const {
-    const int64_t m = min((int64_t)kTcRowsX, n - r0) * kOut;
-    for (int64_t e = threadIdx.x; e < m; e += blockDim.x) Y[r0 * kOut + e] = stage[e];
+  __device__ void store(int64_t r, int64_t n, const float* y, const float*) const {
+    if (r >= n) return;
+    float* o = Y + r * kOut;
+    if ((reinterpret_cast<uintptr_t>(Y) & 15u) == 0) {
+#pragma unroll
+      for (int k = 0; k < kOut; k += 4) *reinterpret_cast<float4*>(o + k) = make_float4(y[k], y[k + 1], y[k + 2], y[k + 3]);
+    } else {
+      for (int k = 0; k < kOut; k++) o[k] = y[k];
+    }
   }
-  __device__ void store(int64_t, int64_t, const float*, const float*) const {}
 };
 template <class T, int MODE>
 struct TcCellFeatures {  // the warm-start features of cell r (MODE 0: Jacobi extrapolation, 1: previous coefficients)
@@ -281,37 +295,53 @@ struct TcCellFeatures {  // the warm-start features of cell r (MODE 0: Jacobi ex
       for (int v = 0; v < 4; v++) sc[v] = 0.f;
     }
   }
-  __device__ void load_tile(int64_t, int64_t, unsigned char*) const {}
+  __device__ void fetch_tile(int64_t, int64_t, float4*) const {}
+  __device__ void put_tile(const float4*, unsigned char*) const {}
 };
 template <class T>
 struct TcWarmStart {  // dst = base + y r (base: x2 for MODE 0, x0 for MODE 1)
-  static constexpr bool kTile = false;
   const T* x2;
   T* dst;
   __device__ void store(int64_t r, int64_t n, const float* y, const float* sc) const {
     if (r < n)
       for (int o = 0; o < kOut; o++) dst[r * 20 + o] = (T)((double)x2[r * 20 + o] + (double)y[o] * (double)sc[o & 3]);
   }
-  __device__ void store_tile(int64_t, int64_t, const float*) const {}
 };
 
 template <class Src, class Dst>
-__global__ void __launch_bounds__(kTcRows) k_mlp_tc(MlpDev m, Src src, Dst dst, int64_t n, unsigned* flags) {
+__global__ void __launch_bounds__(kTcRows, 4) k_mlp_tc(MlpDev m, Src src, Dst dst, int64_t n, unsigned* flags) {
   extern __shared__ __align__(128) unsigned char raw[];
   TcSmem& S = *reinterpret_cast<TcSmem*>(raw);
   const int tid = threadIdx.x, warp = tid >> 5;
-  // the weights (row-major [N][64] BF16 in global memory) into the core-matrix layout, 16 B at a time
+  // the weights (row-major [N][64] BF16 in global memory) into the core-matrix layout, 16 B at a time, halved in
+  // front of a SiLU; then the bias columns
+  constexpr int kLayerBytes = kHid * kTcK * 2;
   for (int e = tid; e < (3 * kHid + kOutP) * 8; e += blockDim.x) {
     const int row = e >> 3, kc = e & 7;
     const int layer = row < 3 * kHid ? row / kHid : 3, rl = row - layer * kHid;
     const int woff = layer == 0 ? kWOff1 : layer == 1 ? kWOff2 : layer == 2 ? kWOff3 : kWOff4;
-    *reinterpret_cast<uint4*>(S.W[layer] + cm_off(rl, 8 * kc)) =
-        *reinterpret_cast<const uint4*>(m.W + woff + rl * 64 + 8 * kc);
+    uint4 q = *reinterpret_cast<const uint4*>(m.W + woff + rl * 64 + 8 * kc);
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+    if (layer < 3)
+      for (int k = 0; k < 4; k++) h[k] = __hmul2(h[k], __float2bfloat162_rn(0.5f));
+    *reinterpret_cast<uint4*>(S.W + layer * kLayerBytes + cm_off_k(rl, 8 * kc)) = q;
   }
-  for (int e = tid; e < 3 * kHid + kOutP; e += blockDim.x) {
-    const int off = e < kHid ? kOffB1 + e : e < 2 * kHid ? kOffB2 + e - kHid : e < 3 * kHid ? kOffB3 + e - 2 * kHid
-                                                                                          : kOffB4 + e - 3 * kHid;
-    S.b[e] = m.P[off];
+  for (int row = tid; row < 3 * kHid + kOutP; row += blockDim.x) {
+    const int layer = row < 3 * kHid ? row / kHid : 3, rl = row - layer * kHid;
+    float bias = tc_bias_s(m.P, layer, rl) * (layer < 3 ? 0.5f : 1.0f);
+    float c[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int k = 0; k < 3; k++) {
+      c[k] = __bfloat162float(__float2bfloat16(bias));
+      bias -= c[k];
+    }
+    unsigned char* w = S.W + layer * kLayerBytes;
+    *reinterpret_cast<uint4*>(w + cm_off_k(rl, 64)) = pack8(c);
+    *reinterpret_cast<uint4*>(w + cm_off_k(rl, 72)) = make_uint4(0, 0, 0, 0);
+  }
+  {
+    const float ones[8] = {1.f, 1.f, 1.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    *reinterpret_cast<uint4*>(S.A + cm_off_k(tid, 64)) = pack8(ones);
+    *reinterpret_cast<uint4*>(S.A + cm_off_k(tid, 72)) = make_uint4(0, 0, 0, 0);
   }
   const uint32_t bar = smem_u32(&S.bar);
   if (warp == 0) {
@@ -328,68 +358,64 @@ __global__ void __launch_bounds__(kTcRows) k_mlp_tc(MlpDev m, Src src, Dst dst, 
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = S.tmem, trow = tbase + ((uint32_t)(warp * 32) << 16);
-  const uint32_t aAddr = smem_u32(S.A);
+  const uint32_t aAddr = smem_u32(S.A), wAddr = smem_u32(S.W);
   uint32_t phase = 0;
-  bool failed = false;
-  for (int64_t tile = blockIdx.x; tile * kTcRows < n && !failed; tile += gridDim.x) {
+  bool failed = false, stop = false;
+  float4 next[16];
+  if constexpr (Src::kTile) src.fetch_tile((int64_t)blockIdx.x * kTcRows, n, next);
+  for (int64_t tile = blockIdx.x; tile * kTcRows < n && !stop; tile += gridDim.x) {
     const int64_t r = tile * kTcRows + tid;
-    float x[kInP], sc[4] = {0.f, 0.f, 0.f, 0.f};
+    float sc[4] = {0.f, 0.f, 0.f, 0.f};
     if constexpr (Src::kTile) {
-      src.load_tile(tile * kTcRows, n, S.A);
+      src.put_tile(next, S.A);
     } else {
+      float x[kInP];
       src.load(r, n, x, sc);
-      tc_store_row(S.A, tid, x);
+      for (int kc = 0; kc < 8; kc++) *reinterpret_cast<uint4*>(S.A + cm_off_k(tid, 8 * kc)) = pack8(x + 8 * kc);
     }
-    for (int layer = 0; layer < 4 && !failed; layer++) {
-      const int N = layer < 3 ? kHid : kOutP;
+#pragma unroll
+    for (int layer = 0; layer < 4; layer++) {
       proxy_fence_smem();  // the operand rows written by this thread, to the tensor cores
-      tc_fence_before();
-      __syncthreads();
+      tc_fence_before();   // and its accumulator reads, before the next product
+      stop = __syncthreads_or(failed);
+      if (stop) break;
       if (tid == 0) {
         tc_fence_after();
-        const uint32_t wAddr = smem_u32(S.W[layer]);
-        for (int ks = 0; ks < 4; ks++)
-          umma_bf16(tbase, umma_desc(aAddr + 256 * ks), umma_desc(wAddr + 256 * ks), layer < 3 ? umma_idesc(kHid)
-                                                                                              : umma_idesc(kOutP),
-                    ks > 0);
+        for (int ks = 0; ks < kTcK / 16; ks++)
+          umma_bf16(tbase, umma_desc_k(aAddr + 256 * ks), umma_desc_k(wAddr + layer * kLayerBytes + 256 * ks),
+                    layer < 3 ? umma_idesc(kHid) : umma_idesc(kOutP), ks > 0);
         umma_commit(bar);
       }
-      const bool ok = mbar_wait(bar, phase, kWaitLimit);
+      if constexpr (Src::kTile)
+        if (layer == 2) src.fetch_tile((tile + gridDim.x) * kTcRows, n, next);
+      failed = !mbar_wait(bar, phase, kWaitLimit);
       phase ^= 1u;
-      if (__syncthreads_or(!ok)) {
-        failed = true;
-        break;
-      }
       tc_fence_after();
-      float z[64];
-      for (int c0 = 0; c0 < N; c0 += 16) tmem_ld16(trow + c0, z + c0);
-      tmem_wait_ld();
       if (layer < 3) {
-        for (int k = 0; k < 64; k++) x[k] = silu_tanh(z[k] + S.b[layer * kHid + k]);
-        tc_store_row(S.A, tid, x);
-      } else {
-        float y[kOut];
-        for (int o = 0; o < kOut; o++) y[o] = z[o] + S.b[3 * kHid + o];
-        if constexpr (Dst::kTile) {  // the operand buffer is free once the last product completed
-          float* stage = reinterpret_cast<float*>(S.A);
-          for (int o = 0; o < kOut; o++) stage[tid * kOut + o] = y[o];
-          __syncthreads();
-          dst.store_tile(tile * kTcRows, n, stage);
-        } else {
-          dst.store(r, n, y, sc);
+#pragma unroll
+        for (int c0 = 0; c0 < kHid; c0 += 32) {
+          float z[32];
+          tmem_ld16(trow + c0, z);
+          tmem_ld16(trow + c0 + 16, z + 16);
+          tmem_wait_ld();
+          for (int k = 0; k < 32; k++) z[k] = silu_half(z[k]);
+          for (int kc = 0; kc < 4; kc++) *reinterpret_cast<uint4*>(S.A + cm_off_k(tid, c0 + 8 * kc)) = pack8(z + 8 * kc);
         }
+      } else {
+        float z[32];
+        tmem_ld16(trow, z);
+        tmem_ld16(trow + 16, z + 16);
+        tmem_wait_ld();
+        if (!failed) dst.store(r, n, z, sc);
       }
     }
-    tc_fence_before();
-    __syncthreads();  // every row is read out before the next tile's products overwrite the accumulator
-    tc_fence_after();
   }
-  if (failed && tid == 0) {
-    atomicOr(flags, kFlagTimeout);
-    mbar_wait(bar, phase ^ 1u, kWaitLimit);  // the last commit, if it is still in flight
-  }
+  if (failed) atomicOr(flags, kFlagTimeout);
   tc_fence_before();
-  __syncthreads();
+  if (__syncthreads_or(failed)) {  // the last commit may still be in flight
+    if (tid == 0) mbar_wait(bar, phase ^ 1u, kWaitLimit);
+    __syncthreads();
+  }
   if (warp == 0) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(kTcCols) : "memory");
