@@ -634,6 +634,7 @@ HotView<T> view(dndsg_ctx* c) {
   h.relax = c->s.jacobi_relax;
   h.faceGrad = (const T*)c->faceGrad;
   h.mu = c->s.mu_gas; h.cp = c->s.cp_gas; h.pr = c->s.pr_gas; h.tRef = c->s.t_ref; h.cSuth = c->s.c_sutherland;
+  if (h.mu > 0) gas_constants(h);
   return h;
 }
 

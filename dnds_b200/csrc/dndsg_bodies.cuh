@@ -300,7 +300,21 @@ struct HotView {
   // AoSoA E = 60: [side][gp][d/dx, d/dy][5], and the gas properties
   const T* faceGrad;
   double mu, cp, pr, tRef, cSuth;
+  // quotients of these that every point would form again
+  double kT;     // gamma / ((gamma - 1) cp): T = kT p / rho
+  double iTRef;  // 1 / tRef
+  double muS;    // mu (tRef + cSuth)
+  double cpPr;   // cp / pr
+  double iMu;    // 1 / mu
 };
+template <class T>
+DG_HD void gas_constants(HotView<T>& h) {
+  h.kT = h.gamma / ((h.gamma - 1) * h.cp);
+  h.iTRef = 1.0 / h.tRef;
+  h.muS = h.mu * (h.tRef + h.cSuth);
+  h.cpPr = h.cp / h.pr;
+  h.iMu = 1.0 / h.mu;
+}
 
 template <class T>
 DG_HD void load4(const double* p, double* v) {
@@ -541,18 +555,18 @@ DG_HD int face_flux(int64_t f, const HotView<T>& h, double t, double out[4], boo
   return nred;
 }
 
-// Sutherland's law at a state (fluxFace, DNDS_FV_EulerEvaluator.hpp:405-412): T = p / ((gamma-1)/gamma Cp rho)
+// Sutherland's law at a state (fluxFace, DNDS_FV_EulerEvaluator.hpp:405-412): T = p / ((gamma-1)/gamma Cp rho),
+// mu (T / TRef)^1.5 (TRef + C) / (T + C); ir = 1 / rho
 template <class T>
-DG_HD double sutherland_mu(const HotView<T>& h, double p, double rho) {
-  const double Tm = p / ((h.gamma - 1) / h.gamma * h.cp * rho);
-  return h.mu * pow(Tm / h.tRef, 1.5) * (h.tRef + h.cSuth) / (Tm + h.cSuth);
+DG_HD double sutherland_mu(const HotView<T>& h, double p, double ir) {
+  const double Tm = p * ir * h.kT, x = Tm * h.iTRef;
+  return h.muS * (x * sqrt(x)) / (Tm + h.cSuth);
 }
 
 // Gas::ViscousFlux_IdealGas (DNDS_Gas.hpp:795-826), 2-D, contracted with the unit normal;
-// G[i][v] = d U_v / d x_i of the conservative variables
-DG_HD void viscous_flux_n(const double U[4], const double G[2][4], double nx, double ny, bool adiabatic,
-                          double gamma, double mu, double k, double cp, double Fn[4]) {
-  const double ir = 1.0 / U[0];
+// G[i][v] = d U_v / d x_i of the conservative variables, ir = 1 / U[0], kT = gamma / ((gamma - 1) cp)
+DG_HD void viscous_flux_n(const double U[4], double ir, const double G[2][4], double nx, double ny, bool adiabatic,
+                          double gamma, double kT, double mu, double k, double Fn[4]) {
   const double v0 = U[1] * ir, v1 = U[2] * ir;
   double S[2][2];  // d u_j / d x_i
   for (int i = 0; i < 2; i++)
@@ -561,7 +575,7 @@ DG_HD void viscous_flux_n(const double U[4], const double G[2][4], double nx, do
   double gT[2];
   for (int i = 0; i < 2; i++) {
     const double gP = (gamma - 1) * (G[i][3] - 0.5 * (G[i][1] * v0 + G[i][2] * v1 + S[i][0] * U[1] + S[i][1] * U[2]));
-    gT[i] = gamma / ((gamma - 1) * cp * U[0] * U[0]) * (U[0] * gP - p * G[i][0]);
+    gT[i] = kT * (ir * ir) * (U[0] * gP - p * G[i][0]);
   }
   if (adiabatic) {
     const double d = gT[0] * nx + gT[1] * ny;
@@ -631,9 +645,10 @@ DG_HD int face_flux_vis(int64_t f, const HotView<T>& h, double t, double out[4],
       G[1][v] = 0.5 * (GL[1][v] + (inner ? GR[1][v] : GL[1][v])) + jump * ny;
       Um[v] = 0.5 * (UL[v] + UR[v]);
     }
-    const double pm = (h.gamma - 1) * (Um[3] - 0.5 * (Um[1] * Um[1] + Um[2] * Um[2]) / Um[0]);
-    const double mu = sutherland_mu(h, pm, Um[0]);
-    viscous_flux_n(Um, G, nx, ny, bc == BC_WALL_NOSLIP, h.gamma, mu, h.cp * mu / h.pr, h.cp, Fv);
+    const double irm = 1.0 / Um[0];
+    const double pm = (h.gamma - 1) * (Um[3] - 0.5 * (Um[1] * Um[1] + Um[2] * Um[2]) * irm);
+    const double mu = sutherland_mu(h, pm, irm);
+    viscous_flux_n(Um, irm, G, nx, ny, bc == BC_WALL_NOSLIP, h.gamma, h.kT, mu, h.cpPr * mu, Fv);
     const double jw = 0.5 * area * l3_weight(g);
     for (int k = 0; k < 4; k++) acc[k] -= (F[k] - Fv[k]) * jw;
   }
@@ -923,7 +938,8 @@ DG_HD void dt_face(int64_t f, const HotView<T>& h) {
   const double pMean = (pL + pR) * 0.5;
   double lam = fabs(vn) + sqrt(h.gamma * pMean / rhoMean);
   if (h.mu > 0) {  // viscous part (DNDS_FV_EulerEvaluator.cpp:80-99)
-    const double lamVis = sutherland_mu(h, pMean, rhoMean) / rhoMean * dmax(4. / 3., h.gamma / h.pr);
+    const double irm = 1.0 / rhoMean;
+    const double lamVis = sutherland_mu(h, pMean, irm) * irm * dmax(4. / 3., h.gamma / h.pr);
     lam += lamVis * area * (1.0 / h.vol[L] + 1.0 / (R >= 0 ? h.vol[R] : h.vol[L]));
   }
   h.lamA[f] = lam * area;

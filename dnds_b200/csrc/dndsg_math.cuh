@@ -82,7 +82,9 @@ DG_HD double rsqrt_of(double x) {
 
 // Roe flux with the Harten-Yee entropy fix, normal frame
 // (Gas::RoeFlux_IdealGas_HartenYee<2,0>, DNDS_Gas.hpp:406-654)
-DG_HD void roe_flux(const double* UL, const double* UR, double gamma, double dLambda, double* F) {
+// vel (may be null): the normal velocities of both sides and the Roe average's magnitude, the upwind speed
+// of a transported scalar
+DG_HD void roe_flux(const double* UL, const double* UR, double gamma, double dLambda, double* F, double* vel = nullptr) {
   const double scaleHY = 0.05, g1 = gamma - 1.0;
   const double iLR = 1.0 / (UL[0] * UR[0]), irL = iLR * UR[0], irR = iLR * UL[0];
   const double uL = UL[1] * irL, vL = UL[2] * irL, uR = UR[1] * irR, vR = UR[2] * irR;
@@ -90,6 +92,7 @@ DG_HD void roe_flux(const double* UL, const double* UR, double gamma, double dLa
   const double HL = (UL[3] + pL) * irL, HR = (UR[3] + pR) * irR;
   const double q = sqrt(UR[0] * irL), i1 = 1.0 / (1.0 + q);
   const double u = (uL + q * uR) * i1, v = (vL + q * vR) * i1;
+  if (vel) { vel[0] = uL; vel[1] = uR; vel[2] = fabs(u); }
   const double vs = u * u + v * v;
   const double H = (HL + q * HR) * i1;
   const double a2 = g1 * (H - 0.5 * vs);
@@ -117,12 +120,14 @@ DG_HD void roe_flux(const double* UL, const double* UR, double gamma, double dLa
 }
 
 // HLLC flux (Gas::HLLCFlux_IdealGas_HartenYee<2>, DNDS_Gas.hpp:312-403)
-DG_HD void hllc_flux(const double* UL, const double* UR, double gamma, double* F) {
+// vel (may be null): the normal velocities of both sides and the magnitude of their mean
+DG_HD void hllc_flux(const double* UL, const double* UR, double gamma, double* F, double* vel = nullptr) {
   const double g1 = gamma - 1.0;
   const double iLR = 1.0 / (UL[0] * UR[0]), irL = iLR * UR[0], irR = iLR * UL[0];
   const double uL = UL[1] * irL, vL = UL[2] * irL, uR = UR[1] * irR, vR = UR[2] * irR;
   const double pL = g1 * (UL[3] - UL[0] * 0.5 * (uL * uL + vL * vL)), pR = g1 * (UR[3] - UR[0] * 0.5 * (uR * uR + vR * vR));
   const double q = sqrt(UR[0] * irL), i1 = 1.0 / (1.0 + q);
+  if (vel) { vel[0] = uL; vel[1] = uR; vel[2] = fabs(uL + uR) * 0.5; }
   const double u = (uL + q * uR) * i1;
   const double dsqr = gamma * (pL * irL + q * (pR * irR)) * i1 + 0.5 * q * (i1 * i1) * sq(uR - uL);
   const double sd = sqrt(dsqr), SL = u - sd, SR = u + sd;

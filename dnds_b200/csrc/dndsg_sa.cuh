@@ -17,6 +17,7 @@
 
 namespace dg {
 
+constexpr double kWallFar = 2.5873402367724347e+33;  // (3e200)^(1/6), the reference's largest wall distance
 constexpr int kSaGp = 9;       // cell quadrature points per cell (QUAD_9; TRI_4 pads with zero weights)
 constexpr int kSaGpE = 16;     // per point: weight x det J, value row (5), d/dx row (5), d/dy row (5)
 
@@ -36,10 +37,10 @@ struct SaView {
   double far5;           // farFieldStaticValue[4]
 };
 
-// SA eddy-viscosity factor (fluxFace, DNDS_FV_EulerEvaluator.hpp:413-425, SA-neg softening below 10)
-DG_HD double sa_mu_factor(double U5, double muRef, double mufPhy) {
+// SA eddy-viscosity factor (fluxFace, DNDS_FV_EulerEvaluator.hpp:413-425, SA-neg softening below 10) at
+// Chi = U5 muRef / mu
+DG_HD double sa_mu_factor(double Chi) {
   const double cnu1 = 7.1;
-  double Chi = U5 * muRef / mufPhy;
   if (Chi < 10) Chi = 0.05 * log(1 + exp(20 * Chi));
   const double Chi3 = Chi * Chi * Chi;
   const double fnu1 = Chi3 / (Chi3 + cnu1 * cnu1 * cnu1);
@@ -98,7 +99,7 @@ DG_HD void setup_sa_cell_gp(int64_t i, const CellSetup* cells, double* gp) {
 
 // first-order wall distance: from the cell barycentre to the nearest wall segment [nw][4]
 DG_HD double sa_wall_distance(double px, double py, const double* seg, int64_t nw) {
-  double best = pow(3e200, 1. / 6.);
+  double best = kWallFar;
   for (int64_t s = 0; s < nw; s++) {
     const double x1 = seg[4 * s], y1 = seg[4 * s + 1], x2 = seg[4 * s + 2], y2 = seg[4 * s + 3];
     const double ex = x2 - x1, ey = y2 - y1, L2 = sqrt(ex * ex + ey * ey);
@@ -266,17 +267,11 @@ DG_HD int face_flux_sa_point(int64_t f, int g, const HotView<T>& h, const SaView
     to_normal_frame(UL, nx, ny, a);
     to_normal_frame(UR, nx, ny, b);
     if (!(a[0] > 0 && b[0] > 0)) bad = true;
-    if (RIEMANN == 2) hllc_flux(a, b, h.gamma, F);
-    else roe_flux(a, b, h.gamma, dl, F);
+    double vel[3];  // both sides' normal velocities, the upwind speed
+    if (RIEMANN == 2) hllc_flux(a, b, h.gamma, F, vel);
+    else roe_flux(a, b, h.gamma, dl, F, vel);
     from_normal_frame(F, nx, ny);
-    double lam123;
-    if (RIEMANN == 2) {
-      lam123 = fabs(a[1] / a[0] + b[1] / b[0]) * 0.5;
-    } else {
-      const double qL = sqrt(a[0]), qR = sqrt(b[0]);
-      lam123 = fabs((qL * a[1] / a[0] + qR * b[1] / b[0]) / (qL + qR));
-    }
-    double FS = ((a[1] / a[0] * sL + b[1] / b[0] * sR) - (sR - sL) * lam123) * 0.5;
+    const double FS = ((vel[0] * sL + vel[1] * sR) - (sR - sL) * vel[2]) * 0.5;
     // gradients of the 5 variables at the point
     double GL[2][4], GR[2][4], G[2][4], Um[4], Fv[4], gS[2];
     face_grad(f, 0, g, L, h, GL);
@@ -298,23 +293,21 @@ DG_HD int face_flux_sa_point(int64_t f, int g, const HotView<T>& h, const SaView
     gS[0] = 0.5 * (gSL[0] + (inner ? gSR[0] : gSL[0])) + jS * nx;
     gS[1] = 0.5 * (gSL[1] + (inner ? gSR[1] : gSL[1])) + jS * ny;
     const double Sm = 0.5 * (sL + sR);
-    const double pm = (h.gamma - 1) * (Um[3] - 0.5 * (Um[1] * Um[1] + Um[2] * Um[2]) / Um[0]);
-    const double mufPhy = sutherland_mu(h, pm, Um[0]);
-    const double muf = mufPhy * sa_mu_factor(Sm, muRef, mufPhy);
-    const double kc = h.cp * (muf - mufPhy) / 0.9 + h.cp * mufPhy / h.pr;
-    viscous_flux_n(Um, G, nx, ny, bc == BC_WALL_NOSLIP, h.gamma, muf, kc, h.cp, Fv);
-    // the U5 diffusion (DNDS_FV_EulerEvaluator.hpp:463-480)
+    const double irm = 1.0 / Um[0];
+    const double pm = (h.gamma - 1) * (Um[3] - 0.5 * (Um[1] * Um[1] + Um[2] * Um[2]) * irm);
+    const double mufPhy = sutherland_mu(h, pm, irm);
+    const double Chi = Sm * muRef / mufPhy;
+    const double muf = mufPhy * sa_mu_factor(Chi);
+    const double kc = h.cp * (muf - mufPhy) * (1.0 / 0.9) + h.cpPr * mufPhy;
+    viscous_flux_n(Um, irm, G, nx, ny, bc == BC_WALL_NOSLIP, h.gamma, h.kT, muf, kc, Fv);
+    // the U5 diffusion (DNDS_FV_EulerEvaluator.hpp:463-480), 1 / sigma = 1.5
     double fn = 1;
     if (Sm < 0) {
-      const double Chi = Sm * muRef / mufPhy, cn1 = 16;
-      fn = (cn1 + Chi * Chi * Chi) / (cn1 - Chi * Chi * Chi);
+      const double cn1 = 16, Chi3 = Chi * Chi * Chi;
+      fn = (cn1 + Chi3) / (cn1 - Chi3);
     }
-    double FvS = 0;
-    const double gn[2] = {nx, ny};
-    for (int d = 0; d < 2; d++) {
-      const double diffNu = (gS[d] * muRef - Sm * muRef / Um[0] * G[d][0]) / Um[0];
-      FvS += gn[d] * diffNu * (mufPhy + Sm * muRef * fn) / (2. / 3.) / muRef;
-    }
+    const double gnS = nx * (gS[0] - Sm * irm * G[0][0]) + ny * (gS[1] - Sm * irm * G[1][0]);
+    const double FvS = gnS * irm * (mufPhy + Sm * muRef * fn) * 1.5;
     const double jw = 0.5 * area * l3_weight(g);
     for (int k = 0; k < 4; k++) c[k] = (F[k] - Fv[k]) * jw;
     cS = (FS - FvS) * jw;
@@ -323,55 +316,58 @@ DG_HD int face_flux_sa_point(int64_t f, int g, const HotView<T>& h, const SaView
 }
 
 // the SA source and its diagonal Jacobian at one point (source / sourceJacobianDiag for NS_SA,
-// DNDS_FV_EulerEvaluator.hpp:593-864, USE_NS_SA_NEGATIVE_MODEL)
+// DNDS_FV_EulerEvaluator.hpp:593-864, USE_NS_SA_NEGATIVE_MODEL).  Bound by its FP64 instructions, so one
+// quotient each for 1 / rho and 1 / d, the sixth root as sqrt(cbrt()), Sutherland's power as x sqrt(x):
+// 75 -> 56 us for the source of 65,536 quads, 784 -> 738 us per RANS-SA iteration (16 parts 438 -> 397)
 template <class T>
 DG_HD void sa_source_point(const HotView<T>& h, const double U[4], double U5, const double G[2][4],
                            const double gS[2], double dWall, double& src, double& jac) {
-  const double d = dmin(dWall, pow(3e200, 1. / 6.));
+  const double d = dmin(dWall, kWallFar);
   const double cb1 = 0.1355, cb2 = 0.622, sigma = 2. / 3., cnu1 = 7.1, cnu2 = 0.7, cnu3 = 0.9, cw2 = 0.3, cw3 = 2,
                kappa = 0.41, rlim = 10, ct3 = 1.2, ct4 = 0.5;
   const double cw1 = cb1 / (kappa * kappa) + (1 + cb2) / sigma;
-  const double p = (h.gamma - 1) * (U[3] - 0.5 * (U[1] * U[1] + U[2] * U[2]) / U[0]);
+  const double ir = 1.0 / U[0], id = 1.0 / d;
+  const double p = (h.gamma - 1) * (U[3] - 0.5 * (U[1] * U[1] + U[2] * U[2]) * ir);
   const double muRef = h.mu;
-  const double nuh = U5 * muRef / U[0];
-  const double mufPhy = sutherland_mu(h, p, U[0]);
+  const double nuh = U5 * muRef * ir;
+  const double mufPhy = sutherland_mu(h, p, ir);
   const double Chi = U5 * muRef / mufPhy;
   const double Chi3 = Chi * Chi * Chi;
   const double fnu1 = Chi3 / (Chi3 + cnu1 * cnu1 * cnu1);
   const double fnu2 = 1 - Chi / (1 + Chi * fnu1);
-  const double vx = U[1] / U[0], vy = U[2] / U[0];
+  const double vx = U[1] * ir, vy = U[2] * ir;
   double diffNu[2], diffRho[2];
   for (int i = 0; i < 2; i++) {
     diffRho[i] = G[i][0];
-    diffNu[i] = (gS[i] * muRef - nuh * G[i][0]) / U[0];
+    diffNu[i] = (gS[i] * muRef - nuh * G[i][0]) * ir;
   }
   // diffU[i][j] = d u_j / d x_i; Omega = (diffU^T - diffU) / 2, S = |Omega|_F sqrt 2
-  const double d10 = (G[1][1] - G[1][0] * vx) / U[0], d01 = (G[0][2] - G[0][0] * vy) / U[0];
-  const double w01 = 0.5 * (d10 - d01);
-  const double S = sqrt(2 * w01 * w01) * sqrt(2.0);
-  const double Sbar = nuh / (kappa * kappa * d * d) * fnu2;
+  const double d10 = (G[1][1] - G[1][0] * vx) * ir, d01 = (G[0][2] - G[0][0] * vy) * ir;
+  const double S = fabs(d10 - d01);
+  const double nd = nuh * id;
+  const double Sbar = nd * id * (1.0 / (kappa * kappa)) * fnu2;
   double Sh;
   if (Sbar < -cnu2 * S) Sh = S + S * (cnu2 * cnu2 * S + cnu3 * Sbar) / ((cnu3 - 2 * cnu2) * S - Sbar);
   else Sh = S + Sbar;
   const double r = dmin(nuh / (Sh * (kappa * d) * (kappa * d) + 1e-200), rlim);
-  const double r6 = r * r * r * r * r * r;
-  const double g = r + cw2 * (r6 - r);
-  const double g6 = g * g * g * g * g * g, c6 = cw3 * cw3 * cw3 * cw3 * cw3 * cw3;
-  const double fw = g * pow((1 + c6) / (g6 + c6), 1. / 6.);
+  const double r3 = r * r * r;
+  const double g = r + cw2 * (r3 * r3 - r);
+  const double g3 = g * g * g, c6 = cw3 * cw3 * cw3 * cw3 * cw3 * cw3;
+  const double fw = g * sqrt(cbrt((1 + c6) / (g3 * g3 + c6)));  // the sixth root
   const double ft2 = ct3 * exp(-ct4 * Chi * Chi);
-  double D = (cw1 * fw - cb1 / (kappa * kappa) * ft2) * (nuh / d) * (nuh / d);
+  double D = (cw1 * fw - cb1 / (kappa * kappa) * ft2) * nd * nd;
   double P = cb1 * (1 - ft2) * Sh * nuh;
   double fn = 1;
   if (U5 < 0) {
     const double cn1 = 16;
     fn = (cn1 + Chi3) / (cn1 - Chi3);
     P = cb1 * (1 - ct3) * S * nuh;
-    D = -cw1 * (nuh / d) * (nuh / d);
+    D = -cw1 * nd * nd;
   }
   const double dn2 = diffNu[0] * diffNu[0] + diffNu[1] * diffNu[1];
   const double rn = diffRho[0] * diffNu[0] + diffRho[1] * diffNu[1];
-  src = U[0] * (P - D + dn2 * cb2 / sigma) / muRef - (U5 * fn * muRef + mufPhy) / (U[0] * sigma) * rn / muRef;
-  jac = -dmin(U[0] * (P * 0 - D * 2) / muRef / (U5 + 1e-200), -1e-200);
+  src = U[0] * (P - D + dn2 * (cb2 / sigma)) * h.iMu - (U5 * fn * muRef + mufPhy) * ir * (1 / sigma) * rn * h.iMu;
+  jac = -dmin(U[0] * (P * 0 - D * 2) * h.iMu / (U5 + 1e-200), -1e-200);
 }
 
 // the SA source and its Jacobian at cell quadrature point ig of cell i, times the point's weight
@@ -387,10 +383,14 @@ DG_HD void sa_cell_point(int64_t i, int ig, const HotView<T>& h, const SaView<T>
   const T* rc = &h.urec[i * 20];
   const T* rs = &sa.urec[i * 5];
   double inc[4] = {0, 0, 0, 0}, G[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, incS = 0, gS[2] = {0, 0};
+  double row[kSaGpE];
+  for (int e = 0; e < kSaGpE; e += 4) load4<double>(gp + e, row + e);
   for (int q = 0; q < 5; q++) {
-    const double b0 = gp[1 + q], bx = gp[6 + q], by = gp[11 + q];
+    const double b0 = row[1 + q], bx = row[6 + q], by = row[11 + q];
+    T r4[4];
+    load_row(rc + 4 * q, r4);
     for (int v = 0; v < 4; v++) {
-      const double a = (double)rc[4 * q + v];
+      const double a = (double)r4[v];
       inc[v] += b0 * a; G[0][v] += bx * a; G[1][v] += by * a;
     }
     const double a = (double)rs[q];
@@ -439,25 +439,23 @@ DG_HD void dt_face_sa(int64_t f, const HotView<T>& h, const SaView<T>& sa) {
   const double nx = h.faceNormal[2 * f], ny = h.faceNormal[2 * f + 1], area = h.faceArea[f];
   double UL[4];
   load4<T>(&h.u[(int64_t)L * 4], UL);
-  double pL, aL2, HL, pR, aR2, HR;
-  double uL = UL[1] / UL[0], vL = UL[2] / UL[0], uR = uL, vR = vL;
-  thermal(UL[3], UL[0], uL * uL + vL * vL, h.gamma, pL, aL2, HL);
-  pR = pL; aR2 = aL2;
-  double rhoMean = UL[0], s5 = sa.u[L];
+  const double g1 = h.gamma - 1;
+  double UR[4] = {UL[0], UL[1], UL[2], UL[3]}, s5 = sa.u[L];
   if (R >= 0) {
-    double UR[4];
     load4<T>(&h.u[(int64_t)R * 4], UR);
-    rhoMean = (UL[0] + UR[0]) * 0.5;
     s5 = (s5 + sa.u[R]) * 0.5;
-    uR = UR[1] / UR[0]; vR = UR[2] / UR[0];
-    thermal(UR[3], UR[0], uR * uR + vR * vR, h.gamma, pR, aR2, HR);
   }
+  const double iLR = 1.0 / (UL[0] * UR[0]), irL = iLR * UR[0], irR = iLR * UL[0];  // one quotient for both densities
+  const double uL = UL[1] * irL, vL = UL[2] * irL, uR = UR[1] * irR, vR = UR[2] * irR;
+  const double pL = g1 * (UL[3] - UL[0] * 0.5 * (uL * uL + vL * vL)), aL2 = h.gamma * pL * irL;
+  const double pR = g1 * (UR[3] - UR[0] * 0.5 * (uR * uR + vR * vR)), aR2 = h.gamma * pR * irR;
+  const double irm = 1.0 / ((UL[0] + UR[0]) * 0.5);
   const double vn = 0.5 * ((uL + uR) * nx + (vL + vR) * ny);
   const double pMean = (pL + pR) * 0.5;
-  double lam = fabs(vn) + sqrt(h.gamma * pMean / rhoMean);
-  double muf = sutherland_mu(h, pMean, rhoMean);
-  muf *= sa_mu_factor(s5, h.mu, muf);
-  const double lamVis = muf / rhoMean * dmax(4. / 3., h.gamma / h.pr);
+  double lam = fabs(vn) + sqrt(h.gamma * pMean * irm);
+  double muf = sutherland_mu(h, pMean, irm);
+  muf *= sa_mu_factor(s5 * h.mu / muf);
+  const double lamVis = muf * irm * dmax(4. / 3., h.gamma / h.pr);
   lam += lamVis * area * (1.0 / h.vol[L] + 1.0 / (R >= 0 ? h.vol[R] : h.vol[L]));
   h.lamA[f] = lam * area;
   h.dLam[f] = fabs((uR - uL) * nx + (vR - vL) * ny) + sqrt(fabs(aR2 - aL2)) * 0.7071;
