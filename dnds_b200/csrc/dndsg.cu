@@ -166,21 +166,6 @@ __device__ __forceinline__ double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-// the sum of v over a block of kBlock threads (all of them call this) added to *acc by one thread:
-// one atomic per block instead of one per warp (many warps adding to one address serialise in L2)
-__device__ __forceinline__ void block_add(double v, double* acc) {
-  __shared__ double part[kBlock / 32];
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double t = threadIdx.x < kBlock / 32 ? part[threadIdx.x] : 0.0;
-    t = warp_sum(t);
-    if (threadIdx.x == 0 && t != 0.0) atomicAdd(acc, t);
-  }
-  __syncthreads();  // part is reused by the next call
-}
-
 // ------------------------------------------------------------------ setup kernels
 __global__ void k_setup_cell(MeshView m, SetupParams p, CellSetup* cells, double* vol, double* bary, int* bad) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -2289,13 +2274,55 @@ __global__ void __launch_bounds__(kBlock) k_lusgs_init(HotView<T> h, double dtPh
   D[i] = d;
 }
 
-// rhs of the first-order BDF pseudo-time system (ImplicitBDFDualTimeStep::Step,
-// DNDS_ODE.hpp:455-465): alpha R(u) - (u - uLast) / dtPhys, in place on rhs
-__global__ void k_bdf_rhs(int64_t n4, const double* u, const double* uLast, double alpha, double dtPhysInv,
-                          double* rhs) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= n4) return;
-  rhs[e] = alpha * rhs[e] - u[e] * dtPhysInv + uLast[e] * dtPhysInv;
+// The right-hand side of an implicit iteration from the residual r = R(x) of a cell (DNDS_ODE.hpp:330-336,
+// 454-466):
+//   BDF    r a0 + x c0 + sum_k p_k a_k        (c0 = -1/dt; p: xLast and the stored earlier steps)
+//   SDIRK  (p_0 - x) c0 + sum_{k>0} p_k a_k + r a0   (c0 = 1/dt; p: xLast, the earlier stages' residuals;
+//          the residual itself is kept in `keep`)
+constexpr int kCombMax = 4;
+struct ImplComb {
+  bool sdirk;
+  int m;
+  double a0, c0;
+  const double* p[kCombMax];
+  double a[kCombMax];
+  double* keep;
+};
+__device__ __forceinline__ double impl_combine(const ImplComb& c, int64_t e, double r, double x) {
+  double o;
+  if (c.sdirk) {
+    o = (c.p[0][e] - x) * c.c0;
+    for (int k = 1; k < c.m; k++) o += c.p[k][e] * c.a[k];
+    o += r * c.a0;
+    c.keep[e] = r;
+  } else {
+    o = r * c.a0;
+    o += x * c.c0;
+    for (int k = 0; k < c.m; k++) o += c.p[k][e] * c.a[k];
+  }
+  return o;
+}
+
+// The cell pass of an implicit iteration after its face fluxes: EvaluateRHS's gather, the local dt of
+// EvaluateDt, the LU-SGS diagonal (LUSGSMatrixInit) and the BDF or SDIRK right-hand side, in one pass over
+// the faces' fluxes and lambda A (five launches of their own before: on 524,288 triangles 67 us of kernels
+// and a copy, now 27 us).  The residual accumulators of the iteration start from zero here.
+template <class T>
+__global__ void __launch_bounds__(kBlock) k_implicit_cell(HotView<T> h, ImplComb cb, double cfl, double dtPhysInv,
+                                                          double alpha, double* Dinv, double* D, double* resAcc) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < 16) resAcc[i] = 0.0;
+  if (i >= h.N) return;
+  double r[4], lam, x[4], o[4];
+  cell_rhs<T, true>(i, h, r, &lam);
+  const double dt = dmin(cfl * h.vol[i] / (lam + 1e-100), 1e100);
+  const double d = alpha / dt + dtPhysInv + 0.5 * alpha * lam / h.vol[i];
+  h.dt[i] = dt;
+  Dinv[i] = 1.0 / d;
+  D[i] = d;
+  load4<T>(&h.u[i * 4], x);
+  for (int v = 0; v < 4; v++) o[v] = impl_combine(cb, i * 4 + v, r[v], x[v]);
+  store_row(&h.rhs[i * 4], o);
 }
 
 // one batch of UpdateLUSGSForward (FWD) or UpdateLUSGSBackward (DNDS_FV_EulerEvaluator.cpp:
@@ -2346,37 +2373,88 @@ __global__ void __launch_bounds__(kBlock) k_lusgs_batch(HotView<T> h, const int3
   if (t < n) lusgs_cell<T, FWD>(h, rankOf, cells[t], alpha, Dinv, rhs, inc);
 }
 
-// x += inc, with the L1 norm of inc per variable (volume-weighted on request) into acc[4]
-__global__ void __launch_bounds__(kBlock) k_add_inc(int64_t N, double* u, const double* inc, const double* vol,
-                                                    int volWise, double* acc) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double a[4] = {0, 0, 0, 0};
-  if (i < N) {
-    const double w = volWise ? vol[i] : 1.0;
-    for (int v = 0; v < 4; v++) {
-      const double d = inc[i * 4 + v];
-      u[i * 4 + v] += d;
-      a[v] = fabs(d) * w;
-    }
-  }
-  for (int v = 0; v < 4; v++) block_add(a[v], &acc[v]);
+// the first colour of a forward sweep: no neighbour comes before it (rhs5 null: flow only)
+__global__ void __launch_bounds__(kBlock) k_lusgs_first(const int32_t* cells, int64_t n, const double* Dinv, const double* rhs,
+                                                        double* inc, const double* Dinv5, const double* rhs5, double* inc5) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int64_t i = cells[t];
+  double r[4];
+  load4<double>(&rhs[i * 4], r);
+  const double di = Dinv[i];
+  for (int v = 0; v < 4; v++) r[v] *= di;
+  store_row(&inc[i * 4], r);
+  if (rhs5) inc5[i] = Dinv5[i] * rhs5[i];
 }
 
-// the wall force: minus the sum of the Riemann fluxes of the Wall_Euler / Wall_NoSlip faces
-// (fluxWallSum, DNDS_FV_EulerEvaluator.cpp:510-516), from the last flux evaluation
-__global__ void __launch_bounds__(kBlock) k_wall_flux(int64_t Fi, int64_t F, const int32_t* faceBC,
-                                                      const double* flux, double* acc) {
-  const int64_t f = Fi + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double a[4] = {0, 0, 0, 0};
-  if (f < F) {
-    const int bc = faceBC[f];
-    if (bc == BC_WALL_NOSLIP || bc == BC_WALL_EULER)
+// sums of NV values over a block of kBlock threads (all of them call this), added to acc[at[v]] with one
+// atomic per block and value
+template <int NV>
+__device__ __forceinline__ void block_add(const double (&v)[NV], double* acc, const int (&at)[NV]) {
+  __shared__ double part[kBlock / 32][NV];
+  for (int k = 0; k < NV; k++) {
+    const double t = warp_sum(v[k]);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][k] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double t = 0;
+    for (int w = 0; w < kBlock / 32; w++) t += part[w][threadIdx.x];
+    if (t != 0.0) atomicAdd(&acc[at[threadIdx.x]], t);
+  }
+}
+
+// the end of an implicit iteration, one launch: x += inc with the L1 norm of inc per variable
+// (volume-weighted on request) into acc[0..3], for SA contexts CompressInc of the U5 increment and U5 += it
+// (norm into acc[8]), and in the blocks past cellBlocks the wall force: minus the sum of the Riemann fluxes
+// of the Wall_Euler / Wall_NoSlip faces [Fi, F) (fluxWallSum, DNDS_FV_EulerEvaluator.cpp:510-516) of the
+// last flux evaluation into acc[4..7] and acc[9]
+template <bool SA>
+__global__ void __launch_bounds__(kBlock) k_implicit_finish(int64_t N, double* u, const double* inc, double* u5, double* inc5,
+                                                            const double* vol, int volWise, unsigned cellBlocks, int64_t Fi,
+                                                            int64_t F, const int32_t* faceBC, const double* flux,
+                                                            const double* flux5, double* acc) {
+  double a[5] = {0, 0, 0, 0, 0};
+  if (blockIdx.x < cellBlocks) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < N) {
+      const double w = volWise ? vol[i] : 1.0;
+      double x[4], d[4];
+      load4<double>(&u[i * 4], x);
+      load4<double>(&inc[i * 4], d);
+      for (int v = 0; v < 4; v++) {
+        x[v] += d[v];
+        a[v] = fabs(d[v]) * w;
+      }
+      store_row(&u[i * 4], x);
+      if (SA) {
+        const double d5 = sa_compress_inc(u5[i], inc5[i]);
+        inc5[i] = d5;
+        u5[i] += d5;
+        a[4] = fabs(d5) * w;
+      }
+    }
+    const int at[5] = {0, 1, 2, 3, 8};
+    block_add(a, acc, at);
+  } else {
+    const int64_t f = Fi + (blockIdx.x - cellBlocks) * (int64_t)blockDim.x + threadIdx.x;
+    if (f < F && (faceBC[f] == BC_WALL_NOSLIP || faceBC[f] == BC_WALL_EULER)) {
       for (int v = 0; v < 4; v++) a[v] = -flux[f * 4 + v];
+      if (SA) a[4] = -flux5[f];
+    }
+    const int at[5] = {4, 5, 6, 7, 9};
+    block_add(a, acc, at);
   }
-  for (int v = 0; v < 4; v++) {
-    const double r = warp_sum(a[v]);
-    if ((threadIdx.x & 31) == 0 && r != 0.0) atomicAdd(&acc[v], r);
-  }
+}
+// walls: with the wall force
+void launch_implicit_finish(dndsg_ctx* c, int volWise, bool walls, cudaStream_t s) {
+  const unsigned nb = grid_for(c->N), nw = walls && c->F > c->Fi ? grid_for(c->F - c->Fi) : 0;
+  if (c->sa)
+    k_implicit_finish<true><<<nb + nw, kBlock, 0, s>>>(c->N, c->u, c->inc, c->saU, c->saInc, c->vol, volWise, nb, c->Fi, c->F,
+                                                       c->faceBC, c->flux, c->saFlux, c->resAcc);
+  else
+    k_implicit_finish<false><<<nb + nw, kBlock, 0, s>>>(c->N, c->u, c->inc, nullptr, nullptr, c->vol, volWise, nb, c->Fi, c->F,
+                                                        c->faceBC, c->flux, nullptr, c->resAcc);
 }
 
 // cell adjacency over the interior faces (CSR), from the device face table
@@ -2640,7 +2718,9 @@ void launch_lusgs_sweep(dndsg_ctx* c, bool forward, double alpha, const double* 
     launch_walk<false>(c, forward, alpha, rhs, inc, nullptr, nullptr, s);
     return;
   }
-  for (int k = 0; k < nb; k++) {
+  // the first batch of a sweep has no neighbour before it: forward it is D^-1 rhs, backward nothing
+  if (forward) k_lusgs_first<<<grid_for(off[1]), kBlock, 0, s>>>(cells, off[1], c->Dinv, rhs, inc, nullptr, nullptr, nullptr);
+  for (int k = 1; k < nb; k++) {
     const int64_t b = off[k], n = off[k + 1] - b;
     if (n == 0) continue;
     if (forward)
@@ -2648,6 +2728,30 @@ void launch_lusgs_sweep(dndsg_ctx* c, bool forward, double alpha, const double* 
     else
       k_lusgs_batch<T, false><<<grid_for(n), kBlock, 0, s>>>(h, c->rankOf, cells + b, n, alpha, c->Dinv, rhs, inc);
   }
+}
+
+// alpha R(x) - (x - xLast) / dt
+inline ImplComb bdf1_comb(const double* xLast, double alpha, double dtInv) {
+  ImplComb cb{};
+  cb.m = 1;
+  cb.a0 = alpha;
+  cb.c0 = -dtInv;
+  cb.p[0] = xLast;
+  cb.a[0] = dtInv;
+  return cb;
+}
+
+// fdtau + frhs + LUSGSMatrixInit of a 4-variable context: nRec Jacobi sweeps, [limiter], the face fluxes at
+// time t with EvaluateDt's face terms (inviscid contexts; viscous ones run the dt pass first), and the cell
+// pass.  Leaves c->rhs, c->dt and the diagonal.
+template <class T>
+void implicit_rhs(dndsg_ctx* c, double cfl, double t, int nRec, const ImplComb& cb, double dtPhysInv, double alpha, cudaStream_t s) {
+  const bool viscous = c->s.mu_gas > 0;
+  if (viscous) k_dt_face<T><<<grid_for(c->F), kBlock, 0, s>>>(view<T>(c));
+  for (int k = 0; k < nRec; k++) run_vr<T>(c, false, s);
+  if (c->s.limiter) run_limiter<T>(c, 0, s);
+  launch_flux<T>(c, 0, t, 0.0, s, !viscous);
+  k_implicit_cell<T><<<grid_for(c->N), kBlock, 0, s>>>(view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
 }
 
 // ImplicitBDFDualTimeStep::Step (DNDS_ODE.hpp:444-486), one pseudo-time iteration at order 1, with
@@ -2659,21 +2763,11 @@ int run_implicit(dndsg_ctx* c, double cfl, double dtPhys, double alpha, int nRec
                  cudaStream_t s) {
   int rc;
   if ((rc = ensure_lusgs(c))) return rc;
-  run_dt<T>(c, cfl, 1e100, false, s);
-  for (int k = 0; k < nRec; k++) run_vr<T>(c, false, s);
-  if (c->s.limiter) run_limiter<T>(c, 0, s);
-  run_rhs<T>(c, t, s);
   const double dtInv = 1.0 / dtPhys;
-  const int64_t n4 = c->N * 4;
-  k_bdf_rhs<<<(unsigned)((n4 + kBlock - 1) / kBlock), kBlock, 0, s>>>(n4, c->u, c->uLast, alpha, dtInv, c->rhs);
-  HotView<T> h = view<T>(c);
-  k_lusgs_init<T><<<grid_for(c->N), kBlock, 0, s>>>(h, dtInv, alpha, c->Dinv, c->Dmat);
+  implicit_rhs<T>(c, cfl, t, nRec, bdf1_comb(c->uLast, alpha, dtInv), dtInv, alpha, s);
   launch_lusgs_sweep<T>(c, true, alpha, c->rhs, c->inc, s);
   launch_lusgs_sweep<T>(c, false, alpha, c->rhs, c->inc, s);
-  DG_CUDA(c, cudaMemsetAsync(c->resAcc, 0, sizeof(double) * 16, s));
-  k_add_inc<<<grid_for(c->N), kBlock, 0, s>>>(c->N, c->u, c->inc, c->vol, volWise, c->resAcc);
-  if (c->F > c->Fi)
-    k_wall_flux<<<grid_for(c->F - c->Fi), kBlock, 0, s>>>(c->Fi, c->F, c->faceBC, c->flux, c->resAcc + 4);
+  launch_implicit_finish(c, volWise, true, s);
   return check_launch(c);
 }
 }  // namespace
@@ -2790,14 +2884,15 @@ int dndsg_implicit_iteration(dndsg_ctx* c, double cfl, double dt_phys, double al
   if (inc_res_out || wall_flux_out) {
     double acc[16];
     DG_CUDA(c, cudaMemcpyAsync(acc, c->resAcc, sizeof(acc), cudaMemcpyDeviceToHost, st(s)));
-    DG_CUDA(c, cudaStreamSynchronize(st(s)));
+    rc = observe_timeout(c, st(s));  // waits for both copies
+    if (rc && rc != DNDSG_TIMEOUT) return rc;
     if (inc_res_out) for (int v = 0; v < 4; v++) inc_res_out[v] = acc[v];
     if (wall_flux_out) for (int v = 0; v < 4; v++) wall_flux_out[v] = acc[4 + v];
     if (c->sa) {
       if (inc_res_out) inc_res_out[4] = acc[8];
       if (wall_flux_out) wall_flux_out[4] = acc[9];
     }
-    return observe_timeout(c, st(s));
+    return rc;
   }
   return 0;
 }
@@ -2815,11 +2910,12 @@ __global__ void __launch_bounds__(kBlock) k_sa_vr(HotView<T> h, SaView<T> sa) {
 
 // one thread per (face, Gauss point), as for the cell source: three times the resident warps for the
 // long per-point chain (Roe, gradients, viscous and U5 fluxes).  Thread g == 0 of each face sums the
-// points in order.
+// points in order.  The chain waits on latency with two blocks per SM (134 registers); a third (96, some
+// words spilled) and a fourth of the source below took a RANS-SA iteration on 65,536 quads from 366 to 356 us
 constexpr int kSaFluxFaces = 64;
 inline unsigned sa_flux_grid(int64_t n) { return (unsigned)((n + kSaFluxFaces - 1) / kSaFluxFaces); }
 template <class T, int RIEMANN, bool BND>
-__global__ void __launch_bounds__(kSaFluxFaces * 3) k_face_flux_sa(HotView<T> h, SaView<T> sa, int64_t f0, int64_t f1,
+__global__ void __launch_bounds__(kSaFluxFaces * 3, 3) k_face_flux_sa(HotView<T> h, SaView<T> sa, int64_t f0, int64_t f1,
                                                                    unsigned* flags, unsigned long long* nred) {
   __shared__ double part[kSaFluxFaces * 3][5];
   const int64_t f = f0 + blockIdx.x * (int64_t)kSaFluxFaces + threadIdx.x / 3;
@@ -2856,8 +2952,13 @@ __global__ void __launch_bounds__(kSaFluxFaces * 3) k_face_flux_sa(HotView<T> h,
 // one thread per cell left too few warps resident on a 65,536-cell mesh; thread ig == 0 of each cell
 // then sums the points in order (the same sum as a sequential loop over the points)
 constexpr int kSaRhsCells = 32;
-template <class T>
-__global__ void __launch_bounds__(kSaRhsCells * kSaGp) k_sa_cell_rhs(HotView<T> h, SaView<T> sa) {
+// IMPL: the pass of an implicit iteration, after k_implicit_cell: the BDF or SDIRK form of the U5 rhs with
+// CompressInc of rhs * dTau (dTau = dt / alpha) as fsolve applies it, and the U5 diagonal: the flow one plus
+// alpha * the source Jacobian (LUSGSMatrixInit), its inverse for the sweeps and (DS, may be null) itself
+// for LUSGSMatrixVec
+template <class T, bool IMPL>
+__global__ void __launch_bounds__(kSaRhsCells * kSaGp, 4) k_sa_cell_rhs(HotView<T> h, SaView<T> sa, ImplComb cb, double alpha,
+                                                                     const double* D, double* DS) {
   __shared__ double sv[kSaRhsCells * kSaGp], sj[kSaRhsCells * kSaGp];
   const int64_t i = blockIdx.x * (int64_t)kSaRhsCells + threadIdx.x / kSaGp;
   const int ig = threadIdx.x % kSaGp;
@@ -2866,7 +2967,18 @@ __global__ void __launch_bounds__(kSaRhsCells * kSaGp) k_sa_cell_rhs(HotView<T> 
   sv[threadIdx.x] = src;
   sj[threadIdx.x] = jac;
   __syncthreads();
-  if (ig == 0 && i < h.N) sa_cell_rhs<T>(i, h, sa, &sv[threadIdx.x], &sj[threadIdx.x]);
+  if (ig != 0 || i >= h.N) return;
+  double r, j;
+  sa_cell_rhs<T>(i, h, sa, &sv[threadIdx.x], &sj[threadIdx.x], r, j);
+  sa.srcJac[i] = j;
+  if (IMPL) {
+    const double x = sa.u[i], dTau = h.dt[i] / alpha, d = D[i] + alpha * j;
+    r = impl_combine(cb, i, r, x);
+    r = sa_compress_inc(x, r * dTau) / dTau;
+    sa.Dinv[i] = 1.0 / d;
+    if (DS) DS[i] = d;
+  }
+  sa.rhs[i] = r;
 }
 
 template <class T>
@@ -2881,50 +2993,6 @@ __global__ void __launch_bounds__(kBlock) k_lusgs_batch_sa(HotView<T> h, SaView<
                                                            const double* Dinv, const double* rhs, double* inc) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t < n) lusgs_cell_sa<T, FWD>(h, sa, rankOf, cells[t], alpha, Dinv, rhs, inc);
-}
-
-// the U5 diagonal: the flow one plus alpha * the source Jacobian (LUSGSMatrixInit), its inverse
-// for the sweeps and (DS, may be null) itself for LUSGSMatrixVec
-__global__ void k_sa_diag(int64_t N, const double* D, const double* srcJac, double alpha, double* DinvS, double* DS) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const double d = D[i] + alpha * srcJac[i];
-  DinvS[i] = 1.0 / d;
-  if (DS) DS[i] = d;
-}
-
-// U5 parts of one pseudo-time iteration: the BDF rhs, CompressInc of rhs * dTau (dTau = dt / alpha)
-__global__ void k_sa_rhs_fix(int64_t N, const double* u, const double* uLast, const double* dt, double alpha,
-                             double dtPhysInv, double* rhs) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  double r = alpha * rhs[i] - u[i] * dtPhysInv + uLast[i] * dtPhysInv;
-  const double dTau = dt[i] / alpha;
-  r = sa_compress_inc(u[i], r * dTau) / dTau;
-  rhs[i] = r;
-}
-
-// CompressInc of the U5 increment, u5 += inc, its L1 norm, and the U5 wall flux
-__global__ void __launch_bounds__(kBlock) k_sa_add_inc(int64_t N, double* u, double* inc, const double* vol,
-                                                       int volWise, double* acc) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double a = 0;
-  if (i < N) {
-    const double d = sa_compress_inc(u[i], inc[i]);
-    inc[i] = d;
-    u[i] += d;
-    a = fabs(d) * (volWise ? vol[i] : 1.0);
-  }
-  block_add(a, acc);
-}
-
-__global__ void __launch_bounds__(kBlock) k_sa_wall_flux(int64_t Fi, int64_t F, const int32_t* faceBC,
-                                                         const double* flux, double* acc) {
-  const int64_t f = Fi + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double a = 0;
-  if (f < F && (faceBC[f] == BC_WALL_NOSLIP || faceBC[f] == BC_WALL_EULER)) a = -flux[f];
-  a = warp_sum(a);
-  if ((threadIdx.x & 31) == 0 && a != 0.0) atomicAdd(acc, a);
 }
 
 template <class T>
@@ -2943,7 +3011,7 @@ void run_dt_sa(dndsg_ctx* c, double cfl, double maxDt, cudaStream_t s) {
 }
 
 template <class T>
-void run_rhs_sa(dndsg_ctx* c, cudaStream_t s) {
+void launch_flux_sa(dndsg_ctx* c, cudaStream_t s) {
   HotView<T> h = view<T>(c);
   SaView<T> sa = sa_view<T>(c);
   const int64_t Fi = c->Fi, F = c->F;
@@ -2954,8 +3022,24 @@ void run_rhs_sa(dndsg_ctx* c, cudaStream_t s) {
     if (Fi > 0) k_face_flux_sa<T, 1, false><<<sa_flux_grid(Fi), kSaFluxFaces * 3, 0, s>>>(h, sa, 0, Fi, c->flags, c->nreduced);
     if (F > Fi) k_face_flux_sa<T, 1, true><<<sa_flux_grid(F - Fi), kSaFluxFaces * 3, 0, s>>>(h, sa, Fi, F, c->flags, c->nreduced);
   }
-  k_cell_update<T, -1><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
-  k_sa_cell_rhs<T><<<(unsigned)((c->N + kSaRhsCells - 1) / kSaRhsCells), kSaRhsCells * kSaGp, 0, s>>>(h, sa);
+}
+inline unsigned sa_rhs_grid(int64_t n) { return (unsigned)((n + kSaRhsCells - 1) / kSaRhsCells); }
+template <class T>
+void run_rhs_sa(dndsg_ctx* c, cudaStream_t s) {
+  launch_flux_sa<T>(c, s);
+  k_cell_update<T, -1><<<grid_for(c->N), kBlock, 0, s>>>(view<T>(c), c->scal);
+  k_sa_cell_rhs<T, false><<<sa_rhs_grid(c->N), kSaRhsCells * kSaGp, 0, s>>>(view<T>(c), sa_view<T>(c), ImplComb{}, 0.0, nullptr, nullptr);
+}
+
+// implicit_rhs of an SA context: cb5 is the combination of the U5 rhs, DS (may be null) receives the U5 diagonal
+template <class T>
+void implicit_rhs_sa(dndsg_ctx* c, double cfl, int nRec, const ImplComb& cb, const ImplComb& cb5, double dtPhysInv, double alpha,
+                     double* DS, cudaStream_t s) {
+  k_dt_face_sa<T><<<grid_for(c->F), kBlock, 0, s>>>(view<T>(c), sa_view<T>(c));
+  for (int k = 0; k < nRec; k++) run_vr_sa<T>(c, s);
+  launch_flux_sa<T>(c, s);
+  k_implicit_cell<T><<<grid_for(c->N), kBlock, 0, s>>>(view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
+  k_sa_cell_rhs<T, true><<<sa_rhs_grid(c->N), kSaRhsCells * kSaGp, 0, s>>>(view<T>(c), sa_view<T>(c), cb5, alpha, c->Dmat, DS);
 }
 
 template <class T>
@@ -2972,7 +3056,8 @@ void launch_lusgs_sweep_sa(dndsg_ctx* c, bool forward, double alpha, const doubl
     launch_walk<true>(c, forward, alpha, rhs4, inc4, rhs5, inc5, s);
     return;
   }
-  for (int k = 0; k < nb; k++) {
+  if (forward) k_lusgs_first<<<grid_for(off[1]), kBlock, 0, s>>>(cells, off[1], c->Dinv, rhs4, inc4, c->saDinv, rhs5, inc5);
+  for (int k = 1; k < nb; k++) {
     const int64_t b = off[k], n = off[k + 1] - b;
     if (n == 0) continue;
     if (forward)
@@ -2988,25 +3073,11 @@ template <class T>
 int run_implicit_sa(dndsg_ctx* c, double cfl, double dtPhys, double alpha, int nRec, int volWise, cudaStream_t s) {
   int rc;
   if ((rc = ensure_lusgs(c))) return rc;
-  run_dt_sa<T>(c, cfl, 1e100, s);
-  for (int k = 0; k < nRec; k++) run_vr_sa<T>(c, s);
-  run_rhs_sa<T>(c, s);
   const double dtInv = 1.0 / dtPhys;
-  const int64_t n4 = c->N * 4;
-  k_bdf_rhs<<<(unsigned)((n4 + kBlock - 1) / kBlock), kBlock, 0, s>>>(n4, c->u, c->uLast, alpha, dtInv, c->rhs);
-  k_sa_rhs_fix<<<grid_for(c->N), kBlock, 0, s>>>(c->N, c->saU, c->saULast, c->dt, alpha, dtInv, c->saRhs);
-  HotView<T> h = view<T>(c);
-  k_lusgs_init<T><<<grid_for(c->N), kBlock, 0, s>>>(h, dtInv, alpha, c->Dinv, c->Dmat);
-  k_sa_diag<<<grid_for(c->N), kBlock, 0, s>>>(c->N, c->Dmat, c->saSrcJac, alpha, c->saDinv, nullptr);
+  implicit_rhs_sa<T>(c, cfl, nRec, bdf1_comb(c->uLast, alpha, dtInv), bdf1_comb(c->saULast, alpha, dtInv), dtInv, alpha, nullptr, s);
   launch_lusgs_sweep_sa<T>(c, true, alpha, c->rhs, c->inc, c->saRhs, c->saInc, s);
   launch_lusgs_sweep_sa<T>(c, false, alpha, c->rhs, c->inc, c->saRhs, c->saInc, s);
-  DG_CUDA(c, cudaMemsetAsync(c->resAcc, 0, sizeof(double) * 16, s));
-  k_add_inc<<<grid_for(c->N), kBlock, 0, s>>>(c->N, c->u, c->inc, c->vol, volWise, c->resAcc);
-  k_sa_add_inc<<<grid_for(c->N), kBlock, 0, s>>>(c->N, c->saU, c->saInc, c->vol, volWise, c->resAcc + 8);
-  if (c->F > c->Fi) {
-    k_wall_flux<<<grid_for(c->F - c->Fi), kBlock, 0, s>>>(c->Fi, c->F, c->faceBC, c->flux, c->resAcc + 4);
-    k_sa_wall_flux<<<grid_for(c->F - c->Fi), kBlock, 0, s>>>(c->Fi, c->F, c->faceBC, c->saFlux, c->resAcc + 9);
-  }
+  launch_implicit_finish(c, volWise, true, s);
   return check_launch(c);
 }
 

@@ -961,9 +961,11 @@ DG_HD double dt_cell(int64_t i, const HotView<T>& h, double cfl, double maxDt) {
 
 // rhs of cell i: gather of face fluxes plus the flux-balance term
 // (DNDS_FV_EulerEvaluator.cpp:501-508): -F(u_i) . sum_f n_f A_f / V_i
-template <class T>
-DG_HD void cell_rhs(int64_t i, const HotView<T>& h, double r[4]) {
+// lam (LAM): the sum of the faces' lambda_f A_f as well
+template <class T, bool LAM = false>
+DG_HD void cell_rhs(int64_t i, const HotView<T>& h, double r[4], double* lam = nullptr) {
   double s[4] = {0, 0, 0, 0};
+  if (LAM) *lam = 0.0;
   for (int k = 0; k < h.nfmax; k++) {
     int32_t sf = h.cellFace[aos(i, k, h.nfmax)];
     if (sf == kEmptySlot) continue;
@@ -971,6 +973,7 @@ DG_HD void cell_rhs(int64_t i, const HotView<T>& h, double r[4]) {
     const double* fl = &h.flux[(int64_t)f * 4];
     if (sf >= 0) { for (int v = 0; v < 4; v++) s[v] += fl[v]; }
     else { for (int v = 0; v < 4; v++) s[v] -= fl[v]; }
+    if (LAM) *lam += h.lamA[f];
   }
   double U[4];
   load4<T>(&h.u[i * 4], U);

@@ -48,30 +48,6 @@ struct VecList {
   double a[kMaxKrylov + 1];
 };
 
-// BDF right-hand side, in place on rhs = R(x) (DNDS_ODE.hpp:454-466):
-// rhs *= a0; rhs += x * (-1/dt); rhs += X_m * (c_m / dt) for xLast and the stored earlier steps
-__global__ void __launch_bounds__(kBlock) k_dual_bdf_rhs(int64_t n, const double* x, double a0, double negInvDt,
-                                                         VecList X, int m, double* rhs) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  double r = rhs[e] * a0;
-  r += x[e] * negInvDt;
-  for (int k = 0; k < m; k++) r += X.p[k][e] * X.a[k];
-  rhs[e] = r;
-}
-
-// SDIRK stage right-hand side (DNDS_ODE.hpp:330-336): rhs = (xLast - x) * (1/dt) + sum_j R_j a_j
-__global__ void __launch_bounds__(kBlock) k_dual_sdirk_rhs(int64_t n, const double* xLast, const double* x,
-                                                           double invDt, VecList R, int m, double* rhs) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  double r = xLast[e];
-  r -= x[e];
-  r *= invDt;
-  for (int k = 0; k < m; k++) r += R.p[k][e] * R.a[k];
-  rhs[e] = r;
-}
-
 // x = base + sum_k V_k a_k (base may alias x; base NULL keeps x)
 __global__ void __launch_bounds__(kBlock) k_vec_combine(int64_t n, const double* base, VecList V, int m, double* x) {
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -191,13 +167,6 @@ __global__ void __launch_bounds__(kBlock) k_lusgs_matvec_sa5(HotView<T> h, const
   Ax5[i] = D5[i] * x5[i] - buf;
 }
 
-// CompressInc of the U5 right-hand side as fsolve applies it: rhs = CompressInc(u, rhs dTau) / dTau
-__global__ void k_sa_compress_rhs(int64_t N, const double* u, const double* dt, double alpha, double* rhs) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const double dTau = dt[i] / alpha;
-  rhs[i] = sa_compress_inc(u[i], rhs[i] * dTau) / dTau;
-}
 // CompressInc of the U5 increment in place
 __global__ void k_sa_compress_inc(int64_t N, const double* u, double* inc) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -351,36 +320,24 @@ int gmres_solve(dndsg_ctx* c, int K, int nRestart, double alpha, const double* b
 }
 
 // fdtau + frhs: local EvaluateDt at cfl (dTau = dt / alphaDiag is folded into the diagonal),
-// nInternalRecStep Jacobi sweeps, [limiter], EvaluateRHS at tEval into c->rhs
+// nInternalRecStep Jacobi sweeps, [limiter], EvaluateRHS at tEval, the scheme's right-hand side cb (cb5 of
+// U5) into c->rhs and the diagonal for the physical step dt
 template <class T>
-void dual_frhs(dndsg_ctx* c, const DualOpts& o, double tEval, cudaStream_t s) {
-  if (c->sa) {
-    run_dt_sa<T>(c, o.cfl, 1e100, s);
-    for (int k = 0; k < o.nRec; k++) run_vr_sa<T>(c, s);
-    run_rhs_sa<T>(c, s);
-    return;
-  }
-  run_dt<T>(c, o.cfl, 1e100, false, s);
-  for (int k = 0; k < o.nRec; k++) run_vr<T>(c, false, s);
-  if (c->s.limiter) run_limiter<T>(c, 0, s);
-  run_rhs<T>(c, tEval, s);
+void dual_frhs(dndsg_ctx* c, const DualOpts& o, double tEval, const ImplComb& cb, const ImplComb& cb5, double dt, double alpha,
+               cudaStream_t s) {
+  if (c->sa) implicit_rhs_sa<T>(c, o.cfl, o.nRec, cb, cb5, 1.0 / dt, alpha, c->saDmat, s);
+  else implicit_rhs<T>(c, o.cfl, tEval, o.nRec, cb, 1.0 / dt, alpha, s);
 }
 
 // fsolve on rhs = c->rhs into c->inc (CompressInc is the identity for 4 variables)
 template <class T>
-int dual_fsolve(dndsg_ctx* c, const DualOpts& o, double dt, double alpha, cudaStream_t s) {
-  HotView<T> h = view<T>(c);
+int dual_fsolve(dndsg_ctx* c, const DualOpts& o, double alpha, cudaStream_t s) {
   const int64_t N = c->N, n4 = 4 * N;
-  k_lusgs_init<T><<<grid_for(N), kBlock, 0, s>>>(h, 1.0 / dt, alpha, c->Dinv, c->Dmat);
-  if (c->sa) {
-    k_sa_diag<<<grid_for(N), kBlock, 0, s>>>(N, c->Dmat, c->saSrcJac, alpha, c->saDinv, c->saDmat);
-    k_sa_compress_rhs<<<grid_for(N), kBlock, 0, s>>>(N, c->saU, c->dt, alpha, c->saRhs);
-  }
   if (o.gmresCode == 0 || o.gmresCode == 2) {
     if (c->sa) {
       launch_lusgs_sweep_sa<T>(c, true, alpha, c->rhs, c->inc, c->saRhs, c->saInc, s);
       launch_lusgs_sweep_sa<T>(c, false, alpha, c->rhs, c->inc, c->saRhs, c->saInc, s);
-      k_sa_compress_inc<<<grid_for(N), kBlock, 0, s>>>(N, c->saU, c->saInc);
+      if (o.gmresCode == 2) k_sa_compress_inc<<<grid_for(N), kBlock, 0, s>>>(N, c->saU, c->saInc);  // (else with U5 += inc)
     } else {
       launch_lusgs_sweep<T>(c, true, alpha, c->rhs, c->inc, s);
       launch_lusgs_sweep<T>(c, false, alpha, c->rhs, c->inc, s);
@@ -412,10 +369,7 @@ struct Fstop {
 };
 template <class T>
 int dual_add_and_test(dndsg_ctx* c, const DualOpts& o, int iter, Fstop& f, bool& stop, cudaStream_t s) {
-  DG_CUDA(c, cudaMemsetAsync(c->resAcc, 0, sizeof(double) * 16, s));
-  k_add_inc<<<grid_for(c->N), kBlock, 0, s>>>(c->N, c->u, c->inc, c->vol, o.volWise, c->resAcc);
-  if (c->sa)  // CompressInc of the U5 increment (after the Krylov solve too), u5 += inc
-    k_sa_add_inc<<<grid_for(c->N), kBlock, 0, s>>>(c->N, c->saU, c->saInc, c->vol, o.volWise, c->resAcc + 8);
+  launch_implicit_finish(c, o.volWise, false, s);
   double acc[16];
   DG_CUDA(c, cudaMemcpyAsync(acc, c->resAcc, sizeof(acc), cudaMemcpyDeviceToHost, s));
   DG_CUDA(c, cudaStreamSynchronize(s));
@@ -446,6 +400,12 @@ int dual_step(dndsg_ctx* c, const DualOpts& o, double dt, double t, int* itersOu
     for (int k = 0; k < m; k++) L.p[k] += n;
     return L;
   };
+  auto comb5 = [&](ImplComb cb) {  // the U5 part of a combination: xLast first, then stored vectors
+    cb.p[0] = c->saULast;
+    for (int k = 1; k < cb.m; k++) cb.p[k] += n;
+    if (cb.keep) cb.keep += n;
+    return cb;
+  };
   if ((rc = copy(c->uLast, c->saULast, c->u, c->saU))) return rc;
   Fstop f;
   if (o.scheme == DNDSG_DUAL_BDF) {
@@ -455,22 +415,18 @@ int dual_step(dndsg_ctx* c, const DualOpts& o, double dt, double t, int* itersOu
     const double* coef = kBdfCoef[kCur - 1];
     int iter = 1;
     for (; iter <= o.maxIter; iter++) {
-      dual_frhs<T>(c, o, t + 1.0 * dt, s);
-      VecList X{};
-      X.p[0] = c->uLast;
-      X.a[0] = coef[1] / dt;
+      ImplComb cb{};
+      cb.a0 = coef[0];
+      cb.c0 = -1. / dt;
+      cb.m = 1 + c->odeCnPrev;
+      cb.p[0] = c->uLast;
+      cb.a[0] = coef[1] / dt;
       for (int k = 0; k < c->odeCnPrev; k++) {
-        X.p[1 + k] = c->odeVec[(size_t)((k + c->odePrevStart) % prevSiz)];
-        X.a[1 + k] = coef[2 + k] / dt;
+        cb.p[1 + k] = c->odeVec[(size_t)((k + c->odePrevStart) % prevSiz)];
+        cb.a[1 + k] = coef[2 + k] / dt;
       }
-      const int m = 1 + c->odeCnPrev;
-      k_dual_bdf_rhs<<<vgrid(n), kBlock, 0, s>>>(n, c->u, coef[0], -1. / dt, X, m, c->rhs);
-      if (sa) {
-        VecList X5 = part5(X, m);
-        X5.p[0] = c->saULast;
-        k_dual_bdf_rhs<<<vgrid(N), kBlock, 0, s>>>(N, c->saU, coef[0], -1. / dt, X5, m, c->saRhs);
-      }
-      if ((rc = dual_fsolve<T>(c, o, dt, coef[0], s))) return rc;
+      dual_frhs<T>(c, o, t + 1.0 * dt, cb, comb5(cb), dt, coef[0], s);
+      if ((rc = dual_fsolve<T>(c, o, coef[0], s))) return rc;
       bool stop = false;
       if ((rc = dual_add_and_test<T>(c, o, iter, f, stop, s))) return rc;
       if (stop) break;
@@ -489,18 +445,19 @@ int dual_step(dndsg_ctx* c, const DualOpts& o, double dt, double t, int* itersOu
       if ((rc = copy(c->u, c->saU, c->uLast, c->saULast))) return rc;
       int iter = 1;
       for (; iter <= o.maxIter; iter++) {
-        dual_frhs<T>(c, o, t + tb.c[iB] * dt, s);
-        if ((rc = copy(c->odeVec[iB], c->odeVec[iB] + n, c->rhs, c->saRhs))) return rc;
-        VecList R{};
-        for (int j = 0; j <= iB; j++) {
-          R.p[j] = c->odeVec[j];
-          R.a[j] = tb.A[iB][j];
+        ImplComb cb{};
+        cb.sdirk = true;
+        cb.a0 = tb.A[iB][iB];
+        cb.c0 = 1.0 / dt;
+        cb.m = 1 + iB;
+        cb.p[0] = c->uLast;
+        for (int j = 0; j < iB; j++) {
+          cb.p[1 + j] = c->odeVec[j];
+          cb.a[1 + j] = tb.A[iB][j];
         }
-        k_dual_sdirk_rhs<<<vgrid(n), kBlock, 0, s>>>(n, c->uLast, c->u, 1.0 / dt, R, iB + 1, c->rhs);
-        if (sa)
-          k_dual_sdirk_rhs<<<vgrid(N), kBlock, 0, s>>>(N, c->saULast, c->saU, 1.0 / dt, part5(R, iB + 1), iB + 1,
-                                                       c->saRhs);
-        if ((rc = dual_fsolve<T>(c, o, dt, tb.A[iB][iB], s))) return rc;
+        cb.keep = c->odeVec[iB];
+        dual_frhs<T>(c, o, t + tb.c[iB] * dt, cb, comb5(cb), dt, tb.A[iB][iB], s);
+        if ((rc = dual_fsolve<T>(c, o, tb.A[iB][iB], s))) return rc;
         bool stop = false;
         if ((rc = dual_add_and_test<T>(c, o, iter, f, stop, s))) return rc;
         if (stop) break;
@@ -540,26 +497,10 @@ int steady_solve(dndsg_ctx* c, const dndsg_steady_settings* st, int* itersOut, d
   int iter = 1;
   for (; iter <= st->max_iter; iter++) {
     o.cfl = cflNow;
-    dual_frhs<T>(c, o, 0.0, s);
-    VecList X{};
-    X.p[0] = c->uLast;
-    X.a[0] = 1.0 / dt;
-    k_dual_bdf_rhs<<<vgrid(n), kBlock, 0, s>>>(n, c->u, 1.0, -1. / dt, X, 1, c->rhs);
-    if (sa) {
-      VecList X5{};
-      X5.p[0] = c->saULast;
-      X5.a[0] = 1.0 / dt;
-      k_dual_bdf_rhs<<<vgrid(N), kBlock, 0, s>>>(N, c->saU, 1.0, -1. / dt, X5, 1, c->saRhs);
-    }
-    if ((rc = dual_fsolve<T>(c, o, dt, 1.0, s))) return rc;
+    dual_frhs<T>(c, o, 0.0, bdf1_comb(c->uLast, 1.0, 1.0 / dt), bdf1_comb(c->saULast, 1.0, 1.0 / dt), dt, 1.0, s);
+    if ((rc = dual_fsolve<T>(c, o, 1.0, s))) return rc;
     // x += inc with the increment norms, and the wall force of this iteration's residual
-    DG_CUDA(c, cudaMemsetAsync(c->resAcc, 0, sizeof(double) * 16, s));
-    k_add_inc<<<grid_for(N), kBlock, 0, s>>>(N, c->u, c->inc, c->vol, o.volWise, c->resAcc);
-    if (sa) k_sa_add_inc<<<grid_for(N), kBlock, 0, s>>>(N, c->saU, c->saInc, c->vol, o.volWise, c->resAcc + 8);
-    if (c->F > c->Fi) {
-      k_wall_flux<<<grid_for(c->F - c->Fi), kBlock, 0, s>>>(c->Fi, c->F, c->faceBC, c->flux, c->resAcc + 4);
-      if (sa) k_sa_wall_flux<<<grid_for(c->F - c->Fi), kBlock, 0, s>>>(c->Fi, c->F, c->faceBC, c->saFlux, c->resAcc + 9);
-    }
+    launch_implicit_finish(c, o.volWise, true, s);
     DG_CUDA(c, cudaMemcpyAsync(acc, c->resAcc, sizeof(acc), cudaMemcpyDeviceToHost, s));
     DG_CUDA(c, cudaStreamSynchronize(s));
     if ((rc = check_launch(c))) return rc;

@@ -408,9 +408,10 @@ DG_HD void sa_cell_point(int64_t i, int ig, const HotView<T>& h, const SaView<T>
 
 // U5 rhs of cell i: the face fluxes, the flux-balance term -U5_i (v_i . closure_i) / V_i, and the
 // source integrated over the cell quadrature (src / jac: the kSaGp weighted point values, summed in
-// point order); the source Jacobian into srcJac
+// point order), into r, and the source Jacobian into sj
 template <class T>
-DG_HD void sa_cell_rhs(int64_t i, const HotView<T>& h, const SaView<T>& sa, const double* src, const double* jac) {
+DG_HD void sa_cell_rhs(int64_t i, const HotView<T>& h, const SaView<T>& sa, const double* src, const double* jac, double& r,
+                       double& sj) {
   double s = 0;
   for (int k = 0; k < h.nfmax; k++) {
     const int32_t sf = h.cellFace[aos(i, k, h.nfmax)];
@@ -421,14 +422,15 @@ DG_HD void sa_cell_rhs(int64_t i, const HotView<T>& h, const SaView<T>& sa, cons
   load4<T>(&h.u[i * 4], U);
   const double u5 = sa.u[i];
   const double vn = (U[1] * h.closure[2 * i] + U[2] * h.closure[2 * i + 1]) / U[0];
-  double r = (s - u5 * vn) / h.vol[i];
-  double sv = 0, sj = 0;
+  const double iv = 1.0 / h.vol[i];
+  double sv = 0;
+  sj = 0;
   for (int ig = 0; ig < kSaGp; ig++) {
     sv += src[ig];
     sj += jac[ig];
   }
-  sa.rhs[i] = r + sv / h.vol[i];
-  sa.srcJac[i] = sj / h.vol[i];
+  r = ((s - u5 * vn) + sv) * iv;
+  sj *= iv;
 }
 
 // EvaluateDt face part for an SA context (DNDS_FV_EulerEvaluator.cpp:25-137): the viscous spectral
