@@ -28,6 +28,7 @@ namespace {
 constexpr int kBlock = 256;
 inline unsigned grid_for(int64_t n) { return (unsigned)((n + kBlock - 1) / kBlock); }
 
+constexpr int64_t kSmallCells = 262144, kSplitMaxFaces = 16384;  // dndsg_ctx::small, splitFlux
 // device scalar slots
 enum { S_T = 0, S_DT = 1, S_DTMIN = 2, S_TEVAL = 3, S_ZERO = 4, S_INC = 5, S_NSLOT = 8 };
 }  // namespace
@@ -118,6 +119,17 @@ struct dndsg_ctx {
   std::vector<void*> allocs;
 
   size_t tsize() const { return fp32 ? sizeof(float) : sizeof(double); }
+  // meshes whose passes are short against a launch: their kernels are launched as programmatic dependents
+  // (FP32 residual on 94,577 quads 113 -> 97 us, on 344,776 quads 174 -> 165, limited FP64 step on 154,714
+  // triangles 473 -> 441, FP64 step on 1,672 triangles 52 -> 36).  On larger ones the early blocks of the next
+  // kernel take room from the running one (dual-time step on 524,288 triangles 3838 -> 4276 us, FP32 step on
+  // 2,097,152 1495 -> 1735), and a captured graph has its short edges already (five FP64 steps on 26,496
+  // triangles 300 -> 346 us with the attribute)
+  bool capturing = false;
+  bool small() const { return N <= kSmallCells && !capturing; }
+  // face passes of few warps per SM: a thread per Gauss point (ten FP64 steps on 1,600 quads 361 -> 337 us;
+  // with three times the blocks a pass still is one wave of the device)
+  bool splitFlux() const { return F <= kSplitMaxFaces; }
 };
 
 namespace {
@@ -166,6 +178,23 @@ __device__ __forceinline__ double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+// a launch whose kernel starts with pdl_enter(); pdl: as a programmatic dependent of the stream's previous
+// kernel, so that its launch and block start overlap that kernel's run
+template <class... P, class... A>
+void launch(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, bool pdl, A... a) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k, P(a)...);
+}
+
 // ------------------------------------------------------------------ setup kernels
 __global__ void k_setup_cell(MeshView m, SetupParams p, CellSetup* cells, double* vol, double* bary, int* bad) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -279,6 +308,7 @@ __global__ void __launch_bounds__(TILE * 4) k_vr_tma4(HotView<T> h, unsigned* fl
   __shared__ __align__(8) unsigned long long bar;
   constexpr int E = NF * 30;
   const int tid = threadIdx.x;
+  pdl_launch_next();
   const int64_t c0 = (int64_t)blockIdx.x * TILE;
   constexpr uint32_t bytes = (uint32_t)(TILE * E * sizeof(T));
   const uint32_t b = smem_u32(&bar);
@@ -291,6 +321,7 @@ __global__ void __launch_bounds__(TILE * 4) k_vr_tma4(HotView<T> h, unsigned* fl
     mbar_expect_tx(b, bytes);
     bulk_g2s(smem_u32(dsm), h.vrOp + c0 * E, bytes, b);
   }
+  pdl_wait_previous();  // the operator tile is constant; the state is not
   const int cl = tid >> 2, v = tid & 3;
   const int64_t i = c0 + cl;
   VrPre<T, NF> pre;
@@ -311,6 +342,7 @@ __global__ void __launch_bounds__(TILE * 4) k_vr_tma4(HotView<T> h, unsigned* fl
 
 template <class T>
 __global__ void k_vr_wall_fixup(HotView<T> h, const int32_t* cells, int64_t n) {  // 4 threads per wall cell
+  pdl_enter();
   int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k < 4 * n) vr_wall_fixup<T>(cells[k >> 2], (int)(k & 3), h);
 }
@@ -404,6 +436,7 @@ template <class T, int RIEMANN, bool BND, bool DT = false>
 __global__ void __launch_bounds__(kBlock, (sizeof(T) == 4 && RIEMANN == 1 && !BND) ? 4 : ((sizeof(T) == 4 && !BND) ? 3 : 2)) k_face_flux(HotView<T> h, int64_t f0, int64_t f1, double* scal,
                                                          int useDev, double tHost, double c, unsigned* flags,
                                                          unsigned long long* nred) {
+  pdl_enter();
   int64_t f = f0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int r = 0;
   bool bad = false;
@@ -432,11 +465,59 @@ __global__ void __launch_bounds__(kBlock, (sizeof(T) == 4 && RIEMANN == 1 && !BN
   }
 }
 
+// the same for small meshes, one thread per (face, Gauss point) and interior and boundary faces in one
+// launch (blocks past innerBlocks take the boundary).  With few faces per SM the pass is the latency of one
+// thread's chain of some hundred dependent FP64 operations per point; the third thread of a face sums the
+// points in their order.
+constexpr int kSplitFaces = 64;
+template <class T, int RIEMANN, bool DT>
+__global__ void __launch_bounds__(kSplitFaces * 3) k_face_flux_split(HotView<T> h, int64_t Fi, int64_t F, unsigned innerBlocks,
+                                                                     double* scal, int useDev, double tHost, double c,
+                                                                     unsigned* flags, unsigned long long* nred) {
+  __shared__ double part[kSplitFaces * 3][4];
+  pdl_enter();
+  const bool bnd = blockIdx.x >= innerBlocks;
+  const int64_t f = (bnd ? Fi + (blockIdx.x - innerBlocks) * (int64_t)kSplitFaces : blockIdx.x * (int64_t)kSplitFaces) +
+                    threadIdx.x / 3, f1 = bnd ? F : Fi;
+  const int g = threadIdx.x % 3;
+  if constexpr (DT) {
+    if (f < f1 && g == 0) {
+      if (f == 0 || f == Fi) reset_dtmin(scal);
+      dt_face<T>(f, h);
+    }
+    __syncthreads();
+  }
+  int r = 0;
+  bool bad = false;
+  if (f < f1) {
+    const double t = stage_time(scal, useDev, tHost, c);
+    double o[4];
+    r = bnd ? face_flux_point<T, RIEMANN, true>(f, g, h, t, o, bad) : face_flux_point<T, RIEMANN, false>(f, g, h, t, o, bad);
+    for (int k = 0; k < 4; k++) part[threadIdx.x][k] = o[k];
+  }
+  __syncthreads();
+  if (f < f1 && g == 0) {
+    double a[4];
+    for (int k = 0; k < 4; k++) {
+      a[k] = (part[threadIdx.x][k] + part[threadIdx.x + 1][k]) + part[threadIdx.x + 2][k];
+      if (!(a[k] == a[k])) bad = true;
+    }
+    store_row(&h.flux[f * 4], a);
+  }
+  const unsigned anyBad = __ballot_sync(0xffffffffu, bad);
+  const int rs = __reduce_add_sync(0xffffffffu, r);
+  if ((threadIdx.x & 31) == 0) {
+    if (anyBad) atomicOr(flags, 1u);
+    if (rs) atomicAdd(nred, (unsigned long long)rs);
+  }
+}
+
 // the same with the Navier-Stokes viscous term (contexts with mu_gas > 0)
 template <class T, int RIEMANN, bool BND>
 __global__ void __launch_bounds__(kBlock) k_face_flux_vis(HotView<T> h, int64_t f0, int64_t f1, const double* scal,
                                                           int useDev, double tHost, double c, unsigned* flags,
                                                           unsigned long long* nred) {
+  pdl_enter();
   int64_t f = f0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int r = 0;
   bool bad = false;
@@ -470,6 +551,7 @@ __global__ void k_face_values(HotView<T> h, double t, double* out) {
 
 template <class T>
 __global__ void __launch_bounds__(kBlock) k_dt_face(HotView<T> h) {
+  pdl_enter();
   int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (f < h.F) dt_face<T>(f, h);
 }
@@ -482,6 +564,7 @@ __global__ void k_init_dtmin(double* scal) {
 // per-cell dt, global min, and (for a step) the copy u -> uLast
 template <class T, bool COPY_LAST>
 __global__ void __launch_bounds__(kBlock) k_dt_cell(HotView<T> h, double cfl, double maxDt, double* scal) {
+  pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   double d = 1e300;
   if (i < h.N) {
@@ -527,7 +610,8 @@ __global__ void k_fill_dt(double* dt, int64_t n, const double* scal) {
 // quads 394 -> 361 us) and no pass that copies the means.  One thread writes each scalar; no other thread of
 // the launch reads that one
 template <class T, int STAGE, bool STEP = false>
-__global__ void __launch_bounds__(kBlock) k_cell_update(HotView<T> h, double* scal, double tEnd = 0.0) {
+__global__ void __launch_bounds__(kBlock) k_cell_update(HotView<T> h, double* scal, double tEnd) {
+  pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= h.N) return;
   double r[4];
@@ -645,11 +729,10 @@ int run_vr(dndsg_ctx* c, bool inc, cudaStream_t s) {
   } else if (r1) {
     constexpr int TILE = vr_tile<T>();
     const size_t smem = (size_t)TILE * c->nfmax * 30 * sizeof(T);
-    if (c->nfmax == 3)
-      k_vr_tma4<T, TILE, 3><<<(unsigned)((c->N + TILE - 1) / TILE), TILE * 4, smem, s>>>(h, c->flags);
-    else
-      k_vr_tma4<T, TILE, 4><<<(unsigned)((c->N + TILE - 1) / TILE), TILE * 4, smem, s>>>(h, c->flags);
-    if (c->nWallCells > 0) k_vr_wall_fixup<T><<<grid_for(4 * c->nWallCells), kBlock, 0, s>>>(h, c->wallCells, c->nWallCells);
+    const unsigned grid = (unsigned)((c->N + TILE - 1) / TILE);
+    launch(c->nfmax == 3 ? k_vr_tma4<T, TILE, 3> : k_vr_tma4<T, TILE, 4>, grid, TILE * 4, smem, s, c->small(), h, c->flags);
+    if (c->nWallCells > 0)
+      launch(k_vr_wall_fixup<T>, (unsigned)((4 * c->nWallCells + 63) / 64), 64, 0, s, c->small(), h, c->wallCells, c->nWallCells);
   } else {
     k_vr<T, false, false><<<grid_for(c->N), kBlock, 0, s>>>(h, nullptr);
   }
@@ -713,17 +796,19 @@ void run_limiter(dndsg_ctx* c, int ifAll, cudaStream_t s) {
 template <class T, bool DT>
 void launch_flux_inviscid(dndsg_ctx* c, const HotView<T>& h, int useDev, double tHost, double cst, cudaStream_t s) {
   const int64_t Fi = c->Fi, F = c->F;
-  if (c->s.riemann == 2) {
-    if (Fi > 0)
-      k_face_flux<T, 2, false, DT><<<grid_for(Fi), kBlock, 0, s>>>(h, 0, Fi, c->scal, useDev, tHost, cst, c->flags, c->nreduced);
-    if (F > Fi)
-      k_face_flux<T, 2, true, DT><<<grid_for(F - Fi), kBlock, 0, s>>>(h, Fi, F, c->scal, useDev, tHost, cst, c->flags, c->nreduced);
-  } else {
-    if (Fi > 0)
-      k_face_flux<T, 1, false, DT><<<grid_for(Fi), kBlock, 0, s>>>(h, 0, Fi, c->scal, useDev, tHost, cst, c->flags, c->nreduced);
-    if (F > Fi)
-      k_face_flux<T, 1, true, DT><<<grid_for(F - Fi), kBlock, 0, s>>>(h, Fi, F, c->scal, useDev, tHost, cst, c->flags, c->nreduced);
+  const bool hllc = c->s.riemann == 2;
+  if (c->splitFlux()) {
+    const unsigned ni = (unsigned)((Fi + kSplitFaces - 1) / kSplitFaces), nb = (unsigned)((F - Fi + kSplitFaces - 1) / kSplitFaces);
+    launch(hllc ? k_face_flux_split<T, 2, DT> : k_face_flux_split<T, 1, DT>, ni + nb, kSplitFaces * 3, 0, s, c->small(), h, Fi, F, ni,
+           c->scal, useDev, tHost, cst, c->flags, c->nreduced);
+    return;
   }
+  if (Fi > 0)
+    launch(hllc ? k_face_flux<T, 2, false, DT> : k_face_flux<T, 1, false, DT>, grid_for(Fi), kBlock, 0, s, c->small(), h, (int64_t)0, Fi,
+           c->scal, useDev, tHost, cst, c->flags, c->nreduced);
+  if (F > Fi)
+    launch(hllc ? k_face_flux<T, 2, true, DT> : k_face_flux<T, 1, true, DT>, (unsigned)((F - Fi + 63) / 64), 64, 0, s, c->small(), h, Fi, F,
+           c->scal, useDev, tHost, cst, c->flags, c->nreduced);
 }
 
 // the face-flux launches of EvaluateRHS over the arrays of h (interior faces, then boundary faces).
@@ -783,10 +868,10 @@ int run_step(dndsg_ctx* c, double cfl, double tEnd, cudaStream_t s) {
     if (c->s.limiter) run_limiter<T>(c, 0, s);
     HotView<T> h = view<T>(c);
     launch_flux<T>(c, 1, 0.0, cst[stg], s, stg == 0 && fuseDt);
-    if (stg == 0 && fuseDt) k_dt_cell<T, false><<<grid_for(c->N), kBlock, 0, s>>>(h, cfl, 1e100, c->scal);
-    if (stg == 0) k_cell_update<T, 0, true><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal, tEnd);
-    else if (stg == 1) k_cell_update<T, 1, true><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal, tEnd);
-    else k_cell_update<T, 2, true><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal, tEnd);
+    if (stg == 0 && fuseDt) launch(k_dt_cell<T, false>, grid_for(c->N), kBlock, 0, s, c->small(), h, cfl, 1e100, c->scal);
+    if (stg == 0) launch(k_cell_update<T, 0, true>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, tEnd);
+    else if (stg == 1) launch(k_cell_update<T, 1, true>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, tEnd);
+    else launch(k_cell_update<T, 2, true>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, tEnd);
   }
   return 0;
 }
@@ -797,9 +882,9 @@ void run_rk_stage(dndsg_ctx* c, int stg, cudaStream_t s) {
   const double cst[3] = {0.0, 1.0, 0.5};
   launch_flux<T>(c, 1, 0.0, cst[stg], s);
   HotView<T> h = view<T>(c);
-  if (stg == 0) k_cell_update<T, 0><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
-  else if (stg == 1) k_cell_update<T, 1><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
-  else k_cell_update<T, 2><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
+  if (stg == 0) launch(k_cell_update<T, 0>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
+  else if (stg == 1) launch(k_cell_update<T, 1>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
+  else launch(k_cell_update<T, 2>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
 }
 
 // halo exchange buffers: PACK buf[k][0..w) = a[cells[k]][0..w), else the reverse
@@ -817,7 +902,7 @@ template <class T>
 int run_rhs(dndsg_ctx* c, double t, cudaStream_t s) {
   launch_flux<T>(c, 0, t, 0.0, s);
   HotView<T> h = view<T>(c);
-  k_cell_update<T, -1><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
+  launch(k_cell_update<T, -1>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
   return 0;
 }
 
@@ -1470,10 +1555,12 @@ int dndsg_ssprk3_steps(dndsg_ctx* c, double cfl, double t_end, int64_t n, void* 
       if (!c->capStream) DG_CUDA(c, cudaStreamCreateWithFlags(&c->capStream, cudaStreamNonBlocking));
       void* urec0 = c->urec;
       DG_CUDA(c, cudaStreamBeginCapture(c->capStream, cudaStreamCaptureModeThreadLocal));
+      c->capturing = true;
       for (int k = 0; k < 2; k++) {  // six buffer swaps: urec is back in its buffer afterwards
         if (c->fp32) run_step<float>(c, cfl, t_end, c->capStream);
         else run_step<double>(c, cfl, t_end, c->capStream);
       }
+      c->capturing = false;
       cudaGraph_t graph = nullptr;
       const cudaError_t e = cudaStreamEndCapture(c->capStream, &graph);
       if (e != cudaSuccess) return fail(c, DNDSG_CUDA_ERROR, std::string("step capture: ") + cudaGetErrorString(e));
@@ -1726,7 +1813,7 @@ void run_rhs_noalloc(dndsg_ctx* c, const double* u, const void* urec, double* rh
   h.rhs = rhs;
   h.flux = scratch;
   launch_flux_h<T>(c, h, 0, t, 0.0, s);
-  k_cell_update<T, -1><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
+  launch(k_cell_update<T, -1>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
@@ -2005,9 +2092,9 @@ int run_step_tol(dndsg_ctx* c, const dndsg_mlp* m, double cfl, double tEnd, doub
     if (c->s.limiter) run_limiter<T>(c, 0, s);
     launch_flux<T>(c, 1, 0.0, cst[stg], s);
     HotView<T> h = view<T>(c);
-    if (stg == 0) k_cell_update<T, 0><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
-    else if (stg == 1) k_cell_update<T, 1><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
-    else k_cell_update<T, 2><<<grid_for(c->N), kBlock, 0, s>>>(h, c->scal);
+    if (stg == 0) launch(k_cell_update<T, 0>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
+    else if (stg == 1) launch(k_cell_update<T, 1>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
+    else launch(k_cell_update<T, 2>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
   }
   k_advance_time<<<1, 1, 0, s>>>(c->scal);
   if (sweepsOut) *sweepsOut = total;
@@ -2310,6 +2397,7 @@ __device__ __forceinline__ double impl_combine(const ImplComb& c, int64_t e, dou
 template <class T>
 __global__ void __launch_bounds__(kBlock) k_implicit_cell(HotView<T> h, ImplComb cb, double cfl, double dtPhysInv,
                                                           double alpha, double* Dinv, double* D, double* resAcc) {
+  pdl_enter();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < 16) resAcc[i] = 0.0;
   if (i >= h.N) return;
@@ -2751,7 +2839,7 @@ void implicit_rhs(dndsg_ctx* c, double cfl, double t, int nRec, const ImplComb& 
   for (int k = 0; k < nRec; k++) run_vr<T>(c, false, s);
   if (c->s.limiter) run_limiter<T>(c, 0, s);
   launch_flux<T>(c, 0, t, 0.0, s, !viscous);
-  k_implicit_cell<T><<<grid_for(c->N), kBlock, 0, s>>>(view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
+  launch(k_implicit_cell<T>, grid_for(c->N), kBlock, 0, s, c->small(), view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
 }
 
 // ImplicitBDFDualTimeStep::Step (DNDS_ODE.hpp:444-486), one pseudo-time iteration at order 1, with
@@ -3027,7 +3115,7 @@ inline unsigned sa_rhs_grid(int64_t n) { return (unsigned)((n + kSaRhsCells - 1)
 template <class T>
 void run_rhs_sa(dndsg_ctx* c, cudaStream_t s) {
   launch_flux_sa<T>(c, s);
-  k_cell_update<T, -1><<<grid_for(c->N), kBlock, 0, s>>>(view<T>(c), c->scal);
+  launch(k_cell_update<T, -1>, grid_for(c->N), kBlock, 0, s, c->small(), view<T>(c), c->scal, 0.0);
   k_sa_cell_rhs<T, false><<<sa_rhs_grid(c->N), kSaRhsCells * kSaGp, 0, s>>>(view<T>(c), sa_view<T>(c), ImplComb{}, 0.0, nullptr, nullptr);
 }
 
@@ -3038,7 +3126,7 @@ void implicit_rhs_sa(dndsg_ctx* c, double cfl, int nRec, const ImplComb& cb, con
   k_dt_face_sa<T><<<grid_for(c->F), kBlock, 0, s>>>(view<T>(c), sa_view<T>(c));
   for (int k = 0; k < nRec; k++) run_vr_sa<T>(c, s);
   launch_flux_sa<T>(c, s);
-  k_implicit_cell<T><<<grid_for(c->N), kBlock, 0, s>>>(view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
+  launch(k_implicit_cell<T>, grid_for(c->N), kBlock, 0, s, c->small(), view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
   k_sa_cell_rhs<T, true><<<sa_rhs_grid(c->N), kSaRhsCells * kSaGp, 0, s>>>(view<T>(c), sa_view<T>(c), cb5, alpha, c->Dmat, DS);
 }
 

@@ -30,6 +30,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
   return done != 0;
 }
+// programmatic dependent launch: lets the next kernel of the stream be launched while this one runs, and
+// waits until the one before it is complete (both do nothing in a launch without that attribute)
+__device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter() {
+  pdl_launch_next();
+  pdl_wait_previous();
+}
 // thread-block clusters: a shared-memory address of this block in block `rank`, and the hardware barrier of all threads of the cluster (release / acquire)
 __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
   uint32_t r;

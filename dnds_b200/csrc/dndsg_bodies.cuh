@@ -488,6 +488,30 @@ DG_HD void face_increments(int64_t f, int32_t L, int32_t R, const HotView<T>& h,
   else for (int g = 0; g < 3; g++) for (int v = 0; v < 4; v++) incR[g][v] = T(0);
 }
 
+// the reconstruction increments of both cells at face Gauss point g (face_increments for one point,
+// the same sums)
+template <class T>
+DG_HD void face_increment_point(int64_t f, int g, int32_t L, int32_t R, const HotView<T>& h, T incL[4], T incR[4]) {
+  for (int v = 0; v < 4; v++) incL[v] = incR[v] = T(0);
+  T phi[5];
+  FaceBasisSide<T>(h.faceBasis, f, 0).at(g, phi);
+  const T* rl = &h.urec[(int64_t)L * 20];
+  for (int q = 0; q < 5; q++) {
+    T row[4];
+    load_row(rl + 4 * q, row);
+    for (int v = 0; v < 4; v++) incL[v] += phi[q] * row[v];
+  }
+  if (R >= 0) {
+    FaceBasisSide<T>(h.faceBasis, f, 1).at(g, phi);
+    const T* rr = &h.urec[(int64_t)R * 20];
+    for (int q = 0; q < 5; q++) {
+      T row[4];
+      load_row(rr + 4 * q, row);
+      for (int v = 0; v < 4; v++) incR[v] += phi[q] * row[v];
+    }
+  }
+}
+
 // positivity-compressed states at gauss point g (CompressRecPart, boundary state on a boundary face)
 template <class T, bool BND = true>
 DG_HD int gp_states(int64_t f, int32_t R, const HotView<T>& h, double t, double nx, double ny, const double uL[4],
@@ -765,6 +789,43 @@ DG_HD bool side_state32(const FaceMeans32& m, int s, float g1, float d[4], Side3
 // q = sqrt(rho_R / rho_L).  The pass is bound by instruction issue, so the velocities, pressures and 1 / rho
 // of the flux differences serve the Roe averages too, and the sum over the points stays in the normal frame
 // (with the launches saved in the step: 1.523 -> 1.421 ms per FP32 step on 2,097,152 triangles).
+// the point's part of the flux difference, weighted, added to acc (normal frame)
+DG_HD int roe_point32(const FaceMeans32& m, const float incL[4], const float incR[4], float nx, float ny, float g1, float dl,
+                      int g, float acc[4], bool& bad) {
+  int nred = 0;
+  float dL[4], dR[4];
+  to_normal_frame(incL, nx, ny, dL);
+  to_normal_frame(incR, nx, ny, dR);
+  Side32 l, r;
+  nred += side_state32(m, 0, g1, dL, l) ? 1 : 0;
+  nred += side_state32(m, 1, g1, dR, r) ? 1 : 0;
+  if (!(l.U[0] > 0.f && r.U[0] > 0.f)) bad = true;
+  // Roe average and wave strengths of dU = (uR - uL) + (dR - dL)
+  const float q = sqrt32(r.U[0] * l.ir), i1 = rcp32(1.f + q);
+  const float u = (l.u + q * r.u) * i1, v = (l.v + q * r.v) * i1;
+  const float H = ((l.U[3] + l.p) * l.ir + q * ((r.U[3] + r.p) * r.ir)) * i1;
+  const float vs = u * u + v * v;
+  const float a2 = g1 * (H - 0.5f * vs);
+  const float ia = rsqrt32(a2), a = a2 * ia;
+  float lam0 = fabsf(u - a), lam1 = fabsf(u), lam3 = fabsf(u + a);
+  const float thr = fmaxf(0.05f * (sqrt32(vs) + a), dl), thrS = thr * thr, ht = 0.5f * rcp32(thr);
+  if (lam0 < thr) lam0 = (lam0 * lam0 + thrS) * ht;
+  if (lam3 < thr) lam3 = (lam3 * lam3 + thrS) * ht;
+  const float d0 = m.dmean[0] + (dR[0] - dL[0]), d1 = m.dmean[1] + (dR[1] - dL[1]);
+  const float d2 = m.dmean[2] + (dR[2] - dL[2]), d3 = m.dmean[3] + (dR[3] - dL[3]);
+  const float al2 = d2 - v * d0;
+  const float d3b = d3 - al2 * v;
+  const float al1 = g1 * (ia * ia) * (d0 * (H - u * u) + u * d1 - d3b);
+  const float al0 = (d0 * (u + a) - d1 - a * al1) * (0.5f * ia);
+  const float al3 = d0 - (al0 + al1);
+  const float w0 = lam0 * al0, w1 = lam1 * al1, w2 = lam1 * al2, w3 = lam3 * al3, ws = w0 + w1 + w3;
+  const float jw = g == 1 ? (float)(8.0 / 18.0) : (float)(5.0 / 18.0);
+  acc[0] += jw * (l.D[0] + r.D[0] - ws);
+  acc[1] += jw * (l.D[1] + r.D[1] - ((u - a) * w0 + u * w1 + (u + a) * w3));
+  acc[2] += jw * (l.D[2] + r.D[2] - (v * ws + w2));
+  acc[3] += jw * (l.D[3] + r.D[3] - ((H - u * a) * w0 + 0.5f * vs * w1 + v * w2 + (H + u * a) * w3));
+  return nred;
+}
 DG_HD int face_flux_roe_delta32(int64_t f, const HotView<float>& h, double out[4], bool& bad) {
   const int32_t L = h.faceL[f], R = h.faceR[f];
   const double nxd = h.faceNormal[2 * f], nyd = h.faceNormal[2 * f + 1], area = h.faceArea[f];
@@ -779,39 +840,7 @@ DG_HD int face_flux_roe_delta32(int64_t f, const HotView<float>& h, double out[4
   face_means32<false>(uL, uR, nxd, nyd, h.gamma, m, nullptr);
   int nred = 0;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int g = 0; g < 3; g++) {
-    float dL[4], dR[4];
-    to_normal_frame(incL[g], nx, ny, dL);
-    to_normal_frame(incR[g], nx, ny, dR);
-    Side32 l, r;
-    nred += side_state32(m, 0, g1, dL, l) ? 1 : 0;
-    nred += side_state32(m, 1, g1, dR, r) ? 1 : 0;
-    if (!(l.U[0] > 0.f && r.U[0] > 0.f)) bad = true;
-    // Roe average and wave strengths of dU = (uR - uL) + (dR - dL)
-    const float q = sqrt32(r.U[0] * l.ir), i1 = rcp32(1.f + q);
-    const float u = (l.u + q * r.u) * i1, v = (l.v + q * r.v) * i1;
-    const float H = ((l.U[3] + l.p) * l.ir + q * ((r.U[3] + r.p) * r.ir)) * i1;
-    const float vs = u * u + v * v;
-    const float a2 = g1 * (H - 0.5f * vs);
-    const float ia = rsqrt32(a2), a = a2 * ia;
-    float lam0 = fabsf(u - a), lam1 = fabsf(u), lam3 = fabsf(u + a);
-    const float thr = fmaxf(0.05f * (sqrt32(vs) + a), dl), thrS = thr * thr, ht = 0.5f * rcp32(thr);
-    if (lam0 < thr) lam0 = (lam0 * lam0 + thrS) * ht;
-    if (lam3 < thr) lam3 = (lam3 * lam3 + thrS) * ht;
-    const float d0 = m.dmean[0] + (dR[0] - dL[0]), d1 = m.dmean[1] + (dR[1] - dL[1]);
-    const float d2 = m.dmean[2] + (dR[2] - dL[2]), d3 = m.dmean[3] + (dR[3] - dL[3]);
-    const float al2 = d2 - v * d0;
-    const float d3b = d3 - al2 * v;
-    const float al1 = g1 * (ia * ia) * (d0 * (H - u * u) + u * d1 - d3b);
-    const float al0 = (d0 * (u + a) - d1 - a * al1) * (0.5f * ia);
-    const float al3 = d0 - (al0 + al1);
-    const float w0 = lam0 * al0, w1 = lam1 * al1, w2 = lam1 * al2, w3 = lam3 * al3, ws = w0 + w1 + w3;
-    const float jw = g == 1 ? (float)(8.0 / 18.0) : (float)(5.0 / 18.0);
-    acc[0] += jw * (l.D[0] + r.D[0] - ws);
-    acc[1] += jw * (l.D[1] + r.D[1] - ((u - a) * w0 + u * w1 + (u + a) * w3));
-    acc[2] += jw * (l.D[2] + r.D[2] - (v * ws + w2));
-    acc[3] += jw * (l.D[3] + r.D[3] - ((H - u * a) * w0 + 0.5f * vs * w1 + v * w2 + (H + u * a) * w3));
-  }
+  for (int g = 0; g < 3; g++) nred += roe_point32(m, incL[g], incR[g], nx, ny, g1, dl, g, acc, bad);
   from_normal_frame(acc, nx, ny);
   const double ha = -0.5 * area;
   for (int k = 0; k < 4; k++) {
@@ -834,6 +863,69 @@ DG_HD int face_flux_roe_delta32(int64_t f, const HotView<float>& h, double out[4
 // increments 1/2 (F(UL) - F(uL) + F(UR) - F(uR)); the jumps dF, du, dp are formed from the FP64 mean
 // difference plus the FP32 increment difference, so every FP32 term's rounding scales with the
 // reconstruction increment or the jump across the face, not with the flux itself.
+DG_HD int hllc_point32(const FaceMeans32& m, const float dFmean[4], const float incL[4], const float incR[4], float nx, float ny,
+                       float gamma, float gm1, int g, float acc[4], bool& bad) {
+  int nred = 0;
+  float dL[4], dR[4];
+  to_normal_frame(incL, nx, ny, dL);
+  to_normal_frame(incR, nx, ny, dR);
+  Side32 l, r;
+  nred += side_state32(m, 0, gm1, dL, l) ? 1 : 0;
+  nred += side_state32(m, 1, gm1, dR, r) ? 1 : 0;
+  const float *UL = l.U, *UR = r.U, *DL = l.D, *DR = r.D;
+  if (!(UL[0] > 0.f && UR[0] > 0.f)) bad = true;
+  float J[4], dF[4], G[4];
+  for (int v = 0; v < 4; v++) {
+    J[v] = m.dmean[v] + (dR[v] - dL[v]);
+    dF[v] = dFmean[v] + (DR[v] - DL[v]);
+    G[v] = 0.5f * (DL[v] + DR[v]);
+  }
+  const float rL = UL[0], rR = UR[0], irL = l.ir, irR = r.ir;
+  const float uL1 = l.u, vL1 = l.v, uR1 = r.u, vR1 = r.v, pL = l.p, pR = r.p;
+  // exact jumps of the normal velocity, tangential velocity and pressure from J
+  const float du = (J[1] - uL1 * J[0]) * irR, dv = (J[2] - vL1 * J[0]) * irR;
+  const float dp = gm1 * (J[3] - 0.5f * (UL[1] * du + J[1] * uR1 + UL[2] * dv + J[2] * vR1));
+  const float q = sqrt32(rR * irL), i1 = rcp32(1.f + q);
+  const float um = (uL1 + q * uR1) * i1;
+  const float eta2 = 0.5f * q * i1 * i1;
+  const float dsqr = gamma * (pL * irL + q * (pR * irR)) * i1 + eta2 * du * du;
+  const float sq = sqrt32(dsqr), SL = um - sq, SR = um + sq;
+  if (0.f <= SL) {
+    for (int v = 0; v < 4; v++) G[v] -= 0.5f * dF[v];
+  } else if (SR <= 0.f) {
+    for (int v = 0; v < 4; v++) G[v] += 0.5f * dF[v];
+  } else {
+    const float div = rL * (SL - uL1) - rR * (SR - uR1);
+    const float sigL = fabsf(div) > 1e-37f ? (dp - rR * (SR - uR1) * du) * rcp32(div) : -uL1;  // S* = 0 if degenerate
+    const float SS = uL1 + sigL;
+    if (SS >= 0.f) {
+      const float d = SL - SS;
+      for (int v = 0; v < 4; v++) G[v] -= 0.5f * dF[v];
+      if (fabsf(d) >= 1e-37f) {
+        const float id = rcp32(d), a = sigL * id, chi = (SL - uL1) * id;
+        const float q1 = chi * sigL * rL, q3 = chi * sigL * (rL * SS + pL * rcp32(SL - uL1));
+        G[0] += SL * (a * UL[0]);
+        G[1] += SL * (a * UL[1] + q1);
+        G[2] += SL * (a * UL[2]);
+        G[3] += SL * (a * UL[3] + q3);
+      }
+    } else {
+      const float d = SR - SS, sigR = sigL - du;
+      for (int v = 0; v < 4; v++) G[v] += 0.5f * dF[v];
+      if (fabsf(d) >= 1e-37f) {
+        const float id = rcp32(d), a = sigR * id, chi = (SR - uR1) * id;
+        const float q1 = chi * sigR * rR, q3 = chi * sigR * (rR * SS + pR * rcp32(SR - uR1));
+        G[0] += SR * (a * UR[0]);
+        G[1] += SR * (a * UR[1] + q1);
+        G[2] += SR * (a * UR[2]);
+        G[3] += SR * (a * UR[3] + q3);
+      }
+    }
+  }
+  const float jw = g == 1 ? (float)(8.0 / 9.0) : (float)(5.0 / 9.0);
+  for (int k = 0; k < 4; k++) acc[k] += G[k] * jw;
+  return nred;
+}
 DG_HD int face_flux_hllc_delta32(int64_t f, const HotView<float>& h, double out[4], bool& bad) {
   const int32_t L = h.faceL[f], R = h.faceR[f];
   const double nxd = h.faceNormal[2 * f], nyd = h.faceNormal[2 * f + 1], area = h.faceArea[f];
@@ -849,71 +941,49 @@ DG_HD int face_flux_hllc_delta32(int64_t f, const HotView<float>& h, double out[
   face_means32<true>(uL, uR, nxd, nyd, h.gamma, m, dFmean);
   int nred = 0;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int g = 0; g < 3; g++) {
-    float dL[4], dR[4];
-    to_normal_frame(incL[g], nx, ny, dL);
-    to_normal_frame(incR[g], nx, ny, dR);
-    Side32 l, r;
-    nred += side_state32(m, 0, gm1, dL, l) ? 1 : 0;
-    nred += side_state32(m, 1, gm1, dR, r) ? 1 : 0;
-    const float *UL = l.U, *UR = r.U, *DL = l.D, *DR = r.D;
-    if (!(UL[0] > 0.f && UR[0] > 0.f)) bad = true;
-    float J[4], dF[4], G[4];
-    for (int v = 0; v < 4; v++) {
-      J[v] = m.dmean[v] + (dR[v] - dL[v]);
-      dF[v] = dFmean[v] + (DR[v] - DL[v]);
-      G[v] = 0.5f * (DL[v] + DR[v]);
-    }
-    const float rL = UL[0], rR = UR[0], irL = l.ir, irR = r.ir;
-    const float uL1 = l.u, vL1 = l.v, uR1 = r.u, vR1 = r.v, pL = l.p, pR = r.p;
-    // exact jumps of the normal velocity, tangential velocity and pressure from J
-    const float du = (J[1] - uL1 * J[0]) * irR, dv = (J[2] - vL1 * J[0]) * irR;
-    const float dp = gm1 * (J[3] - 0.5f * (UL[1] * du + J[1] * uR1 + UL[2] * dv + J[2] * vR1));
-    const float q = sqrt32(rR * irL), i1 = rcp32(1.f + q);
-    const float um = (uL1 + q * uR1) * i1;
-    const float eta2 = 0.5f * q * i1 * i1;
-    const float dsqr = gamma * (pL * irL + q * (pR * irR)) * i1 + eta2 * du * du;
-    const float sq = sqrt32(dsqr), SL = um - sq, SR = um + sq;
-    if (0.f <= SL) {
-      for (int v = 0; v < 4; v++) G[v] -= 0.5f * dF[v];
-    } else if (SR <= 0.f) {
-      for (int v = 0; v < 4; v++) G[v] += 0.5f * dF[v];
-    } else {
-      const float div = rL * (SL - uL1) - rR * (SR - uR1);
-      const float sigL = fabsf(div) > 1e-37f ? (dp - rR * (SR - uR1) * du) * rcp32(div) : -uL1;  // S* = 0 if degenerate
-      const float SS = uL1 + sigL;
-      if (SS >= 0.f) {
-        const float d = SL - SS;
-        for (int v = 0; v < 4; v++) G[v] -= 0.5f * dF[v];
-        if (fabsf(d) >= 1e-37f) {
-          const float id = rcp32(d), a = sigL * id, chi = (SL - uL1) * id;
-          const float q1 = chi * sigL * rL, q3 = chi * sigL * (rL * SS + pL * rcp32(SL - uL1));
-          G[0] += SL * (a * UL[0]);
-          G[1] += SL * (a * UL[1] + q1);
-          G[2] += SL * (a * UL[2]);
-          G[3] += SL * (a * UL[3] + q3);
-        }
-      } else {
-        const float d = SR - SS, sigR = sigL - du;
-        for (int v = 0; v < 4; v++) G[v] += 0.5f * dF[v];
-        if (fabsf(d) >= 1e-37f) {
-          const float id = rcp32(d), a = sigR * id, chi = (SR - uR1) * id;
-          const float q1 = chi * sigR * rR, q3 = chi * sigR * (rR * SS + pR * rcp32(SR - uR1));
-          G[0] += SR * (a * UR[0]);
-          G[1] += SR * (a * UR[1] + q1);
-          G[2] += SR * (a * UR[2]);
-          G[3] += SR * (a * UR[3] + q3);
-        }
-      }
-    }
-    const float jw = g == 1 ? (float)(8.0 / 9.0) : (float)(5.0 / 9.0);
-    for (int k = 0; k < 4; k++) acc[k] += G[k] * jw;
-  }
+  for (int g = 0; g < 3; g++) nred += hllc_point32(m, dFmean, incL[g], incR[g], nx, ny, gamma, gm1, g, acc, bad);
   from_normal_frame(acc, nx, ny);
   const double ha = -0.5 * area;
   for (int k = 0; k < 4; k++) {
     out[k] = ha * (m.FS[k] + (double)acc[k]);
     if (!(out[k] == out[k])) bad = true;
+  }
+  return nred;
+}
+
+// the part of Gauss point g in the face flux (face_flux and its FP32-bulk interior forms, one point of them;
+// point 1 of an FP32 interior face carries the means' central flux): the flux is the sum over the points
+template <class T, int RIEMANN, bool BND>
+DG_HD int face_flux_point(int64_t f, int g, const HotView<T>& h, double t, double c[4], bool& bad) {
+  const int32_t L = h.faceL[f], R = h.faceR[f];
+  const double nx = h.faceNormal[2 * f], ny = h.faceNormal[2 * f + 1], area = h.faceArea[f];
+  double uL[4], uR[4] = {0, 0, 0, 0};
+  load4<T>(&h.u[(int64_t)L * 4], uL);
+  if (!BND || R >= 0) load4<T>(&h.u[(int64_t)R * 4], uR);
+  T incL[4], incR[4];
+  face_increment_point(f, g, L, R, h, incL, incR);
+  int nred;
+  if constexpr (sizeof(T) == 4 && !BND) {
+    FaceMeans32 m;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f}, dFmean[4];
+    face_means32<RIEMANN == 2>(uL, uR, nx, ny, h.gamma, m, dFmean);
+    const float g1 = (float)(h.gamma - 1);
+    if (RIEMANN == 2) nred = hllc_point32(m, dFmean, incL, incR, (float)nx, (float)ny, (float)h.gamma, g1, g, acc, bad);
+    else nred = roe_point32(m, incL, incR, (float)nx, (float)ny, g1, (float)h.dLam[f], g, acc, bad);
+    from_normal_frame(acc, (float)nx, (float)ny);
+    const double ha = -0.5 * area;
+    for (int k = 0; k < 4; k++) c[k] = ha * ((g == 1 ? m.FS[k] : 0.0) + (double)acc[k]);
+  } else {
+    double UL[4], UR[4], a[4], b[4], F[4];
+    nred = gp_states<T, BND>(f, R, h, t, nx, ny, uL, uR, incL, incR, UL, UR);
+    to_normal_frame(UL, nx, ny, a);
+    to_normal_frame(UR, nx, ny, b);
+    if (!(a[0] > 0 && b[0] > 0)) bad = true;
+    if (RIEMANN == 2) hllc_flux(a, b, h.gamma, F);
+    else roe_flux(a, b, h.gamma, h.dLam[f], F);
+    from_normal_frame(F, nx, ny);
+    const double jw = -0.5 * area * l3_weight(g);
+    for (int k = 0; k < 4; k++) c[k] = F[k] * jw;
   }
   return nred;
 }

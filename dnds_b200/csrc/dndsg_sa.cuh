@@ -215,30 +215,6 @@ DG_HD void sa_point(const HotView<T>& h, const SaView<T>& sa, int64_t f, int g, 
   }
 }
 
-// the reconstruction increments of both cells at face Gauss point g (face_increments for one point,
-// the same sums)
-template <class T>
-DG_HD void face_increment_point(int64_t f, int g, int32_t L, int32_t R, const HotView<T>& h, T incL[4], T incR[4]) {
-  for (int v = 0; v < 4; v++) incL[v] = incR[v] = T(0);
-  T phi[5];
-  FaceBasisSide<T>(h.faceBasis, f, 0).at(g, phi);
-  const T* rl = &h.urec[(int64_t)L * 20];
-  for (int q = 0; q < 5; q++) {
-    T row[4];
-    load_row(rl + 4 * q, row);
-    for (int v = 0; v < 4; v++) incL[v] += phi[q] * row[v];
-  }
-  if (R >= 0) {
-    FaceBasisSide<T>(h.faceBasis, f, 1).at(g, phi);
-    const T* rr = &h.urec[(int64_t)R * 20];
-    for (int q = 0; q < 5; q++) {
-      T row[4];
-      load_row(rr + 4 * q, row);
-      for (int v = 0; v < 4; v++) incR[v] += phi[q] * row[v];
-    }
-  }
-}
-
 // face flux of an SA context at Gauss point g: the flow flux with the eddy viscosity and the U5
 // transport and diffusion (fluxFace, DNDS_FV_EulerEvaluator.hpp:371-591, SA branches), weighted;
 // the face flux is minus the sum of the three points' c / cS in point order
