@@ -1845,6 +1845,8 @@ extern "C" int dndsg_eval_rhs_noalloc(dndsg_ctx* c, const double* u, const void*
 struct dndsg_mlp {
   int device = 0;
   float *P = nullptr, *M = nullptr, *V = nullptr, *G = nullptr;
+  float* part = nullptr;  // per CTA of the training kernel: its gradients and loss [sms][kTrPart]
+  int sms = 148, rows = 0;
   __nv_bfloat16* W = nullptr;
   double* loss = nullptr;
   unsigned* flags = nullptr;  // kFlagTimeout from the tensor-core forward
@@ -2124,7 +2126,9 @@ int dndsg_mlp_create(int device, uint64_t seed, dndsg_mlp** out) {
   m->device = device;
   auto bail = [&](int code) { dndsg_mlp_destroy(m); return code; };
   if (cudaSetDevice(device) != cudaSuccess) return bail(DNDSG_CUDA_ERROR);
-  if (cudaMalloc(&m->P, sizeof(float) * kNParam) != cudaSuccess ||
+  cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
+  if (cudaMalloc(&m->part, sizeof(float) * kTrPart * m->sms) != cudaSuccess ||
+      cudaMalloc(&m->P, sizeof(float) * kNParam) != cudaSuccess ||
       cudaMalloc(&m->M, sizeof(float) * kNParam) != cudaSuccess ||
       cudaMalloc(&m->V, sizeof(float) * kNParam) != cudaSuccess ||
       cudaMalloc(&m->G, sizeof(float) * kNParam) != cudaSuccess ||
@@ -2156,7 +2160,7 @@ int dndsg_mlp_create(int device, uint64_t seed, dndsg_mlp** out) {
 void dndsg_mlp_destroy(dndsg_mlp* m) {
   if (!m) return;
   cudaSetDevice(m->device);
-  for (void* q : {(void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->W, (void*)m->loss, (void*)m->flags})
+  for (void* q : {(void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->part, (void*)m->W, (void*)m->loss, (void*)m->flags})
     if (q) cudaFree(q);
   delete m;
 }
@@ -2201,15 +2205,10 @@ int mlp_grad(dndsg_mlp* m, const float* X, const float* Tg, int64_t n, cudaStrea
                                      (int)sizeof(TrTcSmem)));
     m->attrTrain = true;
   }
-  DG_MCUDA(m, cudaMemsetAsync(m->G, 0, sizeof(float) * kNParam, s));
-  DG_MCUDA(m, cudaMemsetAsync(m->loss, 0, sizeof(double), s));
-  if (n == 0) return 0;
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
   const int64_t tiles = (n + kTcRows - 1) / kTcRows;
-  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(tiles, sms));  // one CTA per SM
-  k_mlp_train_tc<<<grid, kTrThreads, sizeof(TrTcSmem), s>>>(mlp_dev(m), X, Tg, n, 1.0f / (float)(n * kOut), m->G,
-                                                         m->loss, m->flags);
+  m->rows = (int)std::min<int64_t>(tiles, m->sms);  // one CTA per SM
+  k_mlp_train_tc<<<(unsigned)m->rows, kTrThreads, sizeof(TrTcSmem), s>>>(mlp_dev(m), X, Tg, n, 1.0f / (float)(n * kOut), m->part,
+                                                                        m->flags);
   DG_MCUDA(m, cudaGetLastError());
   return 0;
 }
@@ -2222,6 +2221,8 @@ int dndsg_mlp_gradient(dndsg_mlp* m, const float* X, const float* Tg, int64_t n,
   DG_MCUDA(m, cudaSetDevice(m->device));
   int rc = mlp_grad(m, X, Tg, n, st(s));
   if (rc) return rc;
+  k_mlp_reduce<<<(kNParam + kRedEntries - 1) / kRedEntries, 256, 0, st(s)>>>(m->part, m->rows, m->G, m->loss);
+  DG_MCUDA(m, cudaGetLastError());
   double l = 0;
   DG_MCUDA(m, cudaMemcpyAsync(&l, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st(s)));
   if (grad) DG_MCUDA(m, cudaMemcpyAsync(grad, m->G, sizeof(float) * kNParam, cudaMemcpyDeviceToHost, st(s)));
@@ -2242,8 +2243,8 @@ int dndsg_mlp_train_step(dndsg_mlp* m, const float* X, const float* Tg, int64_t 
   const double b1 = 0.9, b2 = 0.999;
   const float c1 = (float)(1.0 / (1.0 - std::pow(b1, (double)m->step)));
   const float c2 = (float)(1.0 / (1.0 - std::pow(b2, (double)m->step)));
-  k_mlp_adam<<<(kNParam + 255) / 256, 256, 0, st(s)>>>(m->P, m->M, m->V, m->G, m->W, lr, (float)b1, (float)b2, 1e-8f,
-                                                        c1, c2);
+  k_mlp_adam<<<(kNParam + kRedEntries - 1) / kRedEntries, 256, 0, st(s)>>>(m->P, m->M, m->V, m->part, m->rows, m->loss, m->W, lr,
+                                                                         (float)b1, (float)b2, 1e-8f, c1, c2);
   DG_MCUDA(m, cudaGetLastError());
   if (loss) {
     double l = 0;

@@ -424,12 +424,16 @@ __global__ void __launch_bounds__(kTcRows, 4) k_mlp_tc(MlpDev m, Src src, Dst ds
 
 // loss = mean over rows and the 20 outputs of (y - t)^2; gradients accumulate into G
 // ---------------------------------------------------------------- training on the tensor cores (tcgen05)
-// 128 rows per tile, 512 threads (16 columns of one row each); one CTA per SM holding all 512
-// tensor-memory columns:
-//   cols   0-191  the pre-activations z1, z2, z3 of the tile (FP32, kept for the backward pass)
-//   cols 192-255  the layer-4 output, then each backward product dH = dz W
-//   cols 256-511  dW1 .. dW4, accumulated over all of the CTA's tiles (M = 64: output unit u in
-//                 tensor-memory lane (u & 15) + 32 (u >> 4), the half-subpartition layout of M = 64)
+// 128 rows per tile.  A tile is a chain of eight products with an epilogue after each, so one CTA per SM keeps
+// two tiles in flight: two groups of 256 threads (row 32 (warp % 4) + lane, columns 32 (warp / 4 % 2) .. + 31)
+// work on a tile each, and one thread of a 17th warp issues the products of both, in the order in which the
+// groups' operands get ready (a group arrives on its `ready` barrier, the product commits to its `done`
+// barrier; no barrier of the whole block inside a tile).  All 512 tensor-memory columns:
+//   cols 128 g + 0-63    pre-activations z of group g's current layer (recomputed for the backward pass from the
+//                        stored operand: a product more instead of 128 columns for z1..z3)
+//   cols 128 g + 64-127  group g's backward product dH = dz W
+//   cols 256-511         dW1 .. dW4, accumulated over all of the CTA's tiles (M = 64: output unit u in
+//                        tensor-memory lane (u & 15) + 32 (u >> 4), the half-subpartition layout of M = 64)
 // Every operand stays in the one layout it is written in, the K-major core-matrix layout of the forward
 // products ([rows][64 units], cm_off); the products that need an operand transposed read it as an
 // MN-major operand instead (the same bytes: MN-blocks of 8 units 128 B apart, K-blocks of 8 rows 1024 B
@@ -437,18 +441,21 @@ __global__ void __launch_bounds__(kTcRows, 4) k_mlp_tc(MlpDev m, Src src, Dst ds
 //   forward       z_l  = h_{l-1} W_l^T       A h_{l-1} K-major, B W_l K-major         M 128, N 64 | 32, K 64
 //   input grad    dH   = dz_l W_l            A dz_l K-major,    B W_l MN-major         M 128, N 64, K 64 | 32
 //   weight grad   dW_l += dz_l^T h_{l-1}     A dz_l MN-major,   B h_{l-1} MN-major     M 64, N 64, K 128
-constexpr int kTrCols = 512;
+constexpr int kTrCols = 512, kTrGroups = 2, kTrGroup = 256;  // threads of a group
+constexpr int kTrThreads = kTrGroups * kTrGroup + 32;
 struct TrTcSmem {
   alignas(128) unsigned char Wf[3 * kHid * 128 + kOutP * 128];  // W_l [N][64], core-matrix layout
-  alignas(128) unsigned char X[kTcRows * 128];                   // the tile's features [128][64]
-  alignas(128) unsigned char H[3][kTcRows * 128];                // h1, h2, h3 [128][64]
-  alignas(128) unsigned char DZ[kTcRows * 128];                  // dz_l [128][64] (dz4: units >= 32 zero)
-  float gb[3 * kHid + kOutP];                                    // bias gradients of the CTA
-  uint64_t bar;
+  struct Tile {
+    alignas(128) unsigned char X[kTcRows * 128];     // the tile's features [128][64]
+    alignas(128) unsigned char H[3][kTcRows * 128];  // h1, h2, h3 [128][64]
+    alignas(128) unsigned char DZ[kTcRows * 128];    // dz_l [128][64] (dz4: units >= 32 zero)
+  } t[kTrGroups];
+  alignas(16) float b[3 * kHid + kOutP];  // biases
+  float gb[3 * kHid + kOutP];             // bias gradients of the CTA
+  uint64_t ready[kTrGroups], done[kTrGroups];
   uint32_t tmem;
-  unsigned char pad[8192];  // more than half of an SM's shared memory: one CTA per SM
 };
-static_assert(sizeof(TrTcSmem) > 233472 / 2, "one CTA per SM: it holds all 512 tensor-memory columns");
+static_assert(sizeof(TrTcSmem) > 233472 / 2 && sizeof(TrTcSmem) <= 227 * 1024, "one CTA per SM: it holds all 512 tensor-memory columns");
 
 // MN-major shared-memory descriptor of the same core-matrix layout: leading byte offset (K-blocks of 8 rows)
 // 1024, stride byte offset (MN-blocks of 8 units) 128, descriptor version 1, no swizzle
@@ -472,40 +479,46 @@ __device__ __forceinline__ void tr_bfly(float* v, int lane) {
     v[k] = keep + __shfl_xor_sync(0xffffffffu, send, O);
   }
 }
-// the sums over the warp's 32 rows of 16 column values v (destroyed), added into gb[0 .. 15]: four
-// butterfly rounds halve the columns a lane holds (8 + 4 + 2 + 1 shuffles, against 5 per column for
-// 16 separate reductions), a last one completes the sum, and 16 lanes add one column each
-__device__ __forceinline__ void tr_bias_sum16(float* v, float* gb) {
-  const int lane = threadIdx.x & 31;
+// the sums over the warp's 32 rows of 16 column values v (destroyed): four butterfly rounds halve the
+// columns a lane holds (8 + 4 + 2 + 1 shuffles, against 5 per column for 16 separate reductions), a last one
+// completes the sum; the lane returns that of column tr_sum_col(lane)
+__device__ __forceinline__ float tr_sum16(float* v, int lane) {
   tr_bfly<8, 16>(v, lane);
   tr_bfly<4, 8>(v, lane);
   tr_bfly<2, 4>(v, lane);
   tr_bfly<1, 2>(v, lane);
-  const float sum = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-  const int c = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
-  if ((lane & 1) == 0) atomicAdd(&gb[c], sum);
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
-// 16 values of a row, as BF16, into columns c0 .. c0 + 15 of a 64-wide K-major operand (c0 % 8 == 0)
-__device__ __forceinline__ void tc_store16(unsigned char* A, int row, int c0, const float* x) {
+__device__ __forceinline__ int tr_sum_col(int lane) {
+  return ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+}
+// whether an mbarrier phase is complete, without waiting
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// 32 values of a row, as BF16, into columns c0 .. c0 + 31 of a 64-wide K-major operand (c0 % 8 == 0)
+__device__ __forceinline__ void tc_store32(unsigned char* A, int row, int c0, const float* x) {
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
-    __nv_bfloat162 p[4];
-    for (int e = 0; e < 4; e++) p[e] = __floats2bfloat162_rn(x[8 * h + 2 * e], x[8 * h + 2 * e + 1]);
-    *reinterpret_cast<uint4*>(A + cm_off(row, c0 + 8 * h)) = *reinterpret_cast<uint4*>(p);
-  }
+  for (int h = 0; h < 4; h++) *reinterpret_cast<uint4*>(A + cm_off(row, c0 + 8 * h)) = pack8(x + 8 * h);
 }
 
-// 512 threads: warp w reads tensor-memory lanes 32 (w % 4) .. + 31, i.e. tile rows 32 q + lane (q = w % 4),
-// and handles columns 16 g .. 16 g + 15 (g = w / 4) of every 64-wide layer, so the epilogues of a
-// tile (bias, activation, operand store, bias-gradient sums) are spread over 16 warps
-constexpr int kTrThreads = 512;
+// Each CTA writes its gradients and loss to a row of `part` [gridDim][kTrPart], which k_mlp_adam or
+// k_mlp_reduce sums in row order (atomic adds of 148 CTAs to the same 14,560 addresses took longer, and their
+// order was not fixed).
+// Measured, eight steps of 65,536 rows: 954 us with one tile in flight per SM and atomics, 790 us with two
+// tiles, 579 us with the rows; a step of 1,048,576 rows 1.10 ms -> 0.65 ms.
+constexpr int kTrPart = kNParam + 4;  // parameters' gradients, then the loss in two floats (high and low part)
 __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(MlpDev m, const float* X, const float* Tg, int64_t n,
-                                                                float invCount, float* G, double* lossAcc,
-                                                                unsigned* flags) {
+                                                                float invCount, float* part, unsigned* flags) {
   extern __shared__ __align__(128) unsigned char raw[];
   TrTcSmem& S = *reinterpret_cast<TrTcSmem*>(raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int q = warp & 3, g = warp >> 2, row = 32 * q + lane;
   // the weights (row-major [N][64] BF16 in global memory) into the core-matrix layout, 16 B at a time
   for (int e = tid; e < (3 * kHid + kOutP) * 8; e += blockDim.x) {
     const int row = e >> 3, kc = e & 7;
@@ -514,173 +527,303 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(MlpDev m, const 
     *reinterpret_cast<uint4*>(S.Wf + layer * kHid * 128 + cm_off(rl, 8 * kc)) =
         *reinterpret_cast<const uint4*>(m.W + woff + rl * 64 + 8 * kc);
   }
-  for (int e = tid; e < 3 * kHid + kOutP; e += blockDim.x) S.gb[e] = 0.f;
-  const uint32_t bar = smem_u32(&S.bar);
-  if (warp == 0) {
+  for (int e = tid; e < 3 * kHid + kOutP; e += blockDim.x) {
+    S.gb[e] = 0.f;
+    S.b[e] = tc_bias_s(m.P, e < 3 * kHid ? e / kHid : 3, e < 3 * kHid ? e % kHid : e - 3 * kHid);
+  }
+  if (warp == kTrGroups * kTrGroup / 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.tmem)),
                  "r"(kTrCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    mbar_init(bar, 1);
+    for (int g = 0; g < kTrGroups; g++) {
+      mbar_init(smem_u32(&S.ready[g]), kTrGroup / 32);
+      mbar_init(smem_u32(&S.done[g]), 1);
+    }
     fence_mbar_init();
   }
+  proxy_fence_smem();  // the weights, to the tensor cores
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tb = S.tmem, lane0 = (uint32_t)(q * 32) << 16, col0 = 16u * g;
-  const uint32_t aX = smem_u32(S.X), aDZ = smem_u32(S.DZ), aW = smem_u32(S.Wf);
-  const uint32_t aH[3] = {smem_u32(S.H[0]), smem_u32(S.H[1]), smem_u32(S.H[2])};
-  constexpr uint32_t idFwd64 = umma_idesc_mk(kTcRows, kHid, false, false);
-  constexpr uint32_t idFwd32 = umma_idesc_mk(kTcRows, kOutP, false, false);
-  constexpr uint32_t idDH = umma_idesc_mk(kTcRows, kHid, false, true);
-  constexpr uint32_t idDW = umma_idesc_mk(64, kHid, true, true);
-  uint32_t phase = 0;
-  bool failed = false, first = true;
+  const uint32_t tb = S.tmem;
+  const int64_t tiles = (n + kTcRows - 1) / kTcRows, slots = (int64_t)kTrGroups * gridDim.x;
+  bool failed = false;
   double lossLocal = 0.0;
-  // all threads: make the operand writes visible to the tensor cores, then tid 0 issues `issue`
-  auto run = [&](auto issue) -> bool {
-    proxy_fence_smem();
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
-      tc_fence_after();
-      issue();
-      umma_commit(bar);
-    }
-    const bool ok = mbar_wait(bar, phase, kWaitLimit);
-    phase ^= 1u;
-    if (__syncthreads_or(!ok)) return false;
-    tc_fence_after();
-    return true;
-  };
-  for (int64_t tile = blockIdx.x; tile * kTcRows < n && !failed; tile += gridDim.x) {
-    const int64_t r0 = tile * kTcRows, r = r0 + row;
-    // x: coalesced 32-B pieces into the K-major operand
-    for (int e = tid; e < kTcRows * 8; e += blockDim.x) {
-      const int row = e >> 3, kc = e & 7;
-      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      if (r0 + row < n) {
-        const float4* q = reinterpret_cast<const float4*>(X + (r0 + row) * kIn + 8 * kc);
-        const float4 a = q[0], b = q[1];
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  if (warp == kTrGroups * kTrGroup / 32) {
+    // ---- the products of both groups.  Steps of a tile: 0-3 forward; 4-7 backward of layers 3..0: dW_l, dH and
+    // the previous layer's z again
+    if (lane == 0) {
+      constexpr uint32_t idFwd64 = umma_idesc_mk(kTcRows, kHid, false, false);
+      constexpr uint32_t idFwd32 = umma_idesc_mk(kTcRows, kOutP, false, false);
+      constexpr uint32_t idDH = umma_idesc_mk(kTcRows, kHid, false, true);
+      constexpr uint32_t idDW = umma_idesc_mk(64, kHid, true, true);
+      const uint32_t aW = smem_u32(S.Wf);
+      int64_t step[kTrGroups], steps[kTrGroups];
+      for (int g = 0; g < kTrGroups; g++) {
+        const int64_t first = blockIdx.x + (int64_t)g * gridDim.x;
+        step[g] = 0;
+        steps[g] = first < tiles ? 8 * ((tiles - first + slots - 1) / slots) : 0;
       }
-      __nv_bfloat162 p[4];
-      for (int j = 0; j < 4; j++) p[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-      *reinterpret_cast<uint4*>(S.X + cm_off(row, 8 * kc)) = *reinterpret_cast<uint4*>(p);
-    }
-    // ---- forward: z_l into tensor memory, h_l = SiLU(z_l + b_l) into H[l]
-    for (int l = 0; l < 4 && !failed; l++) {
-      const uint32_t dcol = l < 3 ? 64u * l : 192u;
-      const uint32_t aIn = l == 0 ? aX : aH[l - 1], aWl = aW + (uint32_t)l * kHid * 128;
-      if (!run([&] {
-            for (int ks = 0; ks < 4; ks++)
-              umma_bf16(tb + dcol, umma_desc(aIn + 256 * ks), umma_desc(aWl + 256 * ks), l < 3 ? idFwd64 : idFwd32,
-                        ks > 0);
-          })) {
-        failed = true;
-        break;
-      }
-      if (l < 3) {
-        float h[16];
-        tmem_ld16(tb + lane0 + dcol + col0, h);
-        tmem_wait_ld();
-        for (int k = 0; k < 16; k++) h[k] = silu(h[k] + tc_bias_s(m.P, l, col0 + k));
-        tc_store16(S.H[l], row, col0, h);
-      } else {  // y = z4 + b4, dz4 = 2 (y - t) / count on the 20 outputs (column groups 0 and 1)
-        float dz[16];
-        for (int k = 0; k < 16; k++) dz[k] = 0.f;
-        if (g < 2) {
-          float z[16];
-          tmem_ld16(tb + lane0 + 192 + col0, z);
-          tmem_wait_ld();
-          for (int k = 0; k < 16; k++) {
-            const int o = col0 + k;
-            if (o < kOut && r < n) {
-              const float dd = z[k] + tc_bias_s(m.P, 3, o) - Tg[r * kOut + o];
-              lossLocal += (double)dd * dd;
-              dz[k] = 2.f * dd * invCount;
-            }
-          }
-        }
-        tc_store16(S.DZ, row, col0, dz);  // units 32 .. 63 stay zero
-        if (g < 2) tr_bias_sum16(dz, S.gb + 3 * kHid + col0);
-      }
-    }
-    // ---- backward: dW_l += dz_l^T h_{l-1}; dH = dz_l W_l; dz_{l-1} = dH SiLU'(z_{l-1} + b_{l-1})
-    for (int l = 3; l >= 0 && !failed; l--) {
-      const uint32_t aPrev = l > 0 ? aH[l - 1] : aX, aWl = aW + (uint32_t)l * kHid * 128;
-      const bool acc = !first;
-      if (!run([&] {
+      unsigned started = 0;  // layers whose dW holds something
+      uint32_t idle = 0;
+      while (step[0] < steps[0] || step[1] < steps[1]) {
+        for (int g = 0; g < kTrGroups; g++) {
+          if (step[g] >= steps[g] || !mbar_test(smem_u32(&S.ready[g]), (uint32_t)step[g] & 1u)) continue;
+          tc_fence_after();
+          const uint32_t aX = smem_u32(S.t[g].X), aH = smem_u32(S.t[g].H[0]), aDZ = smem_u32(S.t[g].DZ);
+          const uint32_t z = tb + 128u * g;
+          constexpr uint32_t kOp = kTcRows * 128;
+          const int k = (int)(step[g] & 7);
+          const int f = k < 4 ? k : 6 - k;  // the layer whose z is formed (-1: none)
+          if (k >= 4) {
+            const int l = 7 - k;
+            const uint32_t aPrev = l > 0 ? aH + (l - 1) * kOp : aX, aWl = aW + (uint32_t)l * kHid * 128;
+            const bool acc = started >> l & 1u;
+            started |= 1u << l;
             for (int ks = 0; ks < kTcRows / 16; ks++)
-              umma_bf16(tb + 256 + 64u * l, umma_desc_mn(aDZ + 2048 * ks), umma_desc_mn(aPrev + 2048 * ks), idDW,
-                        acc || ks > 0);
+              umma_bf16(tb + 256 + 64u * l, umma_desc_mn(aDZ + 2048 * ks), umma_desc_mn(aPrev + 2048 * ks), idDW, acc || ks > 0);
             if (l > 0) {
               const int kst = l == 3 ? kOutP / 16 : kHid / 16;  // K = the layer's output units
               for (int ks = 0; ks < kst; ks++)
-                umma_bf16(tb + 192, umma_desc(aDZ + 256 * ks), umma_desc_mn(aWl + 2048 * ks), idDH, ks > 0);
+                umma_bf16(z + 64, umma_desc(aDZ + 256 * ks), umma_desc_mn(aWl + 2048 * ks), idDH, ks > 0);
             }
-          })) {
-        failed = true;
-        break;
+          }
+          if (f >= 0) {
+            const uint32_t aIn = f > 0 ? aH + (f - 1) * kOp : aX, aWf = aW + (uint32_t)f * kHid * 128;
+            for (int ks = 0; ks < 4; ks++)
+              umma_bf16(z, umma_desc(aIn + 256 * ks), umma_desc(aWf + 256 * ks), f < 3 ? idFwd64 : idFwd32, ks > 0);
+          }
+          umma_commit(smem_u32(&S.done[g]));
+          step[g]++;
+          idle = 0;
+        }
+        if (++idle == kWaitLimit) {
+          failed = true;
+          break;
+        }
       }
-      if (l > 0) {
-        float dh[16], z[16];
-        tmem_ld16(tb + lane0 + 192 + col0, dh);
-        tmem_ld16(tb + lane0 + 64u * (l - 1) + col0, z);
-        tmem_wait_ld();
-        for (int k = 0; k < 16; k++)
-          dh[k] = r < n ? dh[k] * silu_grad(z[k] + tc_bias_s(m.P, l - 1, col0 + k)) : 0.f;
-        tc_store16(S.DZ, row, col0, dh);
-        tr_bias_sum16(dh, S.gb + (l - 1) * kHid + col0);
-      }
+      for (int g = 0; g < kTrGroups; g++)  // nothing in flight when the block leaves
+        if (step[g] > 0) mbar_wait(smem_u32(&S.done[g]), (uint32_t)(step[g] - 1) & 1u, kWaitLimit);
     }
-    first = false;
+    __syncwarp();
+  } else {
+    const int grp = tid / kTrGroup, gt = tid % kTrGroup, q = warp & 3, half = (gt >> 5) >> 2, row = 32 * q + lane, c0 = 32 * half;
+    TrTcSmem::Tile& T = S.t[grp];
+    const uint32_t ready = smem_u32(&S.ready[grp]), done = smem_u32(&S.done[grp]);
+    const uint32_t tz = tb + 128u * grp + ((uint32_t)(q * 32) << 16) + c0;
+    uint32_t phase = 0;
+    float bsum[4][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};  // bias gradients of this lane's columns
+    // operands written: hand over to the tensor cores and wait for the product
+    auto product = [&]() {
+      proxy_fence_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ready) : "memory");
+    };
+    auto wait = [&]() {
+      if (!failed) failed = !mbar_wait(done, phase, kWaitLimit);
+      phase ^= 1u;
+      failed = __any_sync(0xffffffffu, failed);
+      tc_fence_after();
+    };
+    // 32 B of X per step: chunk e = gt + 256 j of the tile (row e / 8, columns 8 (e % 8) .. + 7), loaded a tile ahead
+    float4 nx[8];
+    auto fetch = [&](int64_t r0) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int e = gt + j * kTrGroup, rw = e >> 3, kc = e & 7;
+        nx[2 * j] = nx[2 * j + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r0 + rw < n) {
+          const float4* p = reinterpret_cast<const float4*>(X + (r0 + rw) * kIn + 8 * kc);
+          nx[2 * j] = p[0];
+          nx[2 * j + 1] = p[1];
+        }
+      }
+    };
+    int64_t tile = blockIdx.x + (int64_t)grp * gridDim.x;
+    if (tile < tiles) fetch(tile * kTcRows);
+    for (; tile < tiles && !failed; tile += slots) {
+      const int64_t r = tile * kTcRows + row;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int e = gt + j * kTrGroup;
+        *reinterpret_cast<uint4*>(T.X + cm_off(e >> 3, 8 * (e & 7))) = pack8(&nx[2 * j].x);
+      }
+      product();
+      float v[32];
+      // ---- forward: h_l = SiLU(z_l + b_l) into H[l]
+#pragma unroll
+      for (int l = 0; l < 3; l++) {
+        wait();
+        tmem_ld16(tz, v);
+        tmem_ld16(tz + 16, v + 16);
+        tmem_wait_ld();
+        for (int k = 0; k < 32; k += 4) {
+          const float4 b = *reinterpret_cast<const float4*>(&S.b[l * kHid + c0 + k]);
+          v[k] = silu(v[k] + b.x);
+          v[k + 1] = silu(v[k + 1] + b.y);
+          v[k + 2] = silu(v[k + 2] + b.z);
+          v[k + 3] = silu(v[k + 3] + b.w);
+        }
+        tc_store32(T.H[l], row, c0, v);
+        product();
+      }
+      // ---- y = z4 + b4, dz4 = 2 (y - t) / count on the 20 outputs (columns below 32)
+      float tg[kOut];
+      if (half == 0)
+        for (int k = 0; k < kOut; k += 4) {
+          float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (r < n) {
+            const float* p = Tg + r * kOut + k;
+            if ((reinterpret_cast<uintptr_t>(Tg) & 15u) == 0) t4 = *reinterpret_cast<const float4*>(p);
+            else t4 = make_float4(p[0], p[1], p[2], p[3]);
+          }
+          tg[k] = t4.x; tg[k + 1] = t4.y; tg[k + 2] = t4.z; tg[k + 3] = t4.w;
+        }
+      wait();
+      if (half == 0) {
+        tmem_ld16(tz, v);
+        tmem_ld16(tz + 16, v + 16);
+        tmem_wait_ld();
+        for (int k = 0; k < 32; k++) {
+          if (k < kOut && r < n) {
+            const float dd = v[k] + S.b[3 * kHid + k] - tg[k < kOut ? k : 0];
+            lossLocal += (double)dd * dd;
+            v[k] = 2.f * dd * invCount;
+          } else {
+            v[k] = 0.f;
+          }
+        }
+      } else {
+        for (int k = 0; k < 32; k++) v[k] = 0.f;  // units 32 .. 63 stay zero
+      }
+      tc_store32(T.DZ, row, c0, v);
+      product();
+      if (half == 0) {
+        bsum[3][0] += tr_sum16(v, lane);
+        bsum[3][1] += tr_sum16(v + 16, lane);
+      }
+      // ---- backward: dz_{l-1} = dH SiLU'(z_{l-1} + b_{l-1})
+#pragma unroll
+      for (int l = 3; l > 0; l--) {
+        if (l == 1) fetch((tile + slots) * kTcRows);
+        wait();
+#pragma unroll
+        for (int h = 0; h < 32; h += 16) {
+          float z[16];
+          tmem_ld16(tz + 64 + h, v + h);
+          tmem_ld16(tz + h, z);
+          tmem_wait_ld();
+#pragma unroll
+          for (int k = 0; k < 16; k += 4) {
+            const float4 b = *reinterpret_cast<const float4*>(&S.b[(l - 1) * kHid + c0 + h + k]);
+            v[h + k] = r < n ? v[h + k] * silu_grad(z[k] + b.x) : 0.f;
+            v[h + k + 1] = r < n ? v[h + k + 1] * silu_grad(z[k + 1] + b.y) : 0.f;
+            v[h + k + 2] = r < n ? v[h + k + 2] * silu_grad(z[k + 2] + b.z) : 0.f;
+            v[h + k + 3] = r < n ? v[h + k + 3] * silu_grad(z[k + 3] + b.w) : 0.f;
+          }
+        }
+        tc_store32(T.DZ, row, c0, v);
+        product();
+        bsum[l - 1][0] += tr_sum16(v, lane);
+        bsum[l - 1][1] += tr_sum16(v + 16, lane);
+      }
+      wait();  // dW_1: the tile's operands are free
+    }
+    if ((lane & 1) == 0)
+#pragma unroll
+      for (int l = 0; l < 4; l++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          if (l < 3 || half == 0) atomicAdd(&S.gb[l * kHid + c0 + 16 * h + tr_sum_col(lane)], bsum[l][h]);
   }
-  if (failed && tid == 0) {
-    atomicOr(flags, kFlagTimeout);
-    mbar_wait(bar, phase ^ 1u, kWaitLimit);
-  }
+  if (failed) atomicOr(flags, kFlagTimeout);
   tc_fence_before();
-  __syncthreads();
+  const bool bad = __syncthreads_or(failed);
   tc_fence_after();
-  // the CTA's weight gradients and bias gradients into G: dW_l unit u = 16 q + t in lane t < 16 of the
-  // warps of lane quarter q, columns 16 g .. 16 g + 15
-  if (!failed && !first) {
-    const int u = 16 * q + lane;
+  // the CTA's weight gradients and bias gradients: dW_l unit u = 16 q + t in lane t < 16 of the warps of lane
+  // quarter q, columns 16 g .. 16 g + 15
+  float* row = part + (int64_t)blockIdx.x * kTrPart;
+  __shared__ double lossW[kTrThreads / 32];
+  lossLocal = warp_sum_d(lossLocal);
+  if (lane == 0) lossW[warp] = lossLocal;
+  __syncthreads();
+  if (tid == 0) {
+    double t = 0;
+    for (int w = 0; w < kTrThreads / 32; w++) t += lossW[w];
+    row[kNParam] = (float)t;
+    row[kNParam + 1] = (float)(t - (double)(float)t);
+  }
+  if (bad)  // after a timeout: a defined row
+    for (int e = tid; e < kNParam; e += kTrThreads) row[e] = 0.f;
+  if (!bad && warp < 16) {
+    const int q = warp & 3, col0 = 16 * (warp >> 2), u = 16 * q + lane;
     const bool mine = lane < 16;
     for (int l = 0; l < 4; l++) {
       const int N = l < 3 ? kHid : kOutP;
       const int woff = l == 0 ? kOffW1 : l == 1 ? kOffW2 : l == 2 ? kOffW3 : kOffW4;
       float gv[16];
-      tmem_ld16(tb + lane0 + 256 + 64u * l + col0, gv);
+      tmem_ld16(tb + ((uint32_t)(q * 32) << 16) + 256 + 64u * l + col0, gv);
       tmem_wait_ld();
       if (mine && u < N)
-        for (int k = 0; k < 16; k++)
-          if (gv[k] != 0.f) atomicAdd(&G[woff + u * 64 + col0 + k], gv[k]);
+        for (int k = 0; k < 16; k += 4)
+          *reinterpret_cast<float4*>(&row[woff + u * 64 + col0 + k]) = make_float4(gv[k], gv[k + 1], gv[k + 2], gv[k + 3]);
     }
-    for (int e = tid; e < 3 * kHid + kOutP; e += blockDim.x) {
+    for (int e = tid; e < 3 * kHid + kOutP; e += kTrGroups * kTrGroup) {
       const int off = e < kHid ? kOffB1 + e : e < 2 * kHid ? kOffB2 + e - kHid : e < 3 * kHid ? kOffB3 + e - 2 * kHid
                                                                                             : kOffB4 + e - 3 * kHid;
-      if (S.gb[e] != 0.f) atomicAdd(&G[off], S.gb[e]);
+      row[off] = S.gb[e];
     }
   }
-  lossLocal = warp_sum_d(lossLocal);
-  if ((tid & 31) == 0 && lossLocal != 0.0) atomicAdd(lossAcc, lossLocal);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
+  if (warp == kTrGroups * kTrGroup / 32) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(kTrCols) : "memory");
   }
 }
 
-// Adam (Kingma & Ba) on the FP32 master parameters; padded entries stay zero; refreshes the BF16 copy
-__global__ void k_mlp_adam(float* P, float* Mo, float* V, const float* G, bf16* W, float lr, float b1, float b2,
-                           float eps, float c1, float c2) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= kNParam) return;
+// sum over the rows of `part` of entry e: 4 threads per entry (a block of 256: 64 entries), each over a
+// quarter of the rows, added in order; valid in the entry's first thread
+constexpr int kRedEntries = 64;
+__device__ __forceinline__ float tr_sum_rows(const float* part, int rows, int e, float (*sh)[kRedEntries]) {
+  const int k = threadIdx.x / kRedEntries, x = threadIdx.x % kRedEntries;
+  float a = 0.f;
+  if (e < kNParam)
+    for (int b = k * rows / 4; b < (k + 1) * rows / 4; b++) a += part[(int64_t)b * kTrPart + e];
+  sh[k][x] = a;
+  __syncthreads();
+  return (sh[0][x] + sh[1][x]) + (sh[2][x] + sh[3][x]);
+}
+// the loss, by one warp
+__device__ __forceinline__ void tr_sum_loss(const float* part, int rows, double* loss) {
+  double t = 0;
+  for (int b = threadIdx.x & 31; b < rows; b += 32) {
+    const float2 v = *reinterpret_cast<const float2*>(&part[(int64_t)b * kTrPart + kNParam]);
+    t += (double)v.x + (double)v.y;
+  }
+  t = warp_sum_d(t);
+  if ((threadIdx.x & 31) == 0) *loss = t;
+}
+__global__ void __launch_bounds__(256) k_mlp_reduce(const float* part, int rows, float* G, double* loss) {
+  __shared__ float sh[4][kRedEntries];
+  const int e = blockIdx.x * kRedEntries + threadIdx.x % kRedEntries;
+  const float g = tr_sum_rows(part, rows, e, sh);
+  if (threadIdx.x < kRedEntries && e < kNParam) G[e] = g;
+  if (blockIdx.x == 0 && threadIdx.x / 32 == 7) tr_sum_loss(part, rows, loss);
+}
+// Adam (Kingma & Ba) on the FP32 master parameters, from the rows of gradients; padded entries stay zero;
+// refreshes the BF16 copy
+__global__ void __launch_bounds__(256) k_mlp_adam(float* P, float* Mo, float* V, const float* part, int rows, double* loss, bf16* W,
+                                                  float lr, float b1, float b2, float eps, float c1, float c2) {
+  __shared__ float sh[4][kRedEntries];
+  const int e = blockIdx.x * kRedEntries + threadIdx.x % kRedEntries;
+  const float g = tr_sum_rows(part, rows, e, sh);
+  if (blockIdx.x == 0 && threadIdx.x / 32 == 7) tr_sum_loss(part, rows, loss);
+  if (threadIdx.x >= kRedEntries || e >= kNParam) return;
   bool pad = false;
   int wi = -1;
   if (e < kOffB1) { pad = (e % kInP) >= kIn; wi = kWOff1 + e; }
@@ -689,7 +832,6 @@ __global__ void k_mlp_adam(float* P, float* Mo, float* V, const float* G, bf16* 
   else if (e >= kOffW4 && e < kOffB4) { pad = (e - kOffW4) / kHid >= kOut; wi = kWOff4 + (e - kOffW4); }
   else if (e >= kOffB4) pad = (e - kOffB4) >= kOut;
   if (pad) { P[e] = 0.f; if (wi >= 0) W[wi] = __float2bfloat16(0.f); return; }
-  const float g = G[e];
   const float m = b1 * Mo[e] + (1.f - b1) * g, v = b2 * V[e] + (1.f - b2) * g * g;
   Mo[e] = m;
   V[e] = v;
