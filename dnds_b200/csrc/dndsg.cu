@@ -27,6 +27,13 @@ using namespace dg;
 namespace {
 constexpr int kBlock = 256;
 inline unsigned grid_for(int64_t n) { return (unsigned)((n + kBlock - 1) / kBlock); }
+// The block of the passes that wait on gathered rows (face flux, limiter face pass, cell update, the cell
+// pass and the colour batches of an implicit iteration).  Their residency is set by registers, and a small
+// block gives its share back as soon as its own rows have come, not when the slowest of 256 has: on
+// 2,097,152 triangles 256 -> 128 -> 64 threads in the face flux alone takes the FP64 step from 2335 to 2297 to
+// 2284 us, the FP32 one from 1465 to 1455 to 1453 us; the other passes a further 14 us each
+constexpr int kHotBlock = 64;
+inline unsigned hot_grid(int64_t n) { return (unsigned)((n + kHotBlock - 1) / kHotBlock); }
 
 constexpr int64_t kSmallCells = 262144, kSplitMaxFaces = 16384;  // dndsg_ctx::small, splitFlux
 // device scalar slots
@@ -358,10 +365,10 @@ __global__ void k_setup_lim_compact(MeshView m, const CellSetup* cells, const do
   const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   setup_limiter_compact<T>(f, m, cells, faceW, g, cellFr);
 }
-// FP64: 2 blocks per SM.  FP32: 4 blocks per SM (64 registers; the pass waits on its gathers, and the
-// fourth block took the 8,388,608-triangle Riemann step from 8.61 to 8.44 ms against three)
+// FP64: 8 blocks of 64 per SM.  FP32: 16 (64 registers; the pass waits on its gathers, and the last four
+// took the 8,388,608-triangle Riemann step from 8.61 to 8.44 ms against twelve)
 template <class T>
-__global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 4 : 2) k_lim_face(LimView v, const T* urec, int32_t* count) {
+__global__ void __launch_bounds__(kHotBlock, sizeof(T) == 4 ? 16 : 8) k_lim_face(LimView v, const T* urec, int32_t* count) {
   int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (f == 0) *count = 0;  // the list of cells to limit, filled by the next launch
   if (f < v.F) limiter_face_indicator<T>(f, v, urec);
@@ -423,17 +430,20 @@ __device__ __forceinline__ void reset_dtmin(double* scal) {
 }
 
 // faces [f0, f1): interior faces first (BND = false), then boundary faces.  The FP32 Roe interior
-// kernel runs 4 blocks per SM (64 registers, a few spilled words): the gathers want the occupancy
-// more than the registers (measured: 2 blocks 0.296 ms, 3: 0.283, 4: 0.243, 5: 0.318 per RHS on
-// 2,097,152 triangles).  The FP32 HLLC interior kernel (flux-difference form) runs 3 (measured per
-// SSP-RK3 step of the 8,388,608-triangle Riemann problem: 3 blocks 7.79-7.81 ms, 4 blocks with 64
-// registers and 172 B spilled 8.02-8.04 ms)
+// kernel runs 16 blocks of 64 per SM (64 registers, a few spilled words): the gathers want the occupancy
+// more than the registers (measured with blocks of 256: 2 blocks 0.296 ms, 3: 0.283, 4: 0.243, 5: 0.318
+// per RHS on 2,097,152 triangles).  The FP32 HLLC interior kernel (flux-difference form) runs 12 (per
+// SSP-RK3 step of the 8,388,608-triangle Riemann problem, blocks of 256: 3 blocks 7.79-7.81 ms, 4 blocks
+// with 64 registers and 172 B spilled 8.02-8.04 ms).  The FP64 kernels run 8 (128 registers; 10 blocks, 100
+// registers: 2346 us for 2224 us per step).
+// W: the state rows start on 32-byte boundaries and take one load each (side_increments' twelve instead of
+// twenty-four per FP64 face; 2.2% of the FP64 step, 0.4% of the FP32 one, whose coefficient rows have 16 bytes)
 // DT = true (the first stage of an SSP-RK3 step): each thread first writes its face's EvaluateDt terms
 // (dt_face: lambda A and the entropy-fix dLambda, from the same means this stage reads), which the
 // flux then reads back, so the step needs no separate face pass for dt; the dt minimum is reset for the
 // cell pass that follows
-template <class T, int RIEMANN, bool BND, bool DT = false>
-__global__ void __launch_bounds__(kBlock, (sizeof(T) == 4 && RIEMANN == 1 && !BND) ? 4 : ((sizeof(T) == 4 && !BND) ? 3 : 2)) k_face_flux(HotView<T> h, int64_t f0, int64_t f1, double* scal,
+template <class T, int RIEMANN, bool BND, bool DT = false, bool W = true>
+__global__ void __launch_bounds__(kHotBlock, (sizeof(T) == 4 && RIEMANN == 1 && !BND) ? 16 : ((sizeof(T) == 4 && !BND) ? 12 : 8)) k_face_flux(HotView<T> h, int64_t f0, int64_t f1, double* scal,
                                                          int useDev, double tHost, double c, unsigned* flags,
                                                          unsigned long long* nred) {
   pdl_enter();
@@ -448,14 +458,12 @@ __global__ void __launch_bounds__(kBlock, (sizeof(T) == 4 && RIEMANN == 1 && !BN
     double out[4];
     double t = stage_time(scal, useDev, tHost, c);
     if constexpr (sizeof(T) == 4 && RIEMANN == 1 && !BND)
-      r = face_flux_roe_delta32(f, h, out, bad);
+      r = face_flux_roe_delta32<W>(f, h, out, bad);
     else if constexpr (sizeof(T) == 4 && RIEMANN == 2 && !BND)
-      r = face_flux_hllc_delta32(f, h, out, bad);
+      r = face_flux_hllc_delta32<W>(f, h, out, bad);
     else
-      r = face_flux<T, RIEMANN, BND>(f, h, t, out, bad);
-    double* o = &h.flux[f * 4];
-    *reinterpret_cast<double2*>(o) = make_double2(out[0], out[1]);
-    *reinterpret_cast<double2*>(o + 2) = make_double2(out[2], out[3]);
+      r = face_flux<T, RIEMANN, BND, W>(f, h, t, out, bad);
+    store4_wide(&h.flux[f * 4], out);
   }
   unsigned anyBad = __ballot_sync(0xffffffffu, bad);
   int rs = __reduce_add_sync(0xffffffffu, r);
@@ -610,7 +618,7 @@ __global__ void k_fill_dt(double* dt, int64_t n, const double* scal) {
 // quads 394 -> 361 us) and no pass that copies the means.  One thread writes each scalar; no other thread of
 // the launch reads that one
 template <class T, int STAGE, bool STEP = false>
-__global__ void __launch_bounds__(kBlock) k_cell_update(HotView<T> h, double* scal, double tEnd) {
+__global__ void __launch_bounds__(kHotBlock) k_cell_update(HotView<T> h, double* scal, double tEnd) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= h.N) return;
@@ -628,24 +636,20 @@ __global__ void __launch_bounds__(kBlock) k_cell_update(HotView<T> h, double* sc
   double x[4];
   load4<T>(&h.u[i * 4], x);
   if (STEP && STAGE == 0) {
-    double2* o = reinterpret_cast<double2*>(&h.uLast[i * 4]);
-    o[0] = make_double2(x[0], x[1]);
-    o[1] = make_double2(x[2], x[3]);
+    store4_wide(&h.uLast[i * 4], x);
   }
   for (int v = 0; v < 4; v++) x[v] += r[v] * dt;
   if (STAGE > 0) {
     const double cf = STAGE == 1 ? 0.25 : 2.0 / 3.0;
     double xl[4];
-    load4<T>(&h.uLast[i * 4], xl);
+    load4_wide(&h.uLast[i * 4], xl);
     for (int v = 0; v < 4; v++) {
       double a = x[v] * (cf / (1 - cf));
       a += xl[v];
       x[v] = a * (1 - cf);
     }
   }
-  double2* o = reinterpret_cast<double2*>(&h.u[i * 4]);
-  o[0] = make_double2(x[0], x[1]);
-  o[1] = make_double2(x[2], x[3]);
+  store4_wide(&h.u[i * 4], x);
 }
 
 // per-block partial sums / maxima of |rhs|^p (EvaluateResidual)
@@ -757,7 +761,7 @@ LimView lim_view(dndsg_ctx* c, int ifAll) {
 template <class T>
 void run_limiter_v3(dndsg_ctx* c, int ifAll, cudaStream_t s) {
   LimView v = lim_view(c, ifAll);
-  k_lim_face<T><<<grid_for(c->F), kBlock, 0, s>>>(v, (const T*)c->urec, c->limCount);
+  k_lim_face<T><<<hot_grid(c->F), kHotBlock, 0, s>>>(v, (const T*)c->urec, c->limCount);
   k_lim_cell_indicator<T><<<grid_for(c->N), kBlock, 0, s>>>(v, c->limList, c->limCount);
   // urecNew (the previous sweep's coefficients, free until the next sweep) holds the limited ones
   if (!c->sms && cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) c->sms = 148;
@@ -773,7 +777,7 @@ void run_limiter_v3(dndsg_ctx* c, int ifAll, cudaStream_t s) {
 template <class T>
 void run_limiter_v2(dndsg_ctx* c, int ifAll, cudaStream_t s) {
   LimView v = lim_view(c, ifAll);
-  k_lim_face<T><<<grid_for(c->F), kBlock, 0, s>>>(v, (const T*)c->urec, c->limCount);
+  k_lim_face<T><<<hot_grid(c->F), kHotBlock, 0, s>>>(v, (const T*)c->urec, c->limCount);
   k_lim_cell_indicator<T><<<grid_for(c->N), kBlock, 0, s>>>(v, c->limList, c->limCount);
   if (!c->sms && cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) c->sms = 148;
   const unsigned g = (unsigned)std::min<int64_t>(grid_for(c->N), 4 * c->sms);
@@ -793,7 +797,7 @@ void run_limiter(dndsg_ctx* c, int ifAll, cudaStream_t s) {
 }
 
 // the inviscid face-flux launches (interior faces, then boundary faces); DT: with the faces' dt terms
-template <class T, bool DT>
+template <class T, bool DT, bool W = true>
 void launch_flux_inviscid(dndsg_ctx* c, const HotView<T>& h, int useDev, double tHost, double cst, cudaStream_t s) {
   const int64_t Fi = c->Fi, F = c->F;
   const bool hllc = c->s.riemann == 2;
@@ -804,10 +808,10 @@ void launch_flux_inviscid(dndsg_ctx* c, const HotView<T>& h, int useDev, double 
     return;
   }
   if (Fi > 0)
-    launch(hllc ? k_face_flux<T, 2, false, DT> : k_face_flux<T, 1, false, DT>, grid_for(Fi), kBlock, 0, s, c->small(), h, (int64_t)0, Fi,
+    launch(hllc ? k_face_flux<T, 2, false, DT, W> : k_face_flux<T, 1, false, DT, W>, hot_grid(Fi), kHotBlock, 0, s, c->small(), h, (int64_t)0, Fi,
            c->scal, useDev, tHost, cst, c->flags, c->nreduced);
   if (F > Fi)
-    launch(hllc ? k_face_flux<T, 2, true, DT> : k_face_flux<T, 1, true, DT>, (unsigned)((F - Fi + 63) / 64), 64, 0, s, c->small(), h, Fi, F,
+    launch(hllc ? k_face_flux<T, 2, true, DT, W> : k_face_flux<T, 1, true, DT, W>, hot_grid(F - Fi), kHotBlock, 0, s, c->small(), h, Fi, F,
            c->scal, useDev, tHost, cst, c->flags, c->nreduced);
 }
 
@@ -869,9 +873,9 @@ int run_step(dndsg_ctx* c, double cfl, double tEnd, cudaStream_t s) {
     HotView<T> h = view<T>(c);
     launch_flux<T>(c, 1, 0.0, cst[stg], s, stg == 0 && fuseDt);
     if (stg == 0 && fuseDt) launch(k_dt_cell<T, false>, grid_for(c->N), kBlock, 0, s, c->small(), h, cfl, 1e100, c->scal);
-    if (stg == 0) launch(k_cell_update<T, 0, true>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, tEnd);
-    else if (stg == 1) launch(k_cell_update<T, 1, true>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, tEnd);
-    else launch(k_cell_update<T, 2, true>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, tEnd);
+    if (stg == 0) launch(k_cell_update<T, 0, true>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, tEnd);
+    else if (stg == 1) launch(k_cell_update<T, 1, true>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, tEnd);
+    else launch(k_cell_update<T, 2, true>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, tEnd);
   }
   return 0;
 }
@@ -882,9 +886,9 @@ void run_rk_stage(dndsg_ctx* c, int stg, cudaStream_t s) {
   const double cst[3] = {0.0, 1.0, 0.5};
   launch_flux<T>(c, 1, 0.0, cst[stg], s);
   HotView<T> h = view<T>(c);
-  if (stg == 0) launch(k_cell_update<T, 0>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
-  else if (stg == 1) launch(k_cell_update<T, 1>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
-  else launch(k_cell_update<T, 2>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
+  if (stg == 0) launch(k_cell_update<T, 0>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, 0.0);
+  else if (stg == 1) launch(k_cell_update<T, 1>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, 0.0);
+  else launch(k_cell_update<T, 2>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, 0.0);
 }
 
 // halo exchange buffers: PACK buf[k][0..w) = a[cells[k]][0..w), else the reverse
@@ -902,7 +906,7 @@ template <class T>
 int run_rhs(dndsg_ctx* c, double t, cudaStream_t s) {
   launch_flux<T>(c, 0, t, 0.0, s);
   HotView<T> h = view<T>(c);
-  launch(k_cell_update<T, -1>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
+  launch(k_cell_update<T, -1>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, 0.0);
   return 0;
 }
 
@@ -1812,8 +1816,11 @@ void run_rhs_noalloc(dndsg_ctx* c, const double* u, const void* urec, double* rh
   h.urec = (const T*)urec;
   h.rhs = rhs;
   h.flux = scratch;
-  launch_flux_h<T>(c, h, 0, t, 0.0, s);
-  launch(k_cell_update<T, -1>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
+  // the caller's rows may start between two 32-byte boundaries
+  const bool wide = (((uintptr_t)u | (uintptr_t)urec) & 31u) == 0;
+  if (wide) launch_flux_inviscid<T, false>(c, h, 0, t, 0.0, s);
+  else launch_flux_inviscid<T, false, false>(c, h, 0, t, 0.0, s);
+  launch(k_cell_update<T, -1>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, 0.0);
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
@@ -2094,9 +2101,9 @@ int run_step_tol(dndsg_ctx* c, const dndsg_mlp* m, double cfl, double tEnd, doub
     if (c->s.limiter) run_limiter<T>(c, 0, s);
     launch_flux<T>(c, 1, 0.0, cst[stg], s);
     HotView<T> h = view<T>(c);
-    if (stg == 0) launch(k_cell_update<T, 0>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
-    else if (stg == 1) launch(k_cell_update<T, 1>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
-    else launch(k_cell_update<T, 2>, grid_for(c->N), kBlock, 0, s, c->small(), h, c->scal, 0.0);
+    if (stg == 0) launch(k_cell_update<T, 0>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, 0.0);
+    else if (stg == 1) launch(k_cell_update<T, 1>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, 0.0);
+    else launch(k_cell_update<T, 2>, hot_grid(c->N), kHotBlock, 0, s, c->small(), h, c->scal, 0.0);
   }
   k_advance_time<<<1, 1, 0, s>>>(c->scal);
   if (sweepsOut) *sweepsOut = total;
@@ -2394,9 +2401,9 @@ __device__ __forceinline__ double impl_combine(const ImplComb& c, int64_t e, dou
 // The cell pass of an implicit iteration after its face fluxes: EvaluateRHS's gather, the local dt of
 // EvaluateDt, the LU-SGS diagonal (LUSGSMatrixInit) and the BDF or SDIRK right-hand side, in one pass over
 // the faces' fluxes and lambda A (five launches of their own before: on 524,288 triangles 67 us of kernels
-// and a copy, now 27 us).  The residual accumulators of the iteration start from zero here.
+// and a copy; 27 us in one pass, before its gathers were loaded together).  The residual accumulators of the iteration start from zero here.
 template <class T>
-__global__ void __launch_bounds__(kBlock) k_implicit_cell(HotView<T> h, ImplComb cb, double cfl, double dtPhysInv,
+__global__ void __launch_bounds__(kHotBlock) k_implicit_cell(HotView<T> h, const __grid_constant__ ImplComb cb, double cfl, double dtPhysInv,
                                                           double alpha, double* Dinv, double* D, double* resAcc) {
   pdl_enter();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -2421,6 +2428,8 @@ __global__ void __launch_bounds__(kBlock) k_implicit_cell(HotView<T> h, ImplComb
 // sweep in that scan order, level by level.  No two cells of a batch are neighbours and every
 // neighbour a cell reads was finished in an earlier batch, so the result does not depend on the
 // order within a batch.  inc is updated in place, as the reference calls both sweeps.
+// Slots, neighbours and ranks are loaded for all faces before the first neighbour is worked on: a face at a
+// time each cell waits for three chains of four loads.
 template <class T, bool FWD>
 __device__ __forceinline__ void lusgs_cell(const HotView<T>& h, const int32_t* rankOf, int64_t i, double alpha,
                                            const double* Dinv, const double* rhs, double* inc) {
@@ -2429,19 +2438,25 @@ __device__ __forceinline__ void lusgs_cell(const HotView<T>& h, const int32_t* r
   if (FWD) load4<T>(&rhs[i * 4], buf);
   else buf[0] = buf[1] = buf[2] = buf[3] = 0.0;
   const double scale = -0.5 * alpha / h.vol[i];
-  for (int k = 0; k < h.nfmax; k++) {
-    const int32_t sf = h.cellFace[aos(i, k, h.nfmax)];
-    if (sf == kEmptySlot) continue;
-    const int32_t f = sf >= 0 ? sf : ~sf;
-    const int32_t j = sf >= 0 ? h.faceR[f] : h.faceL[f];
-    if (j < 0) continue;
-    const int cj = rankOf[j];
-    if (FWD ? !(cj < ci) : !(cj > ci)) continue;
-    const double sg = sf >= 0 ? 1.0 : -1.0;
+  int32_t sf[kMaxSlots], nb[kMaxSlots], rk[kMaxSlots];
+  cell_slots(i, h, sf);
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++) {
+    nb[k] = -1;
+    if (sf[k] != kEmptySlot) nb[k] = sf[k] >= 0 ? h.faceR[sf[k]] : h.faceL[~sf[k]];
+  }
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++) rk[k] = nb[k] >= 0 ? rankOf[nb[k]] : ci;  // equal ranks: not a neighbour to read
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++) {
+    if (FWD ? !(rk[k] < ci) : !(rk[k] > ci)) continue;
+    const int32_t f = sf[k] >= 0 ? sf[k] : ~sf[k];
+    const int64_t j = nb[k];
+    const double sg = sf[k] >= 0 ? 1.0 : -1.0;
     const double area = h.faceArea[f];
     double U[4], dU[4], dF[4];
-    load4<T>(&h.u[(int64_t)j * 4], U);
-    load4<T>(&inc[(int64_t)j * 4], dU);
+    load4_wide(&h.u[j * 4], U);
+    load4<T>(&inc[j * 4], dU);
     flux_jac_times_du(U, sg * h.faceNormal[2 * f], sg * h.faceNormal[2 * f + 1], dU, h.lamA[f] / area, h.gamma, dF);
     for (int v = 0; v < 4; v++) buf[v] += scale * area * dF[v];
   }
@@ -2455,7 +2470,7 @@ __device__ __forceinline__ void lusgs_cell(const HotView<T>& h, const int32_t* r
 }
 
 template <class T, bool FWD>
-__global__ void __launch_bounds__(kBlock) k_lusgs_batch(HotView<T> h, const int32_t* rankOf,
+__global__ void __launch_bounds__(kHotBlock) k_lusgs_batch(HotView<T> h, const int32_t* rankOf,
                                                         const int32_t* cells, int64_t n, double alpha,
                                                         const double* Dinv, const double* rhs, double* inc) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -2813,9 +2828,9 @@ void launch_lusgs_sweep(dndsg_ctx* c, bool forward, double alpha, const double* 
     const int64_t b = off[k], n = off[k + 1] - b;
     if (n == 0) continue;
     if (forward)
-      k_lusgs_batch<T, true><<<grid_for(n), kBlock, 0, s>>>(h, c->rankOf, cells + b, n, alpha, c->Dinv, rhs, inc);
+      k_lusgs_batch<T, true><<<hot_grid(n), kHotBlock, 0, s>>>(h, c->rankOf, cells + b, n, alpha, c->Dinv, rhs, inc);
     else
-      k_lusgs_batch<T, false><<<grid_for(n), kBlock, 0, s>>>(h, c->rankOf, cells + b, n, alpha, c->Dinv, rhs, inc);
+      k_lusgs_batch<T, false><<<hot_grid(n), kHotBlock, 0, s>>>(h, c->rankOf, cells + b, n, alpha, c->Dinv, rhs, inc);
   }
 }
 
@@ -2840,7 +2855,7 @@ void implicit_rhs(dndsg_ctx* c, double cfl, double t, int nRec, const ImplComb& 
   for (int k = 0; k < nRec; k++) run_vr<T>(c, false, s);
   if (c->s.limiter) run_limiter<T>(c, 0, s);
   launch_flux<T>(c, 0, t, 0.0, s, !viscous);
-  launch(k_implicit_cell<T>, grid_for(c->N), kBlock, 0, s, c->small(), view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
+  launch(k_implicit_cell<T>, hot_grid(c->N), kHotBlock, 0, s, c->small(), view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
 }
 
 // ImplicitBDFDualTimeStep::Step (DNDS_ODE.hpp:444-486), one pseudo-time iteration at order 1, with
@@ -3116,7 +3131,7 @@ inline unsigned sa_rhs_grid(int64_t n) { return (unsigned)((n + kSaRhsCells - 1)
 template <class T>
 void run_rhs_sa(dndsg_ctx* c, cudaStream_t s) {
   launch_flux_sa<T>(c, s);
-  launch(k_cell_update<T, -1>, grid_for(c->N), kBlock, 0, s, c->small(), view<T>(c), c->scal, 0.0);
+  launch(k_cell_update<T, -1>, hot_grid(c->N), kHotBlock, 0, s, c->small(), view<T>(c), c->scal, 0.0);
   k_sa_cell_rhs<T, false><<<sa_rhs_grid(c->N), kSaRhsCells * kSaGp, 0, s>>>(view<T>(c), sa_view<T>(c), ImplComb{}, 0.0, nullptr, nullptr);
 }
 
@@ -3127,7 +3142,7 @@ void implicit_rhs_sa(dndsg_ctx* c, double cfl, int nRec, const ImplComb& cb, con
   k_dt_face_sa<T><<<grid_for(c->F), kBlock, 0, s>>>(view<T>(c), sa_view<T>(c));
   for (int k = 0; k < nRec; k++) run_vr_sa<T>(c, s);
   launch_flux_sa<T>(c, s);
-  launch(k_implicit_cell<T>, grid_for(c->N), kBlock, 0, s, c->small(), view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
+  launch(k_implicit_cell<T>, hot_grid(c->N), kHotBlock, 0, s, c->small(), view<T>(c), cb, cfl, dtPhysInv, alpha, c->Dinv, c->Dmat, c->resAcc);
   k_sa_cell_rhs<T, true><<<sa_rhs_grid(c->N), kSaRhsCells * kSaGp, 0, s>>>(view<T>(c), sa_view<T>(c), cb5, alpha, c->Dmat, DS);
 }
 

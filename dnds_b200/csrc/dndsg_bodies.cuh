@@ -325,6 +325,22 @@ DG_HD void load4(const double* p, double* v) {
   for (int k = 0; k < 4; k++) v[k] = p[k];
 #endif
 }
+// a 32-byte row on a 32-byte boundary as one load: the library's own arrays only (a caller's may start on a
+// 16-byte one).  For rows that nothing in the thread has stored to before
+DG_HD void load4_wide(const double* p, double v[4]) {
+#if defined(__CUDA_ARCH__)
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+#else
+  for (int k = 0; k < 4; k++) v[k] = p[k];
+#endif
+}
+DG_HD void store4_wide(double* p, const double v[4]) {
+#if defined(__CUDA_ARCH__)
+  asm volatile("st.global.v4.f64 [%4], {%0, %1, %2, %3};" ::"d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]), "l"(p) : "memory");
+#else
+  for (int k = 0; k < 4; k++) p[k] = v[k];
+#endif
+}
 // one 4-variable row of a cell's coefficient block (16 B for float, 32 B for double)
 DG_HD void load_row(const float* p, float r[4]) {
 #if defined(__CUDA_ARCH__)
@@ -350,6 +366,17 @@ DG_HD void store_row(double* p, const double r[4]) {
   for (int k = 0; k < 4; k++) p[k] = r[k];
 #endif
 }
+// rows of the flow state: W = true where the arrays are the library's own, so that rows of doubles take one
+// load instead of two
+template <bool W>
+DG_HD void load_state(const double* p, double v[4]) {
+  if constexpr (W) load4_wide(p, v);
+  else load4<double>(p, v);
+}
+template <bool W>
+DG_HD void load_coef(const float* p, float r[4]) { load_row(p, r); }
+template <bool W>
+DG_HD void load_coef(const double* p, double r[4]) { load_state<W>(p, r); }
 template <class T>
 DG_HD void load_rec(const T* p, T r[5][4]) {
   for (int q = 0; q < 5; q++) load_row(p + 4 * q, r[q]);
@@ -461,12 +488,12 @@ DG_HD void vr_cell(int64_t i, const HotView<T>& h) {
 // reconstruction increments phi(gp) . urec of one cell at the 3 gauss points of a face, from the
 // side's compact basis: the dot products of the coefficient rows with v1, B and C (rows 2..4 only),
 // combined per point as phi . r = v1.r + C.r -+ B.r; gauss point 1 is the plain sum v1.r
-template <class T>
+template <bool W, class T>
 DG_HD void side_increments(const FaceBasisSide<T>& b, const T* rec, T inc[3][4]) {
   T a[4] = {T(0), T(0), T(0), T(0)}, o[4] = {T(0), T(0), T(0), T(0)}, e[4] = {T(0), T(0), T(0), T(0)};
   for (int q = 0; q < 5; q++) {
     T row[4];
-    load_row(rec + 4 * q, row);
+    load_coef<W>(rec + 4 * q, row);
     for (int v = 0; v < 4; v++) {
       a[v] += b.v1[q] * row[v];
       o[v] += b.B[q] * row[v];
@@ -481,10 +508,10 @@ DG_HD void side_increments(const FaceBasisSide<T>& b, const T* rec, T inc[3][4])
 
 // reconstruction increments phi(gp) . urec of both cells at the 3 gauss points of
 // face f; the coefficient rows are streamed once (EvaluateRHS, DNDS_FV_EulerEvaluator.cpp:250-360)
-template <class T>
+template <bool W = false, class T>
 DG_HD void face_increments(int64_t f, int32_t L, int32_t R, const HotView<T>& h, T incL[3][4], T incR[3][4]) {
-  side_increments(FaceBasisSide<T>(h.faceBasis, f, 0), &h.urec[(int64_t)L * 20], incL);
-  if (R >= 0) side_increments(FaceBasisSide<T>(h.faceBasis, f, 1), &h.urec[(int64_t)R * 20], incR);
+  side_increments<W>(FaceBasisSide<T>(h.faceBasis, f, 0), &h.urec[(int64_t)L * 20], incL);
+  if (R >= 0) side_increments<W>(FaceBasisSide<T>(h.faceBasis, f, 1), &h.urec[(int64_t)R * 20], incR);
   else for (int g = 0; g < 3; g++) for (int v = 0; v < 4; v++) incR[g][v] = T(0);
 }
 
@@ -548,16 +575,16 @@ DG_HD int face_states(int64_t f, const HotView<T>& h, double t, double UL[3][4],
 // face flux: sum over gauss points of -F(UL,UR).n |n| w (fluxFace, DNDS_FV_EulerEvaluator.hpp:371-591)
 // returns the reduced-order count; *bad is set on non-physical input
 // BND = false: an interior (or periodic) face, so no boundary-state code is compiled in
-template <class T, int RIEMANN, bool BND>
+template <class T, int RIEMANN, bool BND, bool W = false>
 DG_HD int face_flux(int64_t f, const HotView<T>& h, double t, double out[4], bool& bad) {
   int32_t L = h.faceL[f], R = h.faceR[f];
   double nx = h.faceNormal[2 * f], ny = h.faceNormal[2 * f + 1], area = h.faceArea[f];
   double uL[4], uR[4] = {0, 0, 0, 0};
-  load4<T>(&h.u[(int64_t)L * 4], uL);
-  if (!BND || R >= 0) load4<T>(&h.u[(int64_t)R * 4], uR);
+  load_state<W>(&h.u[(int64_t)L * 4], uL);
+  if (!BND || R >= 0) load_state<W>(&h.u[(int64_t)R * 4], uR);
   double dl = h.dLam[f];
   T incL[3][4], incR[3][4];
-  face_increments(f, L, R, h, incL, incR);
+  face_increments<W>(f, L, R, h, incL, incR);
   int nred = 0;
   double acc[4] = {0, 0, 0, 0};
   for (int g = 0; g < 3; g++) {
@@ -826,14 +853,15 @@ DG_HD int roe_point32(const FaceMeans32& m, const float incL[4], const float inc
   acc[3] += jw * (l.D[3] + r.D[3] - ((H - u * a) * w0 + 0.5f * vs * w1 + v * w2 + (H + u * a) * w3));
   return nred;
 }
+template <bool W = false>
 DG_HD int face_flux_roe_delta32(int64_t f, const HotView<float>& h, double out[4], bool& bad) {
   const int32_t L = h.faceL[f], R = h.faceR[f];
   const double nxd = h.faceNormal[2 * f], nyd = h.faceNormal[2 * f + 1], area = h.faceArea[f];
   double uL[4], uR[4];
-  load4<float>(&h.u[(int64_t)L * 4], uL);
-  load4<float>(&h.u[(int64_t)R * 4], uR);
+  load_state<W>(&h.u[(int64_t)L * 4], uL);
+  load_state<W>(&h.u[(int64_t)R * 4], uR);
   float incL[3][4], incR[3][4];
-  face_increments(f, L, R, h, incL, incR);
+  face_increments<W>(f, L, R, h, incL, incR);
   const float g1 = (float)(h.gamma - 1), dl = (float)h.dLam[f];
   const float nx = (float)nxd, ny = (float)nyd;
   FaceMeans32 m;
@@ -926,14 +954,15 @@ DG_HD int hllc_point32(const FaceMeans32& m, const float dFmean[4], const float 
   for (int k = 0; k < 4; k++) acc[k] += G[k] * jw;
   return nred;
 }
+template <bool W = false>
 DG_HD int face_flux_hllc_delta32(int64_t f, const HotView<float>& h, double out[4], bool& bad) {
   const int32_t L = h.faceL[f], R = h.faceR[f];
   const double nxd = h.faceNormal[2 * f], nyd = h.faceNormal[2 * f + 1], area = h.faceArea[f];
   double uL[4], uR[4];
-  load4<float>(&h.u[(int64_t)L * 4], uL);
-  load4<float>(&h.u[(int64_t)R * 4], uR);
+  load_state<W>(&h.u[(int64_t)L * 4], uL);
+  load_state<W>(&h.u[(int64_t)R * 4], uR);
   float incL[3][4], incR[3][4];
-  face_increments(f, L, R, h, incL, incR);
+  face_increments<W>(f, L, R, h, incL, incR);
   const float gamma = (float)h.gamma, gm1 = (float)(h.gamma - 1);
   const float nx = (float)nxd, ny = (float)nyd;
   FaceMeans32 m;
@@ -994,10 +1023,10 @@ DG_HD void dt_face(int64_t f, const HotView<T>& h) {
   int32_t L = h.faceL[f], R = h.faceR[f];
   double nx = h.faceNormal[2 * f], ny = h.faceNormal[2 * f + 1], area = h.faceArea[f];
   double UL[4];
-  load4<T>(&h.u[(int64_t)L * 4], UL);
+  load4_wide(&h.u[(int64_t)L * 4], UL);
   const double g1 = h.gamma - 1;
   double UR[4] = {UL[0], UL[1], UL[2], UL[3]};
-  if (R >= 0) load4<T>(&h.u[(int64_t)R * 4], UR);
+  if (R >= 0) load4_wide(&h.u[(int64_t)R * 4], UR);
   const double iLR = 1.0 / (UL[0] * UR[0]), irL = iLR * UR[0], irR = iLR * UL[0];  // one quotient for both densities
   const double uL = UL[1] * irL, vL = UL[2] * irL;
   const double pL = g1 * (UL[3] - UL[0] * 0.5 * (uL * uL + vL * vL)), aL2 = h.gamma * pL * irL;
@@ -1029,6 +1058,17 @@ DG_HD double dt_cell(int64_t i, const HotView<T>& h, double cfl, double maxDt) {
   return dmin(cfl * h.vol[i] / (lam + 1e-100), maxDt);
 }
 
+// the face slots of cell i, all loaded at once, the ones past nfmax empty.  The cell passes load every slot,
+// then every face's row, then add in slot order: a slot at a time is a chain of two loads per face that
+// nothing overlaps, with a row of flux in four loads.  Ten steps on 1,600 quads 335 -> 315 us, the FP32 step
+// on 2,097,152 triangles 1482 -> 1457 us
+constexpr int kMaxSlots = 4;
+template <class View>
+DG_HD void cell_slots(int64_t i, const View& h, int32_t sf[kMaxSlots]) {
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++) sf[k] = k < h.nfmax ? h.cellFace[aos(i, k, h.nfmax)] : kEmptySlot;
+}
+
 // rhs of cell i: gather of face fluxes plus the flux-balance term
 // (DNDS_FV_EulerEvaluator.cpp:501-508): -F(u_i) . sum_f n_f A_f / V_i
 // lam (LAM): the sum of the faces' lambda_f A_f as well
@@ -1036,14 +1076,22 @@ template <class T, bool LAM = false>
 DG_HD void cell_rhs(int64_t i, const HotView<T>& h, double r[4], double* lam = nullptr) {
   double s[4] = {0, 0, 0, 0};
   if (LAM) *lam = 0.0;
-  for (int k = 0; k < h.nfmax; k++) {
-    int32_t sf = h.cellFace[aos(i, k, h.nfmax)];
-    if (sf == kEmptySlot) continue;
-    int32_t f = sf >= 0 ? sf : ~sf;
-    const double* fl = &h.flux[(int64_t)f * 4];
-    if (sf >= 0) { for (int v = 0; v < 4; v++) s[v] += fl[v]; }
-    else { for (int v = 0; v < 4; v++) s[v] -= fl[v]; }
-    if (LAM) *lam += h.lamA[f];
+  int32_t sf[kMaxSlots];
+  double fl[kMaxSlots][4], fa[kMaxSlots];
+  cell_slots(i, h, sf);
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++) {
+    if (sf[k] == kEmptySlot) continue;
+    const int32_t f = sf[k] >= 0 ? sf[k] : ~sf[k];
+    load4_wide(&h.flux[(int64_t)f * 4], fl[k]);
+    if (LAM) fa[k] = h.lamA[f];
+  }
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++) {
+    if (sf[k] == kEmptySlot) continue;
+    if (sf[k] >= 0) { for (int v = 0; v < 4; v++) s[v] += fl[k][v]; }
+    else { for (int v = 0; v < 4; v++) s[v] -= fl[k][v]; }
+    if (LAM) *lam += fa[k];
   }
   double U[4];
   load4<T>(&h.u[i * 4], U);

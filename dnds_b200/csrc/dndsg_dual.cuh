@@ -118,17 +118,23 @@ __global__ void __launch_bounds__(kBlock) k_lusgs_matvec(HotView<T> h, double al
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= h.N) return;
   double buf[4] = {0, 0, 0, 0};
-  for (int k = 0; k < h.nfmax; k++) {
-    const int32_t sf = h.cellFace[aos(i, k, h.nfmax)];
-    if (sf == kEmptySlot) continue;
-    const int32_t f = sf >= 0 ? sf : ~sf;
-    const int32_t j = sf >= 0 ? h.faceR[f] : h.faceL[f];
-    if (j < 0) continue;
-    const double sg = sf >= 0 ? 1.0 : -1.0;
+  int32_t sf[kMaxSlots], nb[kMaxSlots];
+  cell_slots(i, h, sf);
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++) {
+    nb[k] = -1;
+    if (sf[k] != kEmptySlot) nb[k] = sf[k] >= 0 ? h.faceR[sf[k]] : h.faceL[~sf[k]];
+  }
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++) {
+    if (nb[k] < 0) continue;
+    const int32_t f = sf[k] >= 0 ? sf[k] : ~sf[k];
+    const int64_t j = nb[k];
+    const double sg = sf[k] >= 0 ? 1.0 : -1.0;
     const double area = h.faceArea[f];
     double U[4], dU[4], dF[4];
-    load4<T>(&h.u[(int64_t)j * 4], U);
-    load4<double>(&x[(int64_t)j * 4], dU);
+    load4_wide(&h.u[j * 4], U);
+    load4<double>(&x[j * 4], dU);
     flux_jac_times_du(U, sg * h.faceNormal[2 * f], sg * h.faceNormal[2 * f + 1], dU, h.lamA[f] / area, h.gamma, dF);
     const double w = (0.5 * alpha) * area / h.vol[i];
     for (int v = 0; v < 4; v++) buf[v] -= w * dF[v];

@@ -198,13 +198,16 @@ DG_HD void limiter_face_indicator(int64_t f, const LimView& v, const T* urec) {
 template <class T>
 DG_HD double limiter_cell_indicator(int64_t i, const LimView& v) {
   double sj[2] = {0, 0}, ss[2] = {0, 0};
-  for (int k = 0; k < v.nfmax; k++) {
-    int32_t sf = v.cellFace[aos(i, k, v.nfmax)];
-    if (sf == kEmptySlot) continue;
-    int32_t f = sf >= 0 ? sf : ~sf;
-    T d[4];
-    load_row(static_cast<const T*>(v.faceInd) + (int64_t)f * 4, d);
-    sj[0] += (double)d[0]; sj[1] += (double)d[1]; ss[0] += (double)d[2]; ss[1] += (double)d[3];
+  int32_t sf[kMaxSlots];
+  T d[kMaxSlots][4];
+  cell_slots(i, v, sf);
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++)
+    if (sf[k] != kEmptySlot) load_row(static_cast<const T*>(v.faceInd) + (int64_t)(sf[k] >= 0 ? sf[k] : ~sf[k]) * 4, d[k]);
+#pragma unroll
+  for (int k = 0; k < kMaxSlots; k++) {
+    if (sf[k] == kEmptySlot) continue;
+    sj[0] += (double)d[k][0]; sj[1] += (double)d[k][1]; ss[0] += (double)d[k][2]; ss[1] += (double)d[k][3];
   }
   double s0 = sj[0] / (ss[0] + kVerySmall), s1 = sj[1] / (ss[1] + kVerySmall);
   return sqrt(dmax(fabs(s0), fabs(s1))) * v.porder2;
