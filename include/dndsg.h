@@ -254,7 +254,7 @@ int dndsg_lusgs_set_order(dndsg_ctx* ctx, int mode, const int64_t* scan2cell, in
  * [0, n_parts); NULL or n_parts == 1: one part.  Rebuilds the mode-1 schedule
  * with the scan order last given to dndsg_lusgs_set_order (natural order if
  * none) and switches to it; each sweep then runs the parts' level walks
- * concurrently, one thread block per part.  Parts apply to mode 1 only; a later
+ * concurrently, a block or cluster of blocks per part.  Parts apply to mode 1 only; a later
  * dndsg_lusgs_set_order(mode 1) keeps them.  DNDSG_UNSUPPORTED (nothing
  * changed) when a cell has more than 4 faces or a part more than 4095 levels.
  * n_batches (may be NULL): the most levels of one part, forward plus backward. */
