@@ -30,6 +30,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
   return done != 0;
 }
+// the same for a barrier that the other blocks of the cluster complete: the wait orders the reads after it behind
+// the stores with which they completed it (without a scope the wait does that for this block's stores only)
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t limit) {
+  uint32_t done = 0;
+  for (uint32_t it = 0; it < limit && !done; ++it) {
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  }
+  return done != 0;
+}
 // programmatic dependent launch: lets the next kernel of the stream be launched while this one runs, and
 // waits until the one before it is complete (both do nothing in a launch without that attribute)
 __device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -38,7 +51,8 @@ __device__ __forceinline__ void pdl_enter() {
   pdl_launch_next();
   pdl_wait_previous();
 }
-// thread-block clusters: a shared-memory address of this block in block `rank`, and the hardware barrier of all threads of the cluster (release / acquire)
+// thread-block clusters: a shared-memory address of this block in block `rank`, and the hardware barrier of all
+// threads of the cluster (release / acquire)
 __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));

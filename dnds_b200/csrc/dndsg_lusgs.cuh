@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
       const double x0 = lds1(myX0 + o);
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * st) : "memory");
-      if (K > 1 && cur.z >= 0 && !failed) failed = !mbar_wait(mailB + 8 * cur.z, 0, kWaitLimit);
+      if (K > 1 && cur.z >= 0 && !failed) failed = !mbar_wait_cluster(mailB + 8 * cur.z, 0, kWaitLimit);
       const bool act = pos < cur.y && !failed;
       const int32_t sr[4] = {src4.x, src4.y, src4.z, src4.w}, push[kWalkPush] = {to.x, to.y, to.z};
       uint32_t at[NS], pushAt[kWalkPush], pushBar[kWalkPush];
