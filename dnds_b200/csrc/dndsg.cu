@@ -95,7 +95,7 @@ struct dndsg_ctx {
   // records of one sweep
   struct Walk {
     WalkDev dev{};
-    int ns = 2, blocks = 1;
+    int ns = 2, blocks = 1, width = kWalkW;
   } fwdWalk, bwdWalk;
   void *walkRec = nullptr, *walkRec5 = nullptr;
   std::vector<int32_t> colourHost;  // greedy colouring, kept for dndsg_lusgs_colours
@@ -2641,13 +2641,11 @@ constexpr int kMaxPartLevels = 4095;  // of one part, in partitioned sweeps
 constexpr double kWalkHop = 3.0;      // a value from another block of the part, in batches of the walk
 
 template <int NS, bool SA>
-bool walk_attr(int K, int mail, int bars) {
-  const int bytes = (int)walk_smem(NS, SA, mail, bars);
-  if (cudaFuncSetAttribute(k_lusgs_walk<NS, SA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmemMax) != cudaSuccess)
-    return false;
+bool walk_attr(int K, int width, int mail, int bars) {
+  auto* const k = width == kWalkW ? k_lusgs_walk<NS, SA> : k_lusgs_walk_wide<NS, SA>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmemMax) != cudaSuccess) return false;
   if (K == 1) return true;
-  if (K > 8 && cudaFuncSetAttribute(k_lusgs_walk<NS, SA>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-    return false;
+  if (K > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return false;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = (unsigned)K;
@@ -2655,23 +2653,24 @@ bool walk_attr(int K, int mail, int bars) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)K);
   cfg.blockDim = dim3(walk_threads(SA));
-  cfg.dynamicSmemBytes = bytes;
+  cfg.dynamicSmemBytes = walk_smem(NS, SA, width, mail, bars);
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int n = 0;
-  return cudaOccupancyMaxActiveClusters(&n, k_lusgs_walk<NS, SA>, &cfg) == cudaSuccess && n > 0;
+  return cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0;
 }
 // whether the device runs clusters of K blocks of the walk with this much shared memory (and the
 // kernel attributes for it)
-bool walk_fits(dndsg_ctx* c, int ns, int K, int mail, int bars) {
-  const bool ok = c->sa ? (ns == 2 ? walk_attr<2, true>(K, mail, bars) : ns == 3 ? walk_attr<3, true>(K, mail, bars) : walk_attr<4, true>(K, mail, bars))
-                        : (ns == 2 ? walk_attr<2, false>(K, mail, bars) : ns == 3 ? walk_attr<3, false>(K, mail, bars) : walk_attr<4, false>(K, mail, bars));
+bool walk_fits(dndsg_ctx* c, int ns, int K, int width, int mail, int bars) {
+  const bool ok = c->sa ? (ns == 2 ? walk_attr<2, true>(K, width, mail, bars) : ns == 3 ? walk_attr<3, true>(K, width, mail, bars) : walk_attr<4, true>(K, width, mail, bars))
+                        : (ns == 2 ? walk_attr<2, false>(K, width, mail, bars) : ns == 3 ? walk_attr<3, false>(K, width, mail, bars) : walk_attr<4, false>(K, width, mail, bars));
   if (!ok) cudaGetLastError();  // not an error of the caller's
   return ok;
 }
 int upload_walk(dndsg_ctx* c, const WalkSchedule& w, dndsg_ctx::Walk& d) {
-  if (!walk_fits(c, w.ns, w.K, w.mail, w.bars)) return fail(c, DNDSG_CUDA_ERROR, "kernel attributes of the LU-SGS walk");
+  if (!walk_fits(c, w.ns, w.K, w.width, w.mail, w.bars)) return fail(c, DNDSG_CUDA_ERROR, "kernel attributes of the LU-SGS walk");
   d.ns = w.ns;
+  d.width = w.width;
   d.blocks = w.parts * w.K;
   d.dev.K = w.K;
   d.dev.mail = w.mail;
@@ -2745,27 +2744,9 @@ int set_scan_order(dndsg_ctx* c, const int64_t* scan2cell) {
       slotF[4 * i + k] = sf;
       if (sf != kEmptySlot) slotJ[4 * i + k] = sf >= 0 ? R[sf] : L[~sf];
     }
-  // one block per part walks the part as long as that is about as short as its levels; else a cluster of
-  // blocks, one per 8 cells of a mean level (measured estimates, 512 x 128 quads in natural order, levels of
-  // 103 cells: 1, 4, 8, 16 blocks take 583, 519, 338, 190 us a sweep; 256 x 64, levels of 51: 120, 130, 81, 83 us),
-  // if the walk gets shorter by that and the device and the mailboxes take it
   WalkSchedule fwd, bwd;
-  bool several = false;
-  const double one = walk_length_one(N, P, part, lf, nlf) + walk_length_one(N, P, part, lb, nlb);
-  if (one > 1.05 * (fMax + bMax)) {
-    int K = 2;
-    while (K < kWalkMaxK && K * 8.0 < 2.0 * N / (fMax + bMax) / P) K *= 2;
-    while (K > 1 && (int64_t)P * K > c->sms) K /= 2;
-    const int maxMail = walk_max_mail(std::min(4, c->nfmax), c->sa);
-    several = K > 1 && build_walk(N, P, part, order, pos, lf, slotF, slotJ, true, K, maxMail, kWalkHop, fwd) &&
-              build_walk(N, P, part, order, pos, lb, slotF, slotJ, false, K, maxMail, kWalkHop, bwd) &&
-              fwd.time + bwd.time < 0.95 * one &&
-              walk_fits(c, std::max(fwd.ns, bwd.ns), K, std::max(fwd.mail, bwd.mail), std::max(fwd.bars, bwd.bars));
-  }
-  if (!several) {
-    build_walk(N, P, part, order, pos, lf, slotF, slotJ, true, 1, 0, kWalkHop, fwd);
-    build_walk(N, P, part, order, pos, lb, slotF, slotJ, false, 1, 0, kWalkHop, bwd);
-  }
+  choose_walks(N, P, part, order, pos, lf, nlf, lb, nlb, slotF, slotJ, c->sa, c->sms, kWalkHop,
+               [&](int ns, int K, int mail, int bars) { return walk_fits(c, ns, K, kWalkW, mail, bars); }, fwd, bwd);
   if ((rc = upload_walk(c, fwd, c->fwdWalk)) || (rc = upload_walk(c, bwd, c->bwdWalk))) return rc;
   dfree(c, c->walkRec);
   dfree(c, c->walkRec5);
@@ -2796,11 +2777,11 @@ void launch_walk_ns(dndsg_ctx* c, bool forward, const dndsg_ctx::Walk& w, const 
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)w.blocks);
   cfg.blockDim = dim3(walk_threads(SA));
-  cfg.dynamicSmemBytes = walk_smem(NS, SA, w.dev.mail, w.dev.bars);
+  cfg.dynamicSmemBytes = walk_smem(NS, SA, w.width, w.dev.mail, w.dev.bars);
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_lusgs_walk<NS, SA>, w.dev, (const unsigned char*)rec, (const unsigned char*)rec5, inc, inc5, c->flags);
+  cudaLaunchKernelEx(&cfg, w.width == kWalkW ? k_lusgs_walk<NS, SA> : k_lusgs_walk_wide<NS, SA>, w.dev, (const unsigned char*)rec, (const unsigned char*)rec5, inc, inc5, c->flags);
 }
 template <bool SA>
 void launch_walk(dndsg_ctx* c, bool forward, double alpha, const double* rhs, double* inc, const double* rhs5, double* inc5,

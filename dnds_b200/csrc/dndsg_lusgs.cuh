@@ -23,22 +23,6 @@ namespace dg {
 // level, took longer than the level: 0.6-0.7 us.  Now 0.21 us per level (0.27 us with U5): forward or
 // backward sweep in natural order on 512 x 128 quads with U5 480 -> 190 us, on 256 x 64 quads 203 -> 81 us,
 // 16 parts of the former 97 -> 47 us.
-constexpr int walk_rec_bytes(int ns) { return ns * 128 + 64; }   // rows, x0[4], WalkMeta; 64 mod 128: 16-byte loads of a
-                                                                 // quarter warp (two positions) meet no bank twice
-constexpr int walk_rec5_bytes(int ns) { return ns * 32 + 16; }   // U5: rows, x0, padding (an odd number of 16-byte units)
-constexpr int kWalkStages = 6;                                   // batches of records in flight
-constexpr int kWalkCopy = 2;                                     // copying warps
-constexpr int walk_rows(bool sa) { return 4 * kWalkW + (sa ? 32 : 0); }              // threads that compute a batch: rows, U5
-constexpr int walk_threads(bool sa) { return 2 * walk_rows(sa) + 32 * kWalkCopy; }   // two sets and the copying warps
-// shared memory: the stages' barriers, the mailbox barriers, values, U5 values, the stages' records
-constexpr size_t walk_smem(int ns, bool sa, int mail, int bars) {
-  return 16 * kWalkStages + (((size_t)bars * 8 + 31) & ~(size_t)31) + (size_t)(kWalkZero + 1 + mail) * 32 +
-         (sa ? ((size_t)(kWalkZero + 1 + mail) * 8 + 15) & ~(size_t)15 : 0) +
-         (size_t)kWalkStages * kWalkW * (walk_rec_bytes(ns) + (sa ? walk_rec5_bytes(ns) : 0));
-}
-constexpr size_t kWalkSmemMax = 227 * 1024;
-// the mailbox slots that fit, each with a barrier of its own at worst
-constexpr int walk_max_mail(int ns, bool sa) { return (int)((kWalkSmemMax - walk_smem(ns, sa, 0, 0) - 64) / (sa ? 48 : 40)); }
 
 // the fields of a context that the records are made of
 struct WalkGeom {
@@ -148,6 +132,41 @@ __device__ __forceinline__ int4 lds_i4(uint32_t a) {
 }
 __device__ __forceinline__ void sts1(uint32_t a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
 
+// A copying warp (w of kWalkCopy) of a walk: every kWalkCopy-th batch's records into its stage.  Returns its last
+// batch; failed: a wait ran out.
+template <int RB, int RB5, int S, int W>
+__device__ __forceinline__ int walk_copy(int w, int lane, int32_t nb, const WalkBatch* bat, const unsigned char* rec,
+                                         const unsigned char* rec5, uint32_t full, uint32_t empty, uint32_t stR, uint32_t stR5,
+                                         bool& failed) {
+  int last = -1;
+  int32_t first = 0, cnt = 0;  // lane k keeps the first positions of the warp's k-th next batches
+  for (int l = w, k = 0; l < nb; l += kWalkCopy, k = (k + 1) & 31) {
+    if (k == 0) {
+      const WalkBatch x = bat[min(l + kWalkCopy * lane, nb - 1)];
+      first = x.first;
+      cnt = x.n;
+    }
+    const int32_t a = __shfl_sync(0xffffffffu, first, k), n = __shfl_sync(0xffffffffu, cnt, k);
+    const uint32_t st = (uint32_t)(l % S), bar = full + 8 * st;
+    const bool ok = l < S || mbar_wait(empty + 8 * st, (uint32_t)(l / S - 1) & 1u, kWaitLimit);
+    failed = __any_sync(0xffffffffu, !ok);
+    if (failed) break;
+    if (lane == 0) {
+      mbar_expect_tx(bar, (uint32_t)(n * (RB + RB5)));
+      bulk_g2s(stR + st * W * RB, rec + (int64_t)a * RB, (uint32_t)(n * RB), bar);
+      if (RB5) bulk_g2s(stR5 + st * W * RB5, rec5 + (int64_t)a * RB5, (uint32_t)(n * RB5), bar);
+    }
+    last = l;
+  }
+  return last;
+}
+// after a timeout: the warp's copies in flight land before the block leaves
+template <int S>
+__device__ __forceinline__ void walk_drain(int last, uint32_t full) {
+  for (int l = max(last - S + kWalkCopy, 0); l <= last; l++)
+    if (l % kWalkCopy == last % kWalkCopy) mbar_wait(full + 8 * (l % S), (uint32_t)(l / S) & 1u, kWaitLimit);
+}
+
 // The walk, one block per run of scan positions, K blocks per part in a cluster.  Two sets of warps take the
 // batches in turn.  Of a set, warps 0-3 hold row v = lane & 3 of position 8 warp + lane / 4; SA: one warp
 // more, U5 of position `lane`.  A set loads its next records into registers while the other one
@@ -155,7 +174,7 @@ __device__ __forceinline__ void sts1(uint32_t a, double v) { asm volatile("st.sh
 // product, the store and the barrier between the sets (the set that finished batch l arrives, the one that
 // takes l + 1 waits).  An increment for another block goes by st.async, which completes a barrier of the
 // batch that needs it there: no fence, and the wait for it lies before the barrier between the sets.  The
-// copying warps keep kWalkStages batches of records in flight (two of them: one's round per batch took
+// copying warps keep walk_stages() batches of records in flight (two of them: one's round per batch took
 // longer than a level, 0.29 against 0.22 us).  A wait that runs out sets kFlagTimeout; its warp then skips
 // the rest of its work, keeps to every barrier, and the blocks leave together (a mailbox may be written until
 // its block's peers are done).
@@ -165,7 +184,7 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
                                                                     unsigned* flags) {
   extern __shared__ __align__(128) unsigned char sm[];
   constexpr int RB = walk_rec_bytes(NS), RB5 = SA ? walk_rec5_bytes(NS) : 0;
-  constexpr int S = kWalkStages, NW = walk_rows(SA) / 32;  // warps of a set
+  constexpr int S = walk_stages(kWalkW), NW = walk_rows(SA) / 32;  // warps of a set
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int K = sc.K, nval = kWalkZero + 1 + sc.mail;
   const uint32_t full = smem_u32(sm), empty = full + 8 * S, mailB = full + 16 * S, vals = mailB + ((sc.bars * 8 + 31) & ~31),
@@ -196,27 +215,7 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
   bool failed = false;
   int last = -1;  // the copying warp's last batch
   if (warp >= 2 * NW) {
-    // copying warp w takes every kWalkCopy-th batch; lane k keeps the first positions of its k-th next ones
-    const int w = warp - 2 * NW;
-    int32_t first = 0, cnt = 0;
-    for (int l = w, k = 0; l < nb; l += kWalkCopy, k = (k + 1) & 31) {
-      if (k == 0) {
-        const WalkBatch x = bat[min(l + kWalkCopy * lane, nb - 1)];
-        first = x.first;
-        cnt = x.n;
-      }
-      const int32_t a = __shfl_sync(0xffffffffu, first, k), n = __shfl_sync(0xffffffffu, cnt, k);
-      const uint32_t st = (uint32_t)(l % S), bar = full + 8 * st;
-      const bool ok = l < S || mbar_wait(empty + 8 * st, (uint32_t)(l / S - 1) & 1u, kWaitLimit);
-      failed = __any_sync(0xffffffffu, !ok);
-      if (failed) break;
-      if (lane == 0) {
-        mbar_expect_tx(bar, (uint32_t)(n * (RB + RB5)));
-        bulk_g2s(stR + st * kWalkW * RB, rec + (int64_t)a * RB, (uint32_t)(n * RB), bar);
-        if (SA) bulk_g2s(stR5 + st * kWalkW * RB5, rec5 + (int64_t)a * RB5, (uint32_t)(n * RB5), bar);
-      }
-      last = l;
-    }
+    last = walk_copy<RB, RB5, S, kWalkW>(warp - 2 * NW, lane, nb, bat, rec, rec5, full, empty, stR, stR5, failed);
   } else {
     const int set = warp >= NW ? 1 : 0, sw = warp - set * NW;
     const bool rows = sw < 4;
@@ -272,8 +271,8 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
 #pragma unroll
         for (int q = 0; q < NS; q++) {
           d[q][0] = lds2(at[q]);
-          d[q][1] = lds2(at[q] + 16);
-          if (SA && !rows) d[q][1].y = lds1(vals5 + ((at[q] - vals) >> 2));
+          if (SA && !rows) d[q][1] = make_double2(lds1(at[q] + 16), lds1(vals5 + ((at[q] - vals) >> 2)));
+          else d[q][1] = lds2(at[q] + 16);
         }
         if (old) {
 #pragma unroll
@@ -281,8 +280,9 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
             if (sr[q] < 0) {  // a position of this block that left the ring, stored before an earlier barrier
               const int64_t j = -(int64_t)sr[q] - 1;
               d[q][0] = *reinterpret_cast<const double2*>(&inc[4 * j]);
-              d[q][1] = *reinterpret_cast<const double2*>(&inc[4 * j + 2]);
-              if (SA && !rows) d[q][1].y = inc5[j];
+              // (one load for both and the U5 value over it would make the U5 warp wait once per neighbour)
+              if (SA && !rows) d[q][1] = make_double2(inc[4 * j + 2], inc5[j]);
+              else d[q][1] = *reinterpret_cast<const double2*>(&inc[4 * j + 2]);
             }
         }
         double b = 0.0;
@@ -316,14 +316,150 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
   }
   if (failed) atomicOr(flags, kFlagTimeout);
   __syncwarp();
-  // after a timeout: the copies in flight land before the block leaves
-  if (__syncthreads_or(failed) && lane == 0)
-    for (int l = max(last - S + kWalkCopy, 0); l <= last; l++)
-      if (l % kWalkCopy == last % kWalkCopy) mbar_wait(full + 8 * (l % S), (uint32_t)(l / S) & 1u, kWaitLimit);
+  if (__syncthreads_or(failed) && lane == 0) walk_drain<S>(last, full);
   if (K > 1) {
     __syncwarp();
     cluster_sync_all();
   }
+}
+
+// The walk of parts of one block with wide levels: batches of kWalkWide positions, two of them (32 apart) in every
+// lane.  There the latency of a set's own round (its records into registers, the increments, the store) bounds the
+// walk, and two positions share it: sweeps in one block of 512 x 128 quads in natural order, levels of 103 cells, 462 ->
+// 315 us, of 256 x 64, levels of 51, 127 -> 91 us; of 262,144 quads numbered at random 4,035 -> 3,160 us (65,536 with
+// U5: the iteration 2,830 -> 2,494 us); 75 parts of 112 x 224 quads 538 -> 498 us.  An increment that left the ring was
+// stored at least four batches and as many barriers before.
+template <int NS, bool SA>
+__global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk_wide(WalkDev sc, const unsigned char* rec,
+                                                                                   const unsigned char* rec5, double* inc,
+                                                                                   double* inc5, unsigned* flags) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  constexpr int RB = walk_rec_bytes(NS), RB5 = SA ? walk_rec5_bytes(NS) : 0;
+  constexpr int W = kWalkWide, S = walk_stages(W), NW = walk_rows(SA) / 32, R = W / 32;  // NW: warps of a set
+  constexpr int nval = kWalkZero + 1;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t full = smem_u32(sm), empty = full + 8 * S, vals = full + 16 * S, vals5 = vals + nval * 32;
+  const uint32_t stR = vals5 + (SA ? ((nval * 8 + 15) & ~15) : 0), stR5 = stR + S * W * RB;
+  const int32_t b0 = sc.blockBatch[blockIdx.x], nb = sc.blockBatch[blockIdx.x + 1] - b0;
+  const WalkBatch* bat = sc.batches + b0;
+  if (tid == 0)
+    for (int k = 0; k < S; k++) {
+      mbar_init(full + 8 * k, 1);
+      mbar_init(empty + 8 * k, NW);
+    }
+  fence_mbar_init();
+  if (tid < 4) sts1(vals + kWalkZero * 32 + 8 * tid, 0.0);
+  if (SA && tid == 4) sts1(vals5 + kWalkZero * 8, 0.0);
+  __syncthreads();
+  bool failed = false;
+  int last = -1;
+  if (warp >= 2 * NW) {
+    last = walk_copy<RB, RB5, S, W>(warp - 2 * NW, lane, nb, bat, rec, rec5, full, empty, stR, stR5, failed);
+  } else {
+    const int set = warp >= NW ? 1 : 0, sw = warp - set * NW;
+    const bool rows = sw < 4;
+    const int32_t p0 = nb > 0 ? bat[0].first : 0;
+    const int v = lane & 3;
+    const int pos = rows ? sw * 8 + (lane >> 2) : lane;  // and 32 more
+    const uint32_t myRec = stR + pos * RB, myRow = rows ? myRec + v * 16 : stR5 + pos * RB5,
+                   myX0 = rows ? myRec + NS * 128 + 8 * v : myRow + NS * 32;
+    constexpr int kSets = 2 * walk_rows(SA);  // threads of both sets, which the barriers 1 and 2 count
+    int4 bt = set < nb ? *reinterpret_cast<const int4*>(bat + set) : make_int4(0, 0, -1, 0);
+    for (int l = set; l < nb; l += 2) {
+      // ---- beside the other set's batch: the records of this one
+      const uint32_t st = (uint32_t)(l % S), o = st * (rows ? W * RB : W * RB5);
+      const int4 cur = bt;  // first position, positions
+      if (l + 2 < nb) bt = *reinterpret_cast<const int4*>(bat + l + 2);
+      if (!failed) failed = !mbar_wait(full + 8 * st, (uint32_t)(l / S) & 1u, kWaitLimit);
+      // (lanes past the batch's positions read stale data and drop it)
+      int4 src4[R];
+      int32_t cell[R];
+      double2 m[R][NS][2];
+      double x0[R];
+#pragma unroll
+      for (int e = 0; e < R; e++) {
+        const uint32_t r = myRec + (st * W + 32 * e) * RB, y = o + 32 * e * (rows ? RB : RB5);
+        src4[e] = lds_i4(r + NS * 128 + 32);
+        cell[e] = lds_i4(r + NS * 128 + 48).w;
+#pragma unroll
+        for (int q = 0; q < NS; q++) {
+          m[e][q][0] = lds2(myRow + y + (rows ? q * 128 : q * 32));
+          m[e][q][1] = lds2(myRow + y + (rows ? q * 128 + 64 : q * 32 + 16));
+        }
+        x0[e] = lds1(myX0 + y);
+      }
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * st) : "memory");
+      bool act[R], old = false;
+      uint32_t at[R][NS], mine[R];
+#pragma unroll
+      for (int e = 0; e < R; e++) {
+        act[e] = pos + 32 * e < cur.y && !failed;
+        const int32_t sr[4] = {src4[e].x, src4[e].y, src4[e].z, src4[e].w};
+#pragma unroll
+        for (int q = 0; q < NS; q++) {
+          at[e][q] = vals + (uint32_t)(sr[q] < 0 || !act[e] ? kWalkZero * 32 : sr[q]);
+          old = old || (sr[q] < 0 && act[e]);
+        }
+        const uint32_t slot = (uint32_t)(cur.x + pos + 32 * e - p0) & (kWalkRing - 1);
+        mine[e] = rows ? vals + slot * 32 + 8 * v : vals5 + slot * 8;
+      }
+      // ---- batch l - 1 is finished
+      if (l > 0) asm volatile("bar.sync %0, %1;" ::"r"(1 + ((l - 1) & 1)), "n"(kSets) : "memory");
+      double2 d[R][NS][2];
+#pragma unroll
+      for (int e = 0; e < R; e++)
+#pragma unroll
+        for (int q = 0; q < NS; q++) {
+          d[e][q][0] = lds2(at[e][q]);
+          if (SA && !rows) d[e][q][1] = make_double2(lds1(at[e][q] + 16), lds1(vals5 + ((at[e][q] - vals) >> 2)));
+          else d[e][q][1] = lds2(at[e][q] + 16);
+        }
+      if (old) {
+#pragma unroll
+        for (int e = 0; e < R; e++) {
+          const int32_t sr[4] = {src4[e].x, src4[e].y, src4[e].z, src4[e].w};
+#pragma unroll
+          for (int q = 0; q < NS; q++)
+            if (act[e] && sr[q] < 0) {
+              const int64_t j = -(int64_t)sr[q] - 1;
+              d[e][q][0] = *reinterpret_cast<const double2*>(&inc[4 * j]);
+              if (SA && !rows) d[e][q][1] = make_double2(inc[4 * j + 2], inc5[j]);
+              else d[e][q][1] = *reinterpret_cast<const double2*>(&inc[4 * j + 2]);
+            }
+        }
+      }
+      double a[R];
+#pragma unroll
+      for (int e = 0; e < R; e++) {
+        double b = 0.0;
+        a[e] = x0[e];
+#pragma unroll
+        for (int q = 0; q < NS; q++) {
+          const double s0 = fma(m[e][q][0].y, d[e][q][0].y, m[e][q][0].x * d[e][q][0].x);
+          const double s1 = fma(m[e][q][1].y, d[e][q][1].y, m[e][q][1].x * d[e][q][1].x);
+          if (q & 1) b += s0 + s1;
+          else a[e] += s0 + s1;
+        }
+        a[e] += b;
+      }
+#pragma unroll
+      for (int e = 0; e < R; e++)
+        if (act[e]) sts1(mine[e], a[e]);
+      asm volatile("bar.arrive %0, %1;" ::"r"(1 + (l & 1)), "n"(kSets) : "memory");
+#pragma unroll
+      for (int e = 0; e < R; e++)
+        if (act[e]) {
+          if (rows) inc[4 * (int64_t)cell[e] + v] = a[e];
+          else inc5[cell[e]] = a[e];
+        }
+    }
+    if (nb > 0 && set == (nb & 1))  // the set that did not take the last batch
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + ((nb - 1) & 1)), "n"(kSets) : "memory");
+  }
+  if (failed) atomicOr(flags, kFlagTimeout);
+  __syncwarp();
+  if (__syncthreads_or(failed) && lane == 0) walk_drain<S>(last, full);
 }
 
 }  // namespace dg

@@ -4,10 +4,11 @@
 //
 // A sweep in scan order is a chain of dependency levels (a cell's level is one more than the largest
 // level of its earlier neighbours).  Each part (the reference's rank) is cut into K runs of consecutive
-// scan positions, one thread block per run, the K blocks of a part being one thread-block cluster.  A
-// block walks its own cells level by level in batches of at most kWalkW cells, a block barrier between
-// batches.  Dependencies go from lower runs to higher ones in the forward sweep and the other way in the
-// backward one, so the blocks never wait on one another in a circle.  A neighbour's increment is read from
+// scan positions or of consecutive cells, one thread block per run, the K blocks of a part being one
+// thread-block cluster.  A block walks its own cells level by level in batches of at most kWalkW cells (kWalkWide
+// in parts of one block with wide levels), a block barrier between batches.  Every block takes its levels in order and
+// a cell needs lower levels only, so the blocks never wait on one another in a circle.  A neighbour's increment is
+// read from
 //   * a ring of the block's own last kWalkRing positions (shared memory),
 //   * the block's mailbox (shared memory), one slot per cell of another run that it needs: the block that
 //     computes the cell stores it there over distributed shared memory, signalling a barrier of the batch that
@@ -21,6 +22,8 @@
 namespace dg {
 
 constexpr int kWalkW = 32;      // cells per batch: 4 lanes each, four warps
+constexpr int kWalkWide = 64;   // two cells per lane
+constexpr double kWalkWideCost = 1.3;  // a wide batch (0.24-0.26 us, quads in natural order) in batches of kWalkW (0.19-0.2 us)
 constexpr int kWalkRing = 256;  // positions in the ring (a power of two)
 constexpr int kWalkMaxK = 16;   // blocks per part (one cluster)
 constexpr int kWalkZero = kWalkRing;
@@ -28,6 +31,25 @@ constexpr int kWalkPush = 3;    // mailboxes that one cell's increment can go to
 constexpr int kWalkSlotBits = 13, kWalkMaxMail = (1 << kWalkSlotBits) - 1;
 // a mailbox and its barrier as one non-negative number: block of the part, barrier, slot
 inline int32_t walk_push(int block, int bar, int slot) { return (block << (2 * kWalkSlotBits)) | (bar << kWalkSlotBits) | slot; }
+
+// The walk's shared memory.  A record holds a position's matrix rows (dndsg_lusgs.cuh), x0[4] and its WalkMeta
+constexpr int walk_rec_bytes(int ns) { return ns * 128 + 64; }   // 64 mod 128: 16-byte loads of a quarter warp (two positions)
+                                                                 // meet no bank twice
+constexpr int walk_rec5_bytes(int ns) { return ns * 32 + 16; }   // U5: rows, x0, padding (an odd number of 16-byte units)
+constexpr int walk_stages(int width) { return width == kWalkW ? 6 : 4; }             // batches of records in flight
+constexpr int kWalkCopy = 2;                                                         // copying warps
+constexpr int walk_rows(bool sa) { return 4 * kWalkW + (sa ? 32 : 0); }              // threads that compute a batch: rows, U5
+constexpr int walk_threads(bool sa) { return 2 * walk_rows(sa) + 32 * kWalkCopy; }   // two sets and the copying warps
+// the stages' barriers, the mailbox barriers, values, U5 values, the stages' records
+constexpr size_t walk_smem(int ns, bool sa, int width, int mail, int bars) {
+  return (((size_t)walk_stages(width) * 16 + (size_t)bars * 8 + 31) & ~(size_t)31) + (size_t)(kWalkZero + 1 + mail) * 32 +
+         (sa ? ((size_t)(kWalkZero + 1 + mail) * 8 + 15) & ~(size_t)15 : 0) +
+         (size_t)walk_stages(width) * width * (walk_rec_bytes(ns) + (sa ? walk_rec5_bytes(ns) : 0));
+}
+constexpr size_t kWalkSmemMax = 227 * 1024;
+static_assert(walk_smem(4, true, kWalkWide, 0, 0) <= kWalkSmemMax && walk_smem(4, true, kWalkW, 0, 0) <= kWalkSmemMax, "one block fits");
+// no more mailbox slots than this fit (walk_smem of the schedule itself decides)
+constexpr int walk_max_mail(int ns, bool sa) { return (int)((kWalkSmemMax - walk_smem(ns, sa, kWalkW, 0, 0)) / (sa ? 40 : 32)); }
 
 // per schedule position, 32 bytes, copied into its record:
 //   src[4]   where the increment of used neighbour q is: 32 times a slot of the block's shared values (ring
@@ -48,6 +70,7 @@ static_assert(sizeof(WalkBatch) == 16, "read as one vector");
 
 struct WalkSchedule {
   int K = 1, parts = 1, ns = 2;  // ns: neighbour slots per record (2..4)
+  int width = kWalkW;            // most cells of a batch
   int mail = 0, bars = 0;        // largest mailbox, most mailbox barriers of a block
   int maxBatches = 0;                      // of one block
   double time = 0;                         // estimated length of the walk in batches
@@ -62,7 +85,7 @@ constexpr int32_t kWalkGhost = -2;
 
 // the length of the walk in batches with one block per part; levels[p]: the levels of part p
 inline double walk_length_one(int64_t N, int parts, const std::vector<int32_t>& part, const std::vector<int32_t>& level,
-                              const std::vector<int32_t>& levels) {
+                              const std::vector<int32_t>& levels, int batch = kWalkW) {
   std::vector<int64_t> first(parts + 1, 0);
   for (int p = 0; p < parts; p++) first[p + 1] = first[p] + levels[p];
   std::vector<int32_t> width(first[parts], 0);
@@ -70,7 +93,7 @@ inline double walk_length_one(int64_t N, int parts, const std::vector<int32_t>& 
   int64_t most = 0;
   for (int p = 0; p < parts; p++) {
     int64_t n = 0;
-    for (int64_t l = first[p]; l < first[p + 1]; l++) n += (width[l] + kWalkW - 1) / kWalkW;
+    for (int64_t l = first[p]; l < first[p + 1]; l++) n += (width[l] + batch - 1) / batch;
     most = std::max(most, n);
   }
   return (double)most;
@@ -78,20 +101,23 @@ inline double walk_length_one(int64_t N, int parts, const std::vector<int32_t>& 
 
 // slotF / slotJ [N][4]: a cell's faces and the cells across (-1: none); pos: scan position; level: the
 // cell's dependency level in this sweep.  False if the mailboxes of this K would need more than maxMail
-// slots or a cell more than kWalkPush mailboxes; K = 1 always works.
+// slots or a cell more than kWalkPush mailboxes; K = 1 always works.  width: cells per batch (kWalkWide: K = 1);
+// byCell: runs of consecutive cells instead of scan positions.
 inline bool build_walk(int64_t N, int parts, const std::vector<int32_t>& part, const std::vector<int32_t>& order,
                        const std::vector<int32_t>& pos, const std::vector<int32_t>& level, const std::vector<int32_t>& slotF,
-                       const std::vector<int32_t>& slotJ, bool forward, int K, int maxMail, double hop, WalkSchedule& w) {
+                       const std::vector<int32_t>& slotJ, bool forward, int K, int maxMail, double hop, WalkSchedule& w,
+                       int width = kWalkW, bool byCell = false) {
   w = WalkSchedule();
   w.K = K;
   w.parts = parts;
+  w.width = width;
   const int nblk = parts * K;
-  // runs: consecutive scan positions of a part
+  // runs: consecutive scan positions, or cells, of a part
   std::vector<int64_t> count(parts, 0), seen(parts, 0);
   for (int64_t i = 0; i < N; i++) count[part[i]]++;
   std::vector<int32_t> blk(N);
   for (int64_t s = 0; s < N; s++) {
-    const int32_t i = order[s], p = part[i];
+    const int32_t i = byCell ? (int32_t)s : order[s], p = part[i];
     blk[i] = p * K + (int32_t)(seen[p]++ * K / count[p]);
   }
   // schedule order: block, level, cell
@@ -114,7 +140,7 @@ inline bool build_walk(int64_t N, int parts, const std::vector<int32_t>& part, c
     w.blockBatch[b] = (int32_t)w.batches.size();
     for (int64_t t = start[b]; t < start[b + 1]; t++) {
       const int32_t i = w.cells[t];
-      if (t == start[b] || w.batches.back().n == kWalkW || level[i] != level[w.cells[t - 1]])
+      if (t == start[b] || w.batches.back().n == width || level[i] != level[w.cells[t - 1]])
         w.batches.push_back(WalkBatch{(int32_t)t, 0, -1, 0});
       w.batches.back().n++;
       posn[i] = (int32_t)t;
@@ -171,23 +197,73 @@ inline bool build_walk(int64_t N, int parts, const std::vector<int32_t>& part, c
   w.mail = *std::max_element(mail.begin(), mail.end());
   w.bars = *std::max_element(bars.begin(), bars.end());
   // length of the walk: a batch takes 1, a value from another block `hop` more
-  std::vector<double> done(w.batches.size(), 0.0);
-  for (int p = 0; p < parts; p++)
-    for (int c = 0; c < K; c++) {
-      const int b = p * K + (forward ? c : K - 1 - c);
-      double now = 0;
-      for (int32_t x = w.blockBatch[b]; x < w.blockBatch[b + 1]; x++) {
-        if (w.batches[x].bar >= 0)
-          for (int64_t t = w.batches[x].first; t < w.batches[x].first + w.batches[x].n; t++)
+  if (K == 1) {
+    w.time = w.maxBatches;
+    return true;
+  }
+  std::vector<double> done(w.batches.size(), 0.0), now(nblk, 0.0);
+  std::vector<int32_t> next(w.blockBatch.begin(), w.blockBatch.end() - 1);
+  for (int l = 0; l < nlev; l++)
+    for (int b = 0; b < nblk; b++)
+      for (; next[b] < w.blockBatch[b + 1] && level[w.cells[w.batches[next[b]].first]] == l; next[b]++) {
+        const WalkBatch& x = w.batches[next[b]];
+        if (x.bar >= 0)
+          for (int64_t t = x.first; t < x.first + x.n; t++)
             for (int k = 0; k < 4; k++) {
               const int32_t j = w.nbJ[4 * t + k];
-              if (j >= 0 && blk[j] != b) now = std::max(now, done[batchOf[j]] + hop);
+              if (j >= 0 && blk[j] != b) now[b] = std::max(now[b], done[batchOf[j]] + hop);
             }
-        done[x] = ++now;
+        done[next[b]] = ++now[b];
       }
-      w.time = std::max(w.time, now);
-    }
+  w.time = *std::max_element(now.begin(), now.end());
   return true;
+}
+
+// The schedules of both sweeps.  A part is walked by a cluster of blocks, one per 8 cells of a mean level, where the
+// lengths of the walks make that shorter than one block; sweeps of quads in natural order, us (lengths):
+//                              one block     one block, wide   cluster of 16 or 8
+//   512 x 128, 103 a level     462 (2172)      315 (1495)         201 (684)
+//   1000 x 70, 65 a level      620 (3015)      565 (2613)         331 (2119)
+//   256 x 64, 51 a level       127 (574)        91 (415)          102 (340)
+// (0.15-0.26 us per batch of a cluster, so that near the line the lengths may take the slower one, by a tenth).  The
+// blocks have runs of consecutive scan positions, or of cells where those of the scan order do not fit (an order that
+// jumps about the mesh: its neighbours are in other runs), and there are half as many where those do not either: when
+// the walk does not get shorter by them, the mailboxes do not fit the shared memory, or the device (fits(ns, K, mail,
+// bars)) does not take such a cluster.
+template <class Fits>
+inline void choose_walks(int64_t N, int parts, const std::vector<int32_t>& part, const std::vector<int32_t>& order,
+                         const std::vector<int32_t>& pos, const std::vector<int32_t>& lf, const std::vector<int32_t>& nlf,
+                         const std::vector<int32_t>& lb, const std::vector<int32_t>& nlb, const std::vector<int32_t>& slotF,
+                         const std::vector<int32_t>& slotJ, bool sa, int sms, double hop, Fits&& fits, WalkSchedule& fwd,
+                         WalkSchedule& bwd) {
+  const int levels = *std::max_element(nlf.begin(), nlf.end()) + *std::max_element(nlb.begin(), nlb.end());
+  auto length = [&](int width) {
+    return walk_length_one(N, parts, part, lf, nlf, width) + walk_length_one(N, parts, part, lb, nlb, width);
+  };
+  const double one = length(kWalkW), wide = kWalkWideCost * length(kWalkWide);
+  int K = 1;
+  if (one > 1.05 * levels) {
+    K = 2;
+    while (K < kWalkMaxK && K * 8.0 < 2.0 * N / levels / parts) K *= 2;
+    while (K > 1 && (int64_t)parts * K > sms) K /= 2;
+  }
+  bool natural = true, reverse = true;  // the runs are those of the cells anyway
+  for (int64_t s = 0; s < N && (natural || reverse); s++) {
+    natural = natural && order[s] == s;
+    reverse = reverse && order[s] == N - 1 - s;
+  }
+  for (; K > 1; K /= 2)
+    for (int byCell = 0; byCell < (natural || reverse ? 1 : 2); byCell++) {
+      auto build = [&](bool forward, WalkSchedule& w) {
+        return build_walk(N, parts, part, order, pos, forward ? lf : lb, slotF, slotJ, forward, K, walk_max_mail(2, sa), hop, w,
+                          kWalkW, byCell) &&
+               walk_smem(w.ns, sa, kWalkW, w.mail, w.bars) <= kWalkSmemMax && fits(w.ns, K, w.mail, w.bars);
+      };
+      if (build(true, fwd) && build(false, bwd) && fwd.time + bwd.time < 0.95 * std::min(one, wide)) return;
+    }
+  const int width = wide < one ? kWalkWide : kWalkW;
+  build_walk(N, parts, part, order, pos, lf, slotF, slotJ, true, 1, 0, hop, fwd, width);
+  build_walk(N, parts, part, order, pos, lb, slotF, slotJ, false, 1, 0, hop, bwd, width);
 }
 
 }  // namespace dg
