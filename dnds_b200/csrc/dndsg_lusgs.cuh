@@ -167,6 +167,8 @@ __device__ __forceinline__ void walk_drain(int last, uint32_t full) {
     if (l % kWalkCopy == last % kWalkCopy) mbar_wait(full + 8 * (l % S), (uint32_t)(l / S) & 1u, kWaitLimit);
 }
 
+constexpr uint32_t kWalkDrain = 1u << 10;  // tries of a wait for what is on its way between two blocks (10 us and more)
+
 // The walk, one block per run of scan positions, K blocks per part in a cluster.  Two sets of warps take the
 // batches in turn.  Of a set, warps 0-3 hold row v = lane & 3 of position 8 warp + lane / 4; SA: one warp
 // more, U5 of position `lane`.  A set loads its next records into registers while the other one
@@ -177,7 +179,7 @@ __device__ __forceinline__ void walk_drain(int last, uint32_t full) {
 // copying warps keep walk_stages() batches of records in flight (two of them: one's round per batch took
 // longer than a level, 0.29 against 0.22 us).  A wait that runs out sets kFlagTimeout; its warp then skips
 // the rest of its work, keeps to every barrier, and the blocks leave together (a mailbox may be written until
-// its block's peers are done).
+// its block's peers are done, and a little later for one whose own waits did not see the last increments come).
 template <int NS, bool SA>
 __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, const unsigned char* rec,
                                                                     const unsigned char* rec5, double* inc, double* inc5,
@@ -316,10 +318,16 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
   }
   if (failed) atomicOr(flags, kFlagTimeout);
   __syncwarp();
-  if (__syncthreads_or(failed) && lane == 0) walk_drain<S>(last, full);
+  const bool any = __syncthreads_or(failed);
+  if (any && lane == 0) walk_drain<S>(last, full);
   if (K > 1) {
     __syncwarp();
-    cluster_sync_all();
+    cluster_sync_all();  // no increment is sent after this
+    if (any)  // those on their way here land before the block leaves; the ones that a failed warp left out never do
+      for (int l = tid; l < nb; l += blockDim.x) {
+        const WalkBatch x = bat[l];
+        if (x.bar >= 0) mbar_wait_cluster(mailB + 8 * x.bar, 0, kWalkDrain);
+      }
   }
 }
 
