@@ -98,6 +98,7 @@ struct dndsg_ctx {
     int ns = 2, blocks = 1, width = kWalkW;
   } fwdWalk, bwdWalk;
   void *walkRec = nullptr, *walkRec5 = nullptr;
+  int walkRecNs = 0;  // neighbour slots of the records that these buffers hold
   std::vector<int32_t> colourHost;  // greedy colouring, kept for dndsg_lusgs_colours
   int lusgsOrder = 0;               // 0 colour batches, 1 level-scheduled scan order
   // partitioned scan-order sweeps (the reference on several ranks): the part of every cell (empty:
@@ -156,7 +157,10 @@ template <class P>
 int dalloc(dndsg_ctx* c, P*& p, size_t bytes) {
   void* q = nullptr;
   cudaError_t e = cudaMalloc(&q, bytes > 0 ? bytes : 16);
-  if (e != cudaSuccess) return fail(c, DNDSG_CUDA_ERROR, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here; not the next launch's error
+    return fail(c, DNDSG_CUDA_ERROR, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
   c->allocs.push_back(q);
   p = (P*)q;
   return 0;
@@ -2667,6 +2671,7 @@ bool walk_fits(dndsg_ctx* c, int ns, int K, int width, int mail, int bars) {
   if (!ok) cudaGetLastError();  // not an error of the caller's
   return ok;
 }
+// d: without buffers (after an error drop_walk gives back those that it got)
 int upload_walk(dndsg_ctx* c, const WalkSchedule& w, dndsg_ctx::Walk& d) {
   if (!walk_fits(c, w.ns, w.K, w.width, w.mail, w.bars)) return fail(c, DNDSG_CUDA_ERROR, "kernel attributes of the LU-SGS walk");
   d.ns = w.ns;
@@ -2677,7 +2682,6 @@ int upload_walk(dndsg_ctx* c, const WalkSchedule& w, dndsg_ctx::Walk& d) {
   d.dev.bars = w.bars;
   int rc;
   auto put = [&](auto*& dst, const auto& src) -> int {
-    dfree(c, dst);
     if ((rc = dalloc(c, dst, sizeof(src[0]) * src.size()))) return rc;
     DG_CUDA(c, cudaMemcpy((void*)dst, src.data(), sizeof(src[0]) * src.size(), cudaMemcpyHostToDevice));
     return 0;
@@ -2688,13 +2692,21 @@ int upload_walk(dndsg_ctx* c, const WalkSchedule& w, dndsg_ctx::Walk& d) {
   return 0;
 }
 
+void drop_walk(dndsg_ctx* c, dndsg_ctx::Walk& d) {
+  dfree(c, d.dev.nbF);
+  dfree(c, d.dev.nbJ);
+  dfree(c, d.dev.meta);
+  dfree(c, d.dev.batches);
+  dfree(c, d.dev.blockBatch);
+}
+
 // the reference's sequential sweep in a given scan order, level-scheduled: the forward level of a
 // cell is one more than the largest forward level of its neighbours earlier in the scan (the
 // backward level likewise over the later ones).  With parts (the reference on several ranks,
 // DNDS_FV_EulerEvaluator.cpp:1177-1181, 1313-1317) every part sweeps its own cells in the scan order:
 // levels count only neighbours of the same part, and a neighbour in another part enters the backward
-// sweep only, as a ghost with its post-forward increment
-int set_scan_order(dndsg_ctx* c, const int64_t* scan2cell) {
+// sweep only, as a ghost with its post-forward increment.  After an error the schedule in force is the one before
+int set_scan_order(dndsg_ctx* c, const int64_t* scan2cell, const std::vector<int32_t>& lusgsPart, int P) {
   int rc;
   if ((rc = ensure_lusgs(c))) return rc;
   const int64_t N = c->N;
@@ -2705,11 +2717,8 @@ int set_scan_order(dndsg_ctx* c, const int64_t* scan2cell) {
     pos[i] = (int32_t)s;
     order[s] = (int32_t)i;
   }
-  if (scan2cell) c->scanHost.assign(scan2cell, scan2cell + N);
-  else c->scanHost.clear();
-  const int P = c->lusgsParts;
   std::vector<int32_t> part(N, 0);
-  if (P > 1) part = c->lusgsPart;
+  if (P > 1) part = lusgsPart;
   std::vector<int64_t> deg;
   std::vector<int32_t> adj;
   if ((rc = lusgs_adjacency(c, deg, adj))) return rc;
@@ -2747,13 +2756,35 @@ int set_scan_order(dndsg_ctx* c, const int64_t* scan2cell) {
   WalkSchedule fwd, bwd;
   choose_walks(N, P, part, order, pos, lf, nlf, lb, nlb, slotF, slotJ, c->sa, c->sms, kWalkHop,
                [&](int ns, int K, int mail, int bars) { return walk_fits(c, ns, K, kWalkW, mail, bars); }, fwd, bwd);
-  if ((rc = upload_walk(c, fwd, c->fwdWalk)) || (rc = upload_walk(c, bwd, c->bwdWalk))) return rc;
-  dfree(c, c->walkRec);
-  dfree(c, c->walkRec5);
+  // all of it into buffers of its own first (the records' ones are kept where they are large enough)
+  dndsg_ctx::Walk fw, bw;
+  void *rec = nullptr, *rec5 = nullptr;
   const int ns = std::max(fwd.ns, bwd.ns);
-  if ((rc = dalloc(c, c->walkRec, (size_t)walk_rec_bytes(ns) * N)) ||
-      (c->sa && (rc = dalloc(c, c->walkRec5, (size_t)walk_rec5_bytes(ns) * N))))
+  if ((rc = upload_walk(c, fwd, fw)) || (rc = upload_walk(c, bwd, bw)) ||
+      (ns > c->walkRecNs && ((rc = dalloc(c, rec, (size_t)walk_rec_bytes(ns) * N)) ||
+                             (c->sa && (rc = dalloc(c, rec5, (size_t)walk_rec5_bytes(ns) * N)))))) {
+    drop_walk(c, fw);
+    drop_walk(c, bw);
+    dfree(c, rec);
+    dfree(c, rec5);
     return rc;
+  }
+  drop_walk(c, c->fwdWalk);
+  drop_walk(c, c->bwdWalk);
+  c->fwdWalk = fw;
+  c->bwdWalk = bw;
+  if (ns > c->walkRecNs) {
+    dfree(c, c->walkRec);
+    dfree(c, c->walkRec5);
+    c->walkRec = rec;
+    c->walkRec5 = rec5;
+    c->walkRecNs = ns;
+  }
+  std::vector<int64_t> scan;
+  if (scan2cell) scan.assign(scan2cell, scan2cell + N);  // (scan2cell may be scanHost's own)
+  c->scanHost.swap(scan);
+  c->lusgsPart = P > 1 ? part : std::vector<int32_t>();
+  c->lusgsParts = P;
   c->fwdPartMax = fMax;
   c->bwdPartMax = bMax;
   c->lusgsOrder = 1;
@@ -2875,17 +2906,9 @@ int dndsg_lusgs_set_order(dndsg_ctx* c, int mode, const int64_t* scan2cell, int*
   int rc;
   if ((rc = set_device(c)) || (rc = ensure_lusgs(c))) return rc;
   if (mode == 1) {
-    if ((rc = set_scan_order(c, scan2cell))) return rc;
-  } else if (c->lusgsOrder != 0) {
-    const int64_t N = c->N;
-    const std::vector<int32_t>& col = c->colourHost;
-    const int ncol = 1 + *std::max_element(col.begin(), col.end());
-    std::vector<int32_t> fwd, bwd, rev(N);
-    group_by(col, ncol, fwd, c->fwdOff);
-    for (int64_t i = 0; i < N; i++) rev[i] = ncol - 1 - col[i];
-    group_by(rev, ncol, bwd, c->bwdOff);
-    c->lusgsOrder = 0;
-    if ((rc = upload_schedule(c, col, fwd, bwd))) return rc;
+    if ((rc = set_scan_order(c, scan2cell, c->lusgsPart, c->lusgsParts))) return rc;
+  } else {
+    c->lusgsOrder = 0;  // the colour schedule is still there
   }
   if (n_batches)
     *n_batches = c->lusgsOrder == 1 ? c->fwdPartMax + c->bwdPartMax : (int)(c->fwdOff.size() - 1 + c->bwdOff.size() - 1);
@@ -2900,17 +2923,12 @@ int dndsg_lusgs_set_parts(dndsg_ctx* c, const int32_t* part, int n_parts, int* n
   if (part && n_parts > 1) {
     for (int64_t i = 0; i < c->N; i++)
       if (part[i] < 0 || part[i] >= n_parts) return fail(c, DNDSG_BAD_ARGUMENT, "part index out of range");
-    c->lusgsPart.assign(part, part + c->N);
-    c->lusgsParts = n_parts;
   } else {
-    c->lusgsPart.clear();
-    c->lusgsParts = 1;
+    n_parts = 1;
   }
-  if ((rc = set_scan_order(c, c->scanHost.empty() ? nullptr : c->scanHost.data()))) {
-    c->lusgsPart.clear();
-    c->lusgsParts = 1;
-    return rc;
-  }
+  std::vector<int32_t> of;
+  if (n_parts > 1) of.assign(part, part + c->N);
+  if ((rc = set_scan_order(c, c->scanHost.empty() ? nullptr : c->scanHost.data(), of, n_parts))) return rc;
   if (n_batches) *n_batches = c->fwdPartMax + c->bwdPartMax;
   return 0;
 }
