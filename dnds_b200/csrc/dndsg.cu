@@ -132,9 +132,8 @@ struct dndsg_ctx {
   // triangles 473 -> 441, FP64 step on 1,672 triangles 52 -> 36).  On larger ones the early blocks of the next
   // kernel take room from the running one (dual-time step on 524,288 triangles 3838 -> 4276 us, FP32 step on
   // 2,097,152 1495 -> 1735), and a captured graph has its short edges already (five FP64 steps on 26,496
-  // triangles 300 -> 346 us with the attribute)
-  bool capturing = false;
-  bool small() const { return N <= kSmallCells && !capturing; }
+  // triangles 300 -> 346 us with the attribute): launch() leaves it out of every capture
+  bool small() const { return N <= kSmallCells; }
   // face passes of few warps per SM: a thread per Gauss point (ten FP64 steps on 1,600 quads 361 -> 337 us;
   // with three times the blocks a pass still is one wave of the device)
   bool splitFlux() const { return F <= kSplitMaxFaces; }
@@ -189,8 +188,15 @@ __device__ __forceinline__ double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+// whether launches into s are captured, by this library or by the caller (an error of the query: the launch
+// itself reports it)
+bool captured(cudaStream_t s) {
+  cudaStreamCaptureStatus state = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &state) != cudaSuccess) cudaGetLastError();
+  return state != cudaStreamCaptureStatusNone;
+}
 // a launch whose kernel starts with pdl_enter(); pdl: as a programmatic dependent of the stream's previous
-// kernel, so that its launch and block start overlap that kernel's run
+// kernel, so that its launch and block start overlap that kernel's run (except in a capture)
 template <class... P, class... A>
 void launch(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, bool pdl, A... a) {
   cudaLaunchAttribute attr;
@@ -202,7 +208,7 @@ void launch(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStr
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = &attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = pdl && !captured(s) ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k, P(a)...);
 }
 
@@ -1563,12 +1569,10 @@ int dndsg_ssprk3_steps(dndsg_ctx* c, double cfl, double t_end, int64_t n, void* 
       if (!c->capStream) DG_CUDA(c, cudaStreamCreateWithFlags(&c->capStream, cudaStreamNonBlocking));
       void* urec0 = c->urec;
       DG_CUDA(c, cudaStreamBeginCapture(c->capStream, cudaStreamCaptureModeThreadLocal));
-      c->capturing = true;
       for (int k = 0; k < 2; k++) {  // six buffer swaps: urec is back in its buffer afterwards
         if (c->fp32) run_step<float>(c, cfl, t_end, c->capStream);
         else run_step<double>(c, cfl, t_end, c->capStream);
       }
-      c->capturing = false;
       cudaGraph_t graph = nullptr;
       const cudaError_t e = cudaStreamEndCapture(c->capStream, &graph);
       if (e != cudaSuccess) return fail(c, DNDSG_CUDA_ERROR, std::string("step capture: ") + cudaGetErrorString(e));
