@@ -513,7 +513,8 @@ __device__ __forceinline__ void tc_store32(unsigned char* A, int row, int c0, co
 // order was not fixed).
 // Measured, eight steps of 65,536 rows: 954 us with one tile in flight per SM and atomics, 790 us with two
 // tiles, 579 us with the rows; a step of 1,048,576 rows 1.10 ms -> 0.65 ms.
-constexpr int kTrPart = kNParam + 4;  // parameters' gradients, then the loss in two floats (high and low part)
+constexpr int kTrPart = kNParam + 4;  // parameters' gradients, then the loss as a double, and padding to 16 bytes
+static_assert(kNParam % 2 == 0 && kTrPart % 4 == 0, "the loss and every row are aligned");
 __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(MlpDev m, const float* X, const float* Tg, int64_t n,
                                                                 float invCount, float* part, unsigned* flags) {
   extern __shared__ __align__(128) unsigned char raw[];
@@ -754,8 +755,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(MlpDev m, const 
   if (tid == 0) {
     double t = 0;
     for (int w = 0; w < kTrThreads / 32; w++) t += lossW[w];
-    row[kNParam] = (float)t;
-    row[kNParam + 1] = (float)(t - (double)(float)t);
+    *reinterpret_cast<double*>(row + kNParam) = t;
   }
   if (bad)  // after a timeout: a defined row
     for (int e = tid; e < kNParam; e += kTrThreads) row[e] = 0.f;
@@ -801,10 +801,7 @@ __device__ __forceinline__ float tr_sum_rows(const float* part, int rows, int e,
 // the loss, by one warp
 __device__ __forceinline__ void tr_sum_loss(const float* part, int rows, double* loss) {
   double t = 0;
-  for (int b = threadIdx.x & 31; b < rows; b += 32) {
-    const float2 v = *reinterpret_cast<const float2*>(&part[(int64_t)b * kTrPart + kNParam]);
-    t += (double)v.x + (double)v.y;
-  }
+  for (int b = threadIdx.x & 31; b < rows; b += 32) t += *reinterpret_cast<const double*>(&part[(int64_t)b * kTrPart + kNParam]);
   t = warp_sum_d(t);
   if ((threadIdx.x & 31) == 0) *loss = t;
 }

@@ -132,6 +132,24 @@ def test_gradient_matches_oracle():
 
 
 @pytest.mark.gpu
+def test_loss_above_the_float_range():
+    """Outputs near 1e19 of a diverging run: a CTA's sum of squares is above 3.4e38, the loss is a finite double."""
+    torch, dev = _torch()
+    from dnds_b200.learned import WarmStartNet
+
+    p = np.zeros(mo.N_PARAM, np.float32)
+    p[mo.OFF_B4:mo.OFF_B4 + mo.N_OUT] = 1e19
+    net = WarmStartNet(0, params=p)
+    X = torch.zeros((300, mo.N_IN), device=dev)
+    T = torch.zeros((300, mo.N_OUT), device=dev)
+    loss, _ = net.gradient(X, T)
+    want = float(np.float32(1e19)) ** 2
+    assert abs(loss - want) < 1e-12 * want  # 6,000 equal terms added in doubles: 6000 x 2^-53 at most
+    loss = net.train_step(X, T, 1e-3, want_loss=True)
+    assert abs(loss - want) < 1e-12 * want
+
+
+@pytest.mark.gpu
 def test_adam_step():
     torch, dev = _torch()
     from dnds_b200.learned import WarmStartNet
