@@ -1857,20 +1857,6 @@ extern "C" int dndsg_eval_rhs_noalloc(dndsg_ctx* c, const double* u, const void*
 }
 
 // ====================================================================== learned VR warm start
-struct dndsg_mlp {
-  int device = 0;
-  float *P = nullptr, *M = nullptr, *V = nullptr, *G = nullptr;
-  float* part = nullptr;  // per CTA of the training kernel: its gradients and loss [sms][kTrPart]
-  int sms = 148, rows = 0;
-  __nv_bfloat16* W = nullptr;
-  double* loss = nullptr;
-  unsigned* flags = nullptr;  // kFlagTimeout from the tensor-core forward
-  int64_t step = 0;
-  bool attrFwd = false, attrTrain = false;
-  int featureMode = 0;  // the feature design the network is trained for (dndsg_mlp_set_features)
-  std::string err;
-};
-
 namespace {
 int mfail(dndsg_mlp* m, int code, const std::string& msg) {
   if (m) m->err = msg;
@@ -2258,13 +2244,16 @@ int dndsg_mlp_train_step(dndsg_mlp* m, const float* X, const float* Tg, int64_t 
   const double b1 = 0.9, b2 = 0.999;
   const float c1 = (float)(1.0 / (1.0 - std::pow(b1, (double)m->step)));
   const float c2 = (float)(1.0 / (1.0 - std::pow(b2, (double)m->step)));
-  k_mlp_adam<<<(kNParam + kRedEntries - 1) / kRedEntries, 256, 0, st(s)>>>(m->P, m->M, m->V, m->part, m->rows, m->loss, m->W, lr,
+  k_mlp_adam<<<(kNParam + kRedEntries - 1) / kRedEntries, 256, 0, st(s)>>>(m->P, m->M, m->V, m->part, m->rows, m->loss, m->W, m->flags, lr,
                                                                          (float)b1, (float)b2, 1e-8f, c1, c2);
   DG_MCUDA(m, cudaGetLastError());
   if (loss) {
     double l = 0;
+    unsigned f = 0;
     DG_MCUDA(m, cudaMemcpyAsync(&l, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st(s)));
+    DG_MCUDA(m, cudaMemcpyAsync(&f, m->flags, sizeof(f), cudaMemcpyDeviceToHost, st(s)));
     DG_MCUDA(m, cudaStreamSynchronize(st(s)));
+    if (f) return mfail(m, DNDSG_TIMEOUT, "tensor-core completion wait timed out");
     *loss = l / (double)(n * kOut);
   }
   return 0;

@@ -24,7 +24,24 @@
 #pragma once
 #include <cuda_bf16.h>
 
+#include <string>
+
 #include "dndsg_bodies.cuh"
+
+// a network of the C interface
+struct dndsg_mlp {
+  int device = 0;
+  float *P = nullptr, *M = nullptr, *V = nullptr, *G = nullptr;
+  float* part = nullptr;  // per CTA of the training kernel: its gradients and loss [sms][kTrPart]
+  int sms = 148, rows = 0;
+  __nv_bfloat16* W = nullptr;
+  double* loss = nullptr;
+  unsigned* flags = nullptr;  // kFlagTimeout from the tensor-core kernels
+  int64_t step = 0;
+  bool attrFwd = false, attrTrain = false;
+  int featureMode = 0;  // the feature design the network is trained for (dndsg_mlp_set_features)
+  std::string err;
+};
 
 namespace dg {
 
@@ -813,14 +830,15 @@ __global__ void __launch_bounds__(256) k_mlp_reduce(const float* part, int rows,
   if (blockIdx.x == 0 && threadIdx.x / 32 == 7) tr_sum_loss(part, rows, loss);
 }
 // Adam (Kingma & Ba) on the FP32 master parameters, from the rows of gradients; padded entries stay zero;
-// refreshes the BF16 copy
+// refreshes the BF16 copy.  Nothing changes once a wait of this network ran out (flags): the gradient is then not one
 __global__ void __launch_bounds__(256) k_mlp_adam(float* P, float* Mo, float* V, const float* part, int rows, double* loss, bf16* W,
-                                                  float lr, float b1, float b2, float eps, float c1, float c2) {
+                                                  const unsigned* flags, float lr, float b1, float b2, float eps, float c1, float c2) {
   __shared__ float sh[4][kRedEntries];
+  const unsigned stopped = *flags;  // beside the rows
   const int e = blockIdx.x * kRedEntries + threadIdx.x % kRedEntries;
   const float g = tr_sum_rows(part, rows, e, sh);
   if (blockIdx.x == 0 && threadIdx.x / 32 == 7) tr_sum_loss(part, rows, loss);
-  if (threadIdx.x >= kRedEntries || e >= kNParam) return;
+  if (threadIdx.x >= kRedEntries || e >= kNParam || stopped) return;
   bool pad = false;
   int wi = -1;
   if (e < kOffB1) { pad = (e % kInP) >= kIn; wi = kWOff1 + e; }

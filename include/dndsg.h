@@ -429,15 +429,18 @@ int dndsg_mlp_set_params(dndsg_mlp* mlp, const float* params);
 int dndsg_mlp_get_params(dndsg_mlp* mlp, float* params);
 /* Y [n][20] = network(X [n][64]), device arrays.  Runs on the 5th-generation
  * tensor cores (tcgen05.mma, 128 rows per tile, FP32 accumulator in tensor
- * memory); returns when the forward is complete, DNDSG_CUDA_ERROR if a
- * tensor-core completion wait ran out (bounded wait) */
+ * memory); returns when the forward is complete, DNDSG_TIMEOUT if a
+ * tensor-core completion wait ran out (bounded wait), then and in every later
+ * call that waits for its result */
 int dndsg_mlp_forward(dndsg_mlp* mlp, const float* X, int64_t n, float* Y, void* stream);
 /* mean-square loss over n rows x 20 outputs against targets T [n][20] (device)
  * and its gradient (host [DNDSG_MLP_NPARAM], may be NULL); synchronous */
 int dndsg_mlp_gradient(dndsg_mlp* mlp, const float* X, const float* T, int64_t n, double* loss, float* grad,
                        void* stream);
 /* one Adam step (b1 0.9, b2 0.999, eps 1e-8) on the batch X, T (device);
- * loss (host, may be NULL) is the batch loss before the step */
+ * loss (host, may be NULL) is the batch loss before the step; with it the call
+ * waits and returns DNDSG_TIMEOUT if a tensor-core completion wait ran out.
+ * The network is not updated from there on, with or without loss */
 int dndsg_mlp_train_step(dndsg_mlp* mlp, const float* X, const float* T, int64_t n, float lr, double* loss,
                          void* stream);
 /* The warm start's input design, per context (for harvesting and use) and per

@@ -174,6 +174,24 @@ def test_adam_step():
 
 
 @pytest.mark.gpu
+def test_training_step_after_a_timeout(tmp_path):
+    """tests/mlp_timeout_check.cpp: with the timeout flag set, a step reports it and updates nothing."""
+    import os
+    import subprocess
+
+    from dnds_b200 import build
+
+    exe, cuda = tmp_path / "mlp_timeout_check", os.path.dirname(os.path.dirname(build.NVCC))
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(build.ROOT, "include"), "-I", os.path.join(build.HERE, "csrc"),
+                        "-I", os.path.join(cuda, "include"), os.path.join(build.ROOT, "tests", "mlp_timeout_check.cpp"),
+                        build.LIB, f"-Wl,-rpath,{os.path.dirname(build.LIB)}", "-L", os.path.join(cuda, "lib64"),
+                        f"-Wl,-rpath,{os.path.join(cuda, 'lib64')}", "-lcudart", "-o", str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and "ok" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.gpu
 def test_training_fits_a_teacher_network():
     torch, dev = _torch()
     from dnds_b200.learned import WarmStartNet, train
