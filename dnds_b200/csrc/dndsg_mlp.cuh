@@ -348,8 +348,10 @@ __global__ void __launch_bounds__(kTcRows, 4) k_mlp_tc(MlpDev m, Src src, Dst ds
     float bias = tc_bias_s(m.P, layer, rl) * (layer < 3 ? 0.5f : 1.0f);
     float c[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int k = 0; k < 3; k++) {
-      c[k] = __bfloat162float(__float2bfloat16(bias));
-      bias -= c[k];
+      float h = __bfloat162float(__float2bfloat16(bias));
+      if (isinf(h) && !isinf(bias)) h = __bfloat162float(__float2bfloat16_rz(bias));  // above the largest BF16 number
+      c[k] = h;
+      bias = isinf(h) ? 0.f : bias - h;
     }
     unsigned char* w = S.W + layer * kLayerBytes;
     *reinterpret_cast<uint4*>(w + cm_off_k(rl, 64)) = pack8(c);

@@ -110,6 +110,26 @@ def test_forward_tile_edges_and_row_independence(n):
 
 
 @pytest.mark.gpu
+def test_forward_biases_at_the_ends_of_the_float_range():
+    """A bias enters the product as three BF16 numbers: infinite ones and those that round to infinity in BF16 too."""
+    torch, dev = _torch()
+    from dnds_b200.learned import WarmStartNet
+
+    p = mo.random_params(6)
+    top = np.finfo(np.float32).max
+    bias = np.array([np.inf, -np.inf, top, -top, np.float32(3.395e38), 1.0 + 2.0 ** -23, np.nan], np.float32)
+    p[mo.OFF_B4:mo.OFF_B4 + bias.size] = bias
+    net = WarmStartNet(0, params=p)
+    Y = net.forward(torch.zeros((130, mo.N_IN), device=dev)).cpu().numpy()
+    assert np.isposinf(Y[:, 0]).all() and np.isneginf(Y[:, 1]).all() and np.isnan(Y[:, 6]).all()
+    for k in (2, 3, 4):  # the products with the activations are lost in the sum
+        assert (np.abs(Y[:, k] / bias[k] - 1) < 2.0 ** -22).all(), k
+    p[mo.OFF_B4 + 5] = 0.0
+    net = WarmStartNet(0, params=p)
+    assert np.abs(Y[:, 5] - net.forward(torch.zeros((130, mo.N_IN), device=dev)).cpu().numpy()[:, 5] - bias[5]).max() < 2.0 ** -20
+
+
+@pytest.mark.gpu
 def test_gradient_matches_oracle():
     torch, dev = _torch()
     from dnds_b200.learned import WarmStartNet
