@@ -66,3 +66,8 @@ extern "C" int flux_check(int64_t n, int riemann, const double* u, const float* 
   }
   return flagged;
 }
+
+// compress_rec_part of n means and increments [n][4]: the states r and whether each fell back to the mean
+extern "C" void compress_check(int64_t n, const double* um, const double* inc, double* r, int32_t* reduced) {
+  for (int64_t i = 0; i < n; i++) reduced[i] = compress_rec_part(um + 4 * i, inc + 4 * i, r + 4 * i) ? 1 : 0;
+}

@@ -89,3 +89,33 @@ def test_strong_jumps_within_fp32_of_the_jump(lib, riemann):
     assert reduced < 200
     assert rel.max() < 5e-5, rel.max()
     assert np.median(rel) < 2e-7, np.median(rel)
+
+
+def test_positivity_fallback_as_the_quotient_form(lib):
+    """CompressRecPart (DNDS_FV_EulerEvaluator.hpp:1277-1360) without its quotient: the mean where density or
+    E - |m|^2 / (2 (rho + 1e-200)) is negative, and the state as it is, not finite, where an entry is NaN (the flux then
+    flags it).  Zero and infinite entries too, one per state."""
+    rng = np.random.default_rng(3)
+    n = 40000
+    um = np.stack([rng.uniform(0.1, 2, n), rng.normal(0, 1, n), rng.normal(0, 1, n), rng.uniform(1, 5, n)], 1)
+    inc = um * rng.normal(0, 0.7, (n, 4))
+    at = np.arange(0, n, 4)
+    inc[at, rng.integers(0, 4, at.size)] = rng.choice([np.nan, np.inf, -np.inf], at.size)
+    zero = np.arange(1, n, 16)
+    k = rng.integers(0, 4, zero.size)
+    inc[zero, k] = -um[zero, k]
+    r, red = np.empty((n, 4)), np.empty(n, np.int32)
+    lib.compress_check.argtypes = [C.c_int64] + [C.c_void_p] * 4
+    lib.compress_check.restype = None
+    lib.compress_check(n, um.ctypes.data, inc.ctypes.data, r.ctypes.data, red.ctypes.data)
+    with np.errstate(all="ignore"):
+        want = um + inc
+        low = want[:, 0] < 0
+        want[low] = um[low]
+        kin = 0.5 * (want[:, 1] ** 2 + want[:, 2] ** 2) / (want[:, 0] + 1e-200)
+        cold = want[:, 3] - kin < 0
+        want[cold] = um[cold]
+        tie = np.abs(want[:, 3] - kin) < 1e-12 * np.abs(kin)  # a rounding decides
+    assert not tie.any() and low.sum() > 1000 and cold.sum() > 1000
+    assert np.array_equal(red != 0, low | cold)
+    assert np.array_equal(r, want, equal_nan=True)
