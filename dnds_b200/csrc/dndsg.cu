@@ -2645,7 +2645,7 @@ int ensure_lusgs(dndsg_ctx* c) {
   return upload_schedule(c, col, fwd, bwd);
 }
 
-constexpr int kMaxPartLevels = 4095;  // of one part, in partitioned sweeps
+constexpr int kMaxPartLevels = 4095;  // of one part, in partitioned sweeps: the limit that dndsg.h states (the walk has none)
 constexpr double kWalkHop = 3.0;      // a value from another block of the part, in batches of the walk
 
 template <int NS, bool SA>

@@ -130,6 +130,29 @@ def test_forward_biases_at_the_ends_of_the_float_range():
 
 
 @pytest.mark.gpu
+def test_forward_negative_tail_of_the_activation():
+    """Pre-activations of the last hidden layer from -12 to -2 against SiLU itself: within |z| 2^-12 (the hardware
+    tanh, 2^-11 relative) and the BF16 rounding of the activation, 2^-8 of it.  The layers before pass 16 + x on,
+    x in steps of 1/8: exact in BF16, and SiLU of it is within half a step."""
+    torch, dev = _torch()
+    from dnds_b200.learned import WarmStartNet
+
+    p = np.zeros(mo.N_PARAM)
+    W1, b1, W2, b2, W3, b3, W4, b4 = mo.unpack(p)
+    for W, sign in ((W1, 1.0), (W2, 1.0), (W3, -1.0)):
+        W[np.arange(mo.N_OUT), np.arange(mo.N_OUT)] = sign
+    W4[np.arange(mo.N_OUT), np.arange(mo.N_OUT)] = 1.0
+    b1[:mo.N_OUT], b3[:mo.N_OUT] = 16.0, 14.0
+    x = np.arange(0, 10.125, 0.125)
+    X = np.zeros((x.size, mo.N_IN), np.float32)
+    X[:, :mo.N_OUT] = x[:, None]
+    Y = WarmStartNet(0, params=p.astype(np.float32)).forward(torch.from_numpy(X).to(dev)).cpu().numpy()
+    z = -2.0 - x
+    silu = z / (1 + np.exp(-z))
+    assert (np.abs(Y - silu[:, None]) <= (np.abs(z) * 2.0 ** -12 + np.abs(silu) * 2.0 ** -8)[:, None]).all()
+
+
+@pytest.mark.gpu
 def test_gradient_matches_oracle():
     torch, dev = _torch()
     from dnds_b200.learned import WarmStartNet
