@@ -2128,7 +2128,8 @@ int dndsg_mlp_create(int device, uint64_t seed, dndsg_mlp** out) {
   auto bail = [&](int code) { dndsg_mlp_destroy(m); return code; };
   if (cudaSetDevice(device) != cudaSuccess) return bail(DNDSG_CUDA_ERROR);
   cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
-  if (cudaMalloc(&m->P, sizeof(float) * kNParam) != cudaSuccess ||
+  if (cudaMalloc(&m->part, sizeof(float) * kTrPart * m->sms) != cudaSuccess ||
+      cudaMalloc(&m->P, sizeof(float) * kNParam) != cudaSuccess ||
       cudaMalloc(&m->M, sizeof(float) * kNParam) != cudaSuccess ||
       cudaMalloc(&m->V, sizeof(float) * kNParam) != cudaSuccess ||
       cudaMalloc(&m->G, sizeof(float) * kNParam) != cudaSuccess ||
@@ -2204,18 +2205,6 @@ int mlp_grad(dndsg_mlp* m, const float* X, const float* Tg, int64_t n, cudaStrea
     DG_MCUDA(m, cudaFuncSetAttribute(k_mlp_train_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(TrTcSmem)));
     m->attrTrain = true;
-  }
-  if (!m->part) {  // by the first training call, which a caller may capture: the allocation is no work of its stream
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    DG_MCUDA(m, cudaThreadExchangeStreamCaptureMode(&mode));
-    void* q = nullptr;
-    const cudaError_t e = cudaMalloc(&q, sizeof(float) * kTrPart * m->sms);
-    DG_MCUDA(m, cudaThreadExchangeStreamCaptureMode(&mode));
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return mfail(m, DNDSG_CUDA_ERROR, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-    }
-    m->part = (float*)q;
   }
   const int64_t tiles = (n + kTcRows - 1) / kTcRows;
   m->rows = (int)std::min<int64_t>(tiles, m->sms);  // one CTA per SM

@@ -32,7 +32,7 @@
 struct dndsg_mlp {
   int device = 0;
   float *P = nullptr, *M = nullptr, *V = nullptr, *G = nullptr;
-  float* part = nullptr;  // per CTA of the training kernel: its gradients and loss [sms][kTrPart]; from the first training call
+  float* part = nullptr;  // per CTA of the training kernel: its gradients and loss [sms][kTrPart]
   int sms = 148, rows = 0;
   __nv_bfloat16* W = nullptr;
   double* loss = nullptr;
