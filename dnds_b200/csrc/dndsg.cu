@@ -2649,7 +2649,7 @@ bool walk_attr(int K, int width, int mail, int bars) {
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)K);
-  cfg.blockDim = dim3(walk_threads(SA));
+  cfg.blockDim = dim3(walk_threads(SA, width));
   cfg.dynamicSmemBytes = walk_smem(NS, SA, width, mail, bars);
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
@@ -2800,7 +2800,7 @@ void launch_walk_ns(dndsg_ctx* c, bool forward, const dndsg_ctx::Walk& w, const 
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)w.blocks);
-  cfg.blockDim = dim3(walk_threads(SA));
+  cfg.blockDim = dim3(walk_threads(SA, w.width));
   cfg.dynamicSmemBytes = walk_smem(NS, SA, w.width, w.dev.mail, w.dev.bars);
   cfg.stream = s;
   cfg.attrs = &attr;

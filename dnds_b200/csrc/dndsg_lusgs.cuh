@@ -167,21 +167,44 @@ __device__ __forceinline__ void walk_drain(int last, uint32_t full) {
     if (l % kWalkCopy == last % kWalkCopy) mbar_wait(full + 8 * (l % S), (uint32_t)(l / S) & 1u, kWaitLimit);
 }
 
+// The mailbox warp of a cluster's block: a batch's stage is full once its records are there and, by this warp, the
+// increments that it is the first to need.  The wait acquires at cluster scope, which takes longer than a wait at the
+// block's own: in the computing warps it was on the way of every level (natural order, RANS-SA on 512 x 128 cells 745 us
+// an iteration, laminar flow with GMRES on 256 x 64 cells 7.91 ms; by this warp 656 us and 6.63 ms).
+template <int S>
+__device__ __forceinline__ void walk_mail(int lane, int32_t nb, const WalkBatch* bat, uint32_t full, uint32_t empty, uint32_t mailB,
+                                          bool& failed) {
+  int32_t bars = -1, next = lane < nb ? bat[lane].bar : -1;  // lane k: batch l + k's barrier
+  for (int l = 0; l < nb; l++) {
+    if ((l & 31) == 0) {
+      bars = next;
+      next = l + 32 + lane < nb ? bat[l + 32 + lane].bar : -1;
+    }
+    const int32_t bar = __shfl_sync(0xffffffffu, bars, l & 31);
+    const uint32_t st = (uint32_t)(l % S);
+    bool ok = l < S || mbar_wait(empty + 8 * st, (uint32_t)(l / S - 1) & 1u, kWaitLimit);
+    if (ok && bar >= 0) ok = mbar_wait_cluster(mailB + 8 * bar, 0, kWaitLimit);
+    failed = __any_sync(0xffffffffu, !ok);
+    if (failed) break;
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full + 8 * st) : "memory");
+  }
+}
+
 constexpr uint32_t kWalkDrain = 1u << 10;  // tries of a wait for what is on its way between two blocks (10 us and more)
 
-// The walk, one block per run of scan positions, K blocks per part in a cluster.  Two sets of warps take the
+// The walk, one block per run of scan positions or cells, K blocks per part in a cluster.  Two sets of warps take the
 // batches in turn.  Of a set, warps 0-3 hold row v = lane & 3 of position 8 warp + lane / 4; SA: one warp
 // more, U5 of position `lane`.  A set loads its next records into registers while the other one
 // computes, so that a level is on its critical path only with the increments from shared memory, the row
 // product, the store and the barrier between the sets (the set that finished batch l arrives, the one that
 // takes l + 1 waits).  An increment for another block goes by st.async, which completes a barrier of the
-// batch that needs it there: no fence, and the wait for it lies before the barrier between the sets.  The
-// copying warps keep walk_stages() batches of records in flight (two of them: one's round per batch took
-// longer than a level, 0.29 against 0.22 us).  A wait that runs out sets kFlagTimeout; its warp then skips
-// the rest of its work, keeps to every barrier, and the blocks leave together (a mailbox may be written until
-// its block's peers are done, and a little later for one whose own waits did not see the last increments come).
+// batch that needs it there: no fence, and the mailbox warp waits for it beside the sets.  The copying warps
+// keep walk_stages() batches of records in flight (two of them: one's round per batch took longer than a level,
+// 0.29 against 0.22 us).  A wait that runs out sets kFlagTimeout; its warp then skips the rest of its work, keeps
+// to every barrier, and the blocks leave together (a mailbox may be written until its block's peers are done, and
+// a little later for one whose own waits did not see the last increments come).
 template <int NS, bool SA>
-__global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, const unsigned char* rec,
+__global__ void __launch_bounds__(walk_threads(SA, kWalkW), 1) k_lusgs_walk(WalkDev sc, const unsigned char* rec,
                                                                     const unsigned char* rec5, double* inc, double* inc5,
                                                                     unsigned* flags) {
   extern __shared__ __align__(128) unsigned char sm[];
@@ -196,7 +219,7 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
   const WalkBatch* bat = sc.batches + b0;
   if (tid == 0)
     for (int k = 0; k < S; k++) {
-      mbar_init(full + 8 * k, 1);
+      mbar_init(full + 8 * k, K > 1 ? 2 : 1);
       mbar_init(empty + 8 * k, NW);
     }
   if (K > 1)
@@ -216,7 +239,9 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
   if (K > 1) cluster_sync_all();
   bool failed = false;
   int last = -1;  // the copying warp's last batch
-  if (warp >= 2 * NW) {
+  if (warp == 2 * NW + kWalkCopy) {
+    if (K > 1) walk_mail<S>(lane, nb, bat, full, empty, mailB, failed);
+  } else if (warp >= 2 * NW) {
     last = walk_copy<RB, RB5, S, kWalkW>(warp - 2 * NW, lane, nb, bat, rec, rec5, full, empty, stR, stR5, failed);
   } else {
     const int set = warp >= NW ? 1 : 0, sw = warp - set * NW;
@@ -230,7 +255,7 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
     for (int l = set; l < nb; l += 2) {
       // ---- beside the other set's batch: the records of this one
       const uint32_t st = (uint32_t)(l % S), o = st * (rows ? kWalkW * RB : kWalkW * RB5), r = myRec + st * kWalkW * RB;
-      const int4 cur = bt;  // first position, positions, mailbox barrier
+      const int4 cur = bt;  // first position, positions
       if (l + 2 < nb) bt = *reinterpret_cast<const int4*>(bat + l + 2);
       if (!failed) failed = !mbar_wait(full + 8 * st, (uint32_t)(l / S) & 1u, kWaitLimit);
       // (lanes past the batch's positions read stale data and drop it)
@@ -244,7 +269,6 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
       const double x0 = lds1(myX0 + o);
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * st) : "memory");
-      if (K > 1 && cur.z >= 0 && !failed) failed = !mbar_wait_cluster(mailB + 8 * cur.z, 0, kWaitLimit);
       const bool act = pos < cur.y && !failed;
       const int32_t sr[4] = {src4.x, src4.y, src4.z, src4.w}, push[kWalkPush] = {to.x, to.y, to.z};
       uint32_t at[NS], pushAt[kWalkPush], pushBar[kWalkPush];
@@ -338,7 +362,7 @@ __global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk(WalkDev sc, 
 // U5: the iteration 2,830 -> 2,494 us); 75 parts of 112 x 224 quads 538 -> 498 us.  An increment that left the ring was
 // stored at least four batches and as many barriers before.
 template <int NS, bool SA>
-__global__ void __launch_bounds__(walk_threads(SA), 1) k_lusgs_walk_wide(WalkDev sc, const unsigned char* rec,
+__global__ void __launch_bounds__(walk_threads(SA, kWalkWide), 1) k_lusgs_walk_wide(WalkDev sc, const unsigned char* rec,
                                                                                    const unsigned char* rec5, double* inc,
                                                                                    double* inc5, unsigned* flags) {
   extern __shared__ __align__(128) unsigned char sm[];

@@ -39,7 +39,8 @@ constexpr int walk_rec5_bytes(int ns) { return ns * 32 + 16; }   // U5: rows, x0
 constexpr int walk_stages(int width) { return width == kWalkW ? 6 : 4; }             // batches of records in flight
 constexpr int kWalkCopy = 2;                                                         // copying warps
 constexpr int walk_rows(bool sa) { return 4 * kWalkW + (sa ? 32 : 0); }              // threads that compute a batch: rows, U5
-constexpr int walk_threads(bool sa) { return 2 * walk_rows(sa) + 32 * kWalkCopy; }   // two sets and the copying warps
+// two sets, the copying warps and the mailbox warp (a wide walk has no mailbox)
+constexpr int walk_threads(bool sa, int width) { return 2 * walk_rows(sa) + 32 * kWalkCopy + (width == kWalkW ? 32 : 0); }
 // the stages' barriers, the mailbox barriers, values, U5 values, the stages' records
 constexpr size_t walk_smem(int ns, bool sa, int width, int mail, int bars) {
   return (((size_t)walk_stages(width) * 16 + (size_t)bars * 8 + 31) & ~(size_t)31) + (size_t)(kWalkZero + 1 + mail) * 32 +
