@@ -2133,9 +2133,10 @@ int dndsg_mlp_create(int device, uint64_t seed, dndsg_mlp** out) {
       cudaMalloc(&m->M, sizeof(float) * kNParam) != cudaSuccess ||
       cudaMalloc(&m->V, sizeof(float) * kNParam) != cudaSuccess ||
       cudaMalloc(&m->G, sizeof(float) * kNParam) != cudaSuccess ||
-      cudaMalloc(&m->W, sizeof(__nv_bfloat16) * kNW) != cudaSuccess || cudaMalloc(&m->loss, sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&m->flags, sizeof(unsigned)) != cudaSuccess || cudaMemset(m->flags, 0, sizeof(unsigned)) != cudaSuccess)
+      cudaMalloc(&m->W, sizeof(__nv_bfloat16) * kNW) != cudaSuccess || cudaMalloc(&m->loss, sizeof(MlpResult)) != cudaSuccess ||
+      cudaMemset(m->loss, 0, sizeof(MlpResult)) != cudaSuccess)
     return bail(DNDSG_CUDA_ERROR);
+  m->flags = (unsigned*)(m->loss + 1);
   // Glorot-uniform weights from a 64-bit LCG, zero biases and padding
   std::vector<float> p(kNParam, 0.f);
   uint64_t st = seed * 6364136223846793005ull + 1442695040888963407ull;
@@ -2161,7 +2162,7 @@ int dndsg_mlp_create(int device, uint64_t seed, dndsg_mlp** out) {
 void dndsg_mlp_destroy(dndsg_mlp* m) {
   if (!m) return;
   cudaSetDevice(m->device);
-  for (void* q : {(void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->part, (void*)m->W, (void*)m->loss, (void*)m->flags})
+  for (void* q : {(void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->part, (void*)m->W, (void*)m->loss})
     if (q) cudaFree(q);
   delete m;
 }
@@ -2224,14 +2225,12 @@ int dndsg_mlp_gradient(dndsg_mlp* m, const float* X, const float* Tg, int64_t n,
   if (rc) return rc;
   k_mlp_reduce<<<(kNParam + kRedEntries - 1) / kRedEntries, 256, 0, st(s)>>>(m->part, m->rows, m->G, m->loss);
   DG_MCUDA(m, cudaGetLastError());
-  double l = 0;
-  DG_MCUDA(m, cudaMemcpyAsync(&l, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st(s)));
+  MlpResult r{};
   if (grad) DG_MCUDA(m, cudaMemcpyAsync(grad, m->G, sizeof(float) * kNParam, cudaMemcpyDeviceToHost, st(s)));
-  unsigned f = 0;
-  DG_MCUDA(m, cudaMemcpyAsync(&f, m->flags, sizeof(f), cudaMemcpyDeviceToHost, st(s)));
+  DG_MCUDA(m, cudaMemcpyAsync(&r, m->loss, sizeof(r), cudaMemcpyDeviceToHost, st(s)));
   DG_MCUDA(m, cudaStreamSynchronize(st(s)));
-  if (f) return mfail(m, DNDSG_TIMEOUT, "tensor-core completion wait timed out");
-  if (loss) *loss = l / (double)(n * kOut);
+  if (r.flags) return mfail(m, DNDSG_TIMEOUT, "tensor-core completion wait timed out");
+  if (loss) *loss = r.loss / (double)(n * kOut);
   return 0;
 }
 
@@ -2248,13 +2247,11 @@ int dndsg_mlp_train_step(dndsg_mlp* m, const float* X, const float* Tg, int64_t 
                                                                          (float)b1, (float)b2, 1e-8f, c1, c2);
   DG_MCUDA(m, cudaGetLastError());
   if (loss) {
-    double l = 0;
-    unsigned f = 0;
-    DG_MCUDA(m, cudaMemcpyAsync(&l, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st(s)));
-    DG_MCUDA(m, cudaMemcpyAsync(&f, m->flags, sizeof(f), cudaMemcpyDeviceToHost, st(s)));
+    MlpResult r{};
+    DG_MCUDA(m, cudaMemcpyAsync(&r, m->loss, sizeof(r), cudaMemcpyDeviceToHost, st(s)));
     DG_MCUDA(m, cudaStreamSynchronize(st(s)));
-    if (f) return mfail(m, DNDSG_TIMEOUT, "tensor-core completion wait timed out");
-    *loss = l / (double)(n * kOut);
+    if (r.flags) return mfail(m, DNDSG_TIMEOUT, "tensor-core completion wait timed out");
+    *loss = r.loss / (double)(n * kOut);
   }
   return 0;
 }

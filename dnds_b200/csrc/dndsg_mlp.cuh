@@ -28,15 +28,21 @@
 
 #include "dndsg_bodies.cuh"
 
+// what a training call reads back, in one copy (a copy of its own for the flags took 3 us per step)
+struct MlpResult {
+  double loss;
+  unsigned flags;  // kFlagTimeout from the tensor-core kernels
+};
 // a network of the C interface
 struct dndsg_mlp {
   int device = 0;
   float *P = nullptr, *M = nullptr, *V = nullptr, *G = nullptr;
-  float* part = nullptr;  // per CTA of the training kernel: its gradients and loss [sms][kTrPart]
+  float* part = nullptr;  // per CTA of the training kernel: its gradients and loss [sms][kTrPart], 8.6 MB.  (From the first training
+                          // call instead of the creation: that call took 1.2-2.4 ms for 0.6)
   int sms = 148, rows = 0;
   __nv_bfloat16* W = nullptr;
-  double* loss = nullptr;
-  unsigned* flags = nullptr;  // kFlagTimeout from the tensor-core kernels
+  double* loss = nullptr;     // of an MlpResult
+  unsigned* flags = nullptr;  // of the same
   int64_t step = 0;
   bool attrFwd = false, attrTrain = false;
   int featureMode = 0;  // the feature design the network is trained for (dndsg_mlp_set_features)
@@ -839,11 +845,12 @@ __global__ void __launch_bounds__(256) k_mlp_reduce(const float* part, int rows,
 __global__ void __launch_bounds__(256) k_mlp_adam(float* P, float* Mo, float* V, const float* part, int rows, double* loss, bf16* W,
                                                   const unsigned* flags, float lr, float b1, float b2, float eps, float c1, float c2) {
   __shared__ float sh[4][kRedEntries];
-  const unsigned stopped = *flags;  // beside the rows
   const int e = blockIdx.x * kRedEntries + threadIdx.x % kRedEntries;
   const float g = tr_sum_rows(part, rows, e, sh);
   if (blockIdx.x == 0 && threadIdx.x / 32 == 7) tr_sum_loss(part, rows, loss);
-  if (threadIdx.x >= kRedEntries || e >= kNParam || stopped) return;
+  if (threadIdx.x >= kRedEntries || e >= kNParam) return;
+  const float m0 = Mo[e], v0 = V[e], p0 = P[e];  // and the flag, one wait for all (read before the rows it took 2 us per step)
+  if (*flags) return;
   bool pad = false;
   int wi = -1;
   if (e < kOffB1) { pad = (e % kInP) >= kIn; wi = kWOff1 + e; }
@@ -852,10 +859,10 @@ __global__ void __launch_bounds__(256) k_mlp_adam(float* P, float* Mo, float* V,
   else if (e >= kOffW4 && e < kOffB4) { pad = (e - kOffW4) / kHid >= kOut; wi = kWOff4 + (e - kOffW4); }
   else if (e >= kOffB4) pad = (e - kOffB4) >= kOut;
   if (pad) { P[e] = 0.f; if (wi >= 0) W[wi] = __float2bfloat16(0.f); return; }
-  const float m = b1 * Mo[e] + (1.f - b1) * g, v = b2 * V[e] + (1.f - b2) * g * g;
+  const float m = b1 * m0 + (1.f - b1) * g, v = b2 * v0 + (1.f - b2) * g * g;
   Mo[e] = m;
   V[e] = v;
-  const float p = P[e] - lr * (m * c1) / (sqrtf(v * c2) + eps);
+  const float p = p0 - lr * (m * c1) / (sqrtf(v * c2) + eps);
   P[e] = p;
   if (wi >= 0) W[wi] = __float2bfloat16(p);
 }
