@@ -245,7 +245,8 @@ DG_HD bool compress_rec_part(const double* um, const double* inc, double* r) {
   bool red = false;
   if (r[0] < 0) { for (int k = 0; k < 4; k++) r[k] = um[k]; red = true; }
   // internal energy E - |m|^2 / (2 (rho + 1e-200)) < 0, without the quotient (as that one, false where an entry is NaN)
-  if (2.0 * (kVerySmall + r[0]) * r[3] < r[1] * r[1] + r[2] * r[2]) {
+  const double w = kVerySmall + r[0];
+  if ((w + w) * r[3] < r[1] * r[1] + r[2] * r[2]) {
     for (int k = 0; k < 4; k++) r[k] = um[k];
     red = true;
   }
