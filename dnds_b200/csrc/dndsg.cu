@@ -29,9 +29,9 @@ constexpr int kBlock = 256;
 inline unsigned grid_for(int64_t n) { return (unsigned)((n + kBlock - 1) / kBlock); }
 // The block of the passes that wait on gathered rows (face flux, limiter face pass, cell update, the cell
 // pass and the colour batches of an implicit iteration).  Their residency is set by registers, and a small
-// block gives its share back as soon as its own rows have come, not when the slowest of 256 has: on
-// 2,097,152 triangles 256 -> 128 -> 64 threads in the face flux alone takes the FP64 step from 2335 to 2297 to
-// 2284 us, the FP32 one from 1465 to 1455 to 1453 us; the other passes a further 14 us each
+// block gives its share back as soon as its own rows have come, not when the slowest of 256 has.  Blocks of 256 and
+// of 64 threads in all of them: on 2,097,152 triangles 2294 and 2252 us per FP64 step, 1447 and 1430 us per FP32
+// step, 2056 and 2023 us per limited FP32 step, on 524,288 triangles 3555 and 3438 us per dual-time step
 constexpr int kHotBlock = 64;
 inline unsigned hot_grid(int64_t n) { return (unsigned)((n + kHotBlock - 1) / kHotBlock); }
 
@@ -624,8 +624,8 @@ __global__ void k_fill_dt(double* dt, int64_t n, const double* scal) {
 // rhs gather + (optionally) SSP-RK3 stage update (ExplicitSSPRK3LocalDt::Step, DNDS_ODE.hpp:140-163).
 // STEP = true, the whole-step composition: the first stage takes dt from the minimum itself (and writes it
 // for the later stages) and keeps its means as uLast, the last stage advances the time, so that a step
-// needs no launches of their own for these (10 launches instead of 13; ten graph-replayed steps on 1,600
-// quads 394 -> 361 us) and no pass that copies the means.  One thread writes each scalar; no other thread of
+// needs no launches of their own for these (10 launches instead of 13; the change took ten graph-replayed steps
+// on 1,600 quads from 394 to 361 us) and no pass that copies the means.  One thread writes each scalar; no other thread of
 // the launch reads that one
 template <class T, int STAGE, bool STEP = false>
 __global__ void __launch_bounds__(kHotBlock) k_cell_update(HotView<T> h, double* scal, double tEnd) {
@@ -2394,8 +2394,8 @@ __device__ __forceinline__ double impl_combine(const ImplComb& c, int64_t e, dou
 
 // The cell pass of an implicit iteration after its face fluxes: EvaluateRHS's gather, the local dt of
 // EvaluateDt, the LU-SGS diagonal (LUSGSMatrixInit) and the BDF or SDIRK right-hand side, in one pass over
-// the faces' fluxes and lambda A (five launches of their own before: on 524,288 triangles 67 us of kernels
-// and a copy; 27 us in one pass, before its gathers were loaded together).  The residual accumulators of the iteration start from zero here.
+// the faces' fluxes and lambda A.  On 524,288 triangles 26 us; as five launches of their own 67 us and a copy.  The
+// residual accumulators of the iteration start from zero here.
 template <class T>
 __global__ void __launch_bounds__(kHotBlock) k_implicit_cell(HotView<T> h, const __grid_constant__ ImplComb cb, double cfl, double dtPhysInv,
                                                           double alpha, double* Dinv, double* D, double* resAcc) {

@@ -20,9 +20,9 @@ namespace dg {
 // holds finished matrix rows: four lanes compute a cell, each one row, a chain of two products and three
 // sums per level.  Records with the generating quantities of a matrix (10 values instead of 16) made that
 // chain 15 operations and one thread's work per cell, and the copying of the records, in step with every
-// level, took longer than the level: 0.6-0.7 us.  Now 0.21 us per level (0.27 us with U5): forward or
-// backward sweep in natural order on 512 x 128 quads with U5 480 -> 190 us, on 256 x 64 quads 203 -> 81 us,
-// 16 parts of the former 97 -> 47 us.
+// level, took longer than the level: 0.6-0.7 us.  Now 0.23-0.30 us per level: in natural order on 512 x 128 quads with
+// U5, 639 levels, 482 -> 172 us forward and 464 -> 194 us backward (three neighbours per record, at the wake cut), on
+// 256 x 64 quads, 319 levels, 203 -> 74 and 80 us, in 16 parts of the former, 159 levels, 97 -> 40 us.
 
 // the fields of a context that the records are made of
 struct WalkGeom {

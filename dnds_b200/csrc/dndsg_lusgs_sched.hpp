@@ -223,11 +223,10 @@ inline bool build_walk(int64_t N, int parts, const std::vector<int32_t>& part, c
 // The schedules of both sweeps.  A part is walked by a cluster of blocks, one per 8 cells of a mean level, where the
 // lengths of the walks make that shorter than one block; sweeps of quads in natural order, us (lengths):
 //                              one block     one block, wide   cluster of 16 or 8
-//   512 x 128, 103 a level     462 (2172)      315 (1495)         201 (684)
-//   1000 x 70, 65 a level      620 (3015)      565 (2613)         331 (2119)
-//   256 x 64, 51 a level       127 (574)        91 (415)          102 (340)
-// (0.15-0.26 us per batch of a cluster, so that near the line the lengths may take the slower one, by a tenth).  The
-// blocks have runs of consecutive scan positions, or of cells where those of the scan order do not fit (an order that
+//   512 x 128, 103 a level     462 (2172)      315 (1495)         157 (684)
+//   1000 x 70, 65 a level      620 (3015)      565 (2613)         250 (2119)
+//   256 x 64, 51 a level       127 (574)        91 (415)           81 (340)
+// The blocks have runs of consecutive scan positions, or of cells where those of the scan order do not fit (an order that
 // jumps about the mesh: its neighbours are in other runs), and there are half as many where those do not either: when
 // the walk does not get shorter by them, the mailboxes do not fit the shared memory, or the device (fits(ns, K, mail,
 // bars)) does not take such a cluster.

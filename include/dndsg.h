@@ -243,7 +243,9 @@ int dndsg_lusgs_colours(dndsg_ctx* ctx, int32_t* colour_out, int* n_colours);
  * reference's SOR_iScan2iCell default), run as dependency levels (one batch
  * per level) so that it computes what the sequential sweep computes.
  * n_batches (may be NULL): forward plus backward batches per iteration (mode 1
- * with parts: the most levels of one part, forward plus backward). */
+ * with parts: the most levels of one part, forward plus backward).
+ * After an error of this call or the next one the order and the parts in force
+ * stay as they were. */
 int dndsg_lusgs_set_order(dndsg_ctx* ctx, int mode, const int64_t* scan2cell, int* n_batches);
 /* partitioned sweeps: the mode-1 sweep as the reference runs it on n_parts MPI
  * ranks (DNDS_FV_EulerEvaluator.cpp:1177-1181, 1313-1317; replaces the ranks'

@@ -242,9 +242,9 @@ def test_level_scheduled_natural_order_matches_sequential_oracle(oracle_lib):
 @pytest.mark.gpu
 def test_scan_order_beyond_the_shared_level_table_matches_oracle(oracle_lib):
     """A 2200 x 2 channel in the natural order has 2201 levels per sweep; a scan order that walks the
-    channel back and forth (rows alternately forward and reversed) makes more than 4095 levels
-    (the level table one block keeps in shared memory), so the sweep runs on the general
-    level-by-level path.  Both agree with the oracle's sequential sweep."""
+    channel back and forth (rows alternately forward and reversed) makes 4400 levels of one cell, more than
+    a part of a partitioned sweep may have: an unpartitioned one takes any number.  The sweeps agree with the
+    oracle's sequential one."""
     from dnds_b200.solver import DndsgError
 
     m = M.structured_grid(2200, 2, 440.0, 0.4, periodic=False)
@@ -292,11 +292,11 @@ def test_line_scan_order_matches_oracle(oracle_lib):
 
 @pytest.mark.gpu
 def test_wide_levels_read_records_and_increments_from_global_memory(oracle_lib):
-    """The line order on a C-mesh 300 cells around makes levels of about 300 positions: a level
-    holds more positions than the walk buffers records for (128; the rest are read from global
-    memory), and a neighbour one level back is sometimes more than the 256 positions of the
-    increment ring behind (read from global memory), sometimes not.  The sweep still computes what
-    the oracle's sequential sweep in that order computes."""
+    """The line order on a C-mesh 300 cells around makes levels of about 300 positions, which a cluster of
+    blocks with runs of cells walks (runs of the scan order hold even lines or odd ones, and nearly every
+    neighbour is in another run).  The sweep computes what the oracle's sequential sweep in that order
+    computes.  (Increments that left a block's ring of 256 positions, and so come from global memory:
+    tests/test_lusgs_walk.py, shuffled orders and cells.)"""
     m = M.naca0012_cmesh(200, 50, 8, first=2e-3, far=10.0, wall_bc=M.BC_WALL_EULER)
     cfg = _cfg()
     scan = M.line_scan_order(m)
