@@ -160,11 +160,14 @@ __device__ __forceinline__ int walk_copy(int w, int lane, int32_t nb, const Walk
   }
   return last;
 }
-// after a timeout: the warp's copies in flight land before the block leaves
+// After a timeout: the warp's copies in flight land before the block leaves.  A stage's phase may never complete then
+// (the mailbox warp or a computing warp left its part out), so these waits are short against kWaitLimit and long
+// against a copy, or an increment on its way between two blocks
+constexpr uint32_t kWalkDrain = 1u << 14;
 template <int S>
 __device__ __forceinline__ void walk_drain(int last, uint32_t full) {
   for (int l = max(last - S + kWalkCopy, 0); l <= last; l++)
-    if (l % kWalkCopy == last % kWalkCopy) mbar_wait(full + 8 * (l % S), (uint32_t)(l / S) & 1u, kWaitLimit);
+    if (l % kWalkCopy == last % kWalkCopy) mbar_wait(full + 8 * (l % S), (uint32_t)(l / S) & 1u, kWalkDrain);
 }
 
 // The mailbox warp of a cluster's block: a batch's stage is full once its records are there and, by this warp, the
@@ -189,8 +192,6 @@ __device__ __forceinline__ void walk_mail(int lane, int32_t nb, const WalkBatch*
     if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full + 8 * st) : "memory");
   }
 }
-
-constexpr uint32_t kWalkDrain = 1u << 10;  // tries of a wait for what is on its way between two blocks (10 us and more)
 
 // The walk, one block per run of scan positions or cells, K blocks per part in a cluster.  Two sets of warps take the
 // batches in turn.  Of a set, warps 0-3 hold row v = lane & 3 of position 8 warp + lane / 4; SA: one warp
